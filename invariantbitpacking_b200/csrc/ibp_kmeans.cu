@@ -5,19 +5,20 @@
 //  * a host-resident table is copied to HBM once by the copy engine (when the caller's
 //    workspace has room) and all ten rounds read HBM; the reference re-reads pinned host
 //    memory over PCIe in every round.
-//  * assignment: one warp per row, centroids in shared memory, warp-reduced Hamming
-//    distances; ties go to the highest centroid id (a deterministic choice among the
-//    reference's racy outcomes, see include/preproc/ibp_preproc_kmeans.cuh:139-146).
-//  * update: per-(cluster, word, bit) set counts.  A warp takes 32 rows (lane = row),
-//    forms one membership ballot per cluster and one ballot per bit, and adds
-//    popc(bit ballot & membership) into per-block shared-memory counters (lane = cluster:
-//    one shared atomic per (cluster, bit) per 32 rows, no bank conflicts); the reference
-//    issues one global atomic per set bit.
+//  * a round is one kernel over row tiles and a small one for the centroids.  The tile kernel
+//    takes Hamming distances as an integer matrix product on the tensor cores; ties go to the
+//    highest centroid id (a deterministic choice among the reference's racy outcomes, see
+//    include/preproc/ibp_preproc_kmeans.cuh:139-146).  It then lists the tile's rows by cluster
+//    in shared memory and counts the set bits of each cluster's rows in bit planes
+//    (ibp_bitcount.cuh); the reference issues one global atomic per set bit.
+//  * centroids too many or too long for shared memory once expanded take their distances in
+//    assign_kernel (a warp per row, population counts), and the tile kernel counts only.
 //  * the counts of the last round are exactly those of the final assignment, so the
 //    final masks need no extra pass over the data.
 #include <algorithm>
 #include <vector>
 
+#include "ibp_bitcount.cuh"
 #include "ibp_common.cuh"
 #include "ibp_internal.cuh"
 
@@ -78,121 +79,374 @@ assign_kernel(const U *__restrict__ data, int64_t n, int64_t v, const U *__restr
     }
 }
 
-// bits[(cl*v + k)*W + b] += rows of cluster cl with bit b of word k set.
-// Block (bx, tile) covers words [tile*kt, tile*kt + kt); shared counters [C][kt*W + 1].
-template <typename U>
-__global__ void __launch_bounds__(256)
-cluster_bits_kernel(const U *__restrict__ data, int64_t n, int64_t v,
-                    const int32_t *__restrict__ clusters, int c, int kt,
-                    uint32_t *__restrict__ bits) {
-    constexpr int W = 8 * sizeof(U);
-    extern __shared__ uint32_t sc[];
-    const int stride = kt * W + 1;
-    const int64_t k0 = (int64_t)blockIdx.y * kt;
-    const int kn = (int)((v - k0) < kt ? (v - k0) : kt);
-    for (int e = threadIdx.x; e < c * stride; e += blockDim.x) sc[e] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t g = warp; g * 32 < n; g += nwarps) {
-        const int64_t r = g * 32 + lane;
-        const bool live = r < n;
-        const int cl = live ? clusters[r] : -1;
-        for (int cb = 0; cb < c; cb += 32) {
-            uint32_t mine = 0;
-            const int lim = (c - cb) < 32 ? (c - cb) : 32;
-            for (int q = 0; q < lim; ++q) {
-                const uint32_t m = __ballot_sync(0xffffffffu, cl == cb + q);
-                if (lane == q) mine = m;
+// ------------------------------------------------------------------ one round
+// Distances as an integer matrix product.  popc(x ^ c) = popc(x) + popc(c) - 2 popc(x & c),
+// and popc(x) is the same for every centroid, so the nearest one minimises
+// popc(c) - 2 popc(x & c), and popc(x & c) over all centroids is a product of 0/1 matrices.
+// A 32-bit unit of a row becomes eight registers of four bytes, x & (0x01010101 << s): byte
+// values 2^s, one AND each.  The centroids are expanded once per block into shared memory
+// with byte values 2^(7 - s), so every common bit adds 128 to a 32-bit accumulator of
+// mma.m16n8k32 (u8 x u8, exact).  The order of K is free, so a lane takes 16 consecutive
+// bytes of a row and no operand is shuffled.  mma.sync rather than tcgen05: A exists only in
+// registers (expanding it into shared memory or TMEM would cost more than the product), and N
+// is the number of centroids.  Bound: issue (8 ANDs, 4 products and one 16-byte shared read
+// per 32 rows x 8 bits of a lane's unit).
+__device__ __forceinline__ void mma_u8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                       uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, "
+                 "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr int kRoundThreads = 512;
+constexpr int kRoundWarps = kRoundThreads / 32;
+constexpr int kTileRows = 4096;   // most rows of a tile (16-bit row numbers in shared memory)
+constexpr int kTaskRows = 255;    // rows a lane's eight bit planes can count
+constexpr int kFlushStride = 17;  // words per lane of a warp's flush buffer (16 + 1 of padding)
+
+// Shared memory of kmeans_round_kernel: expanded centroids, their set bits, three words per
+// cluster (histogram, first list entry, first task), the tile's clusters and row list, and a
+// flush buffer per warp.
+struct RoundShape {
+    int units;    // 32-bit units per row
+    int groups;   // 64-byte groups of a row
+    int pairs;    // pairs of 8-centroid tiles
+    bool assign;  // false: the clusters are already in `assign`
+    __host__ __device__ size_t expanded() const { return assign ? (size_t)pairs * groups * 8192 : 0; }
+    size_t bytes(int c) const {
+        return expanded() + align_up(sizeof(int32_t) * 16 * (size_t)pairs, 16) +
+               align_up(sizeof(uint32_t) * (3 * (size_t)c + 2), 16) + 2 * 2 * (size_t)kTileRows +
+               sizeof(uint32_t) * 32 * kFlushStride * kRoundWarps;
+    }
+};
+
+// Nearest centroids of the 32 rows r0.. (highest centroid on ties), into scl[r - base] and
+// `assign`; hist counts them.  V16: rows are 16-byte aligned.
+template <bool V16>
+__device__ __forceinline__ void assign_rows(const uint32_t *__restrict__ data, int64_t r0,
+                                            int64_t rend, int64_t base, const RoundShape &sh,
+                                            int c, const uint4 *__restrict__ expanded,
+                                            const int32_t *__restrict__ pcs, uint16_t *scl,
+                                            uint32_t *hist, int32_t *__restrict__ assign) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    int bestd[4], bestj[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        bestd[q] = 0x7fffffff;
+        bestj[q] = 0;
+    }
+    const uint32_t *row[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int64_t r = r0 + g + 8 * q;
+        row[q] = data + (r < rend ? r : r0) * sh.units;  // rows past the end: a valid row, unused
+    }
+    for (int p = 0; p < sh.pairs; ++p) {
+        const bool two = 16 * p + 8 < c;  // centroids in the pair's second tile
+        int32_t acc[2][2][4];
+#pragma unroll
+        for (int x = 0; x < 16; ++x) acc[x >> 3][(x >> 2) & 1][x & 3] = 0;
+        const uint4 *bp = expanded + (size_t)p * sh.groups * 512 + lane;
+        for (int k = 0; k < sh.groups; ++k, bp += 512) {
+            const int u = 16 * k + 4 * t;
+            uint32_t x[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if constexpr (V16) {
+                    uint4 y = make_uint4(0, 0, 0, 0);
+                    if (u < sh.units) y = *reinterpret_cast<const uint4 *>(row[q] + u);
+                    x[q][0] = y.x, x[q][1] = y.y, x[q][2] = y.z, x[q][3] = y.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[q][i] = u + i < sh.units ? row[q][u + i] : 0u;
+                }
             }
-            if (__ballot_sync(0xffffffffu, mine != 0) == 0) continue;
-            uint32_t *myc = sc + (int64_t)(cb + lane) * stride;
-            for (int kk = 0; kk < kn; ++kk) {
-                const U x = live ? data[r * v + k0 + kk] : (U)0;
-#pragma unroll 8
-                for (int b = 0; b < W; ++b) {
-                    const uint32_t bm = __ballot_sync(0xffffffffu, (x >> b) & 1);
-                    // the block's warps share these counters: shared-memory atomics
-                    if (lane < lim && (bm & mine)) atomicAdd(&myc[kk * W + b], __popc(bm & mine));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const uint4 b = bp[(i * 4 + s) * 32];
+                    const uint32_t lo = 0x01010101u << (2 * s), hi = lo << 1;
+                    const uint32_t a0[4] = {x[0][i] & lo, x[1][i] & lo, x[0][i] & hi, x[1][i] & hi};
+                    const uint32_t a1[4] = {x[2][i] & lo, x[3][i] & lo, x[2][i] & hi, x[3][i] & hi};
+                    mma_u8(acc[0][0], a0, b.x, b.y);
+                    mma_u8(acc[1][0], a1, b.x, b.y);
+                    if (two) {
+                        mma_u8(acc[0][1], a0, b.z, b.w);
+                        mma_u8(acc[1][1], a1, b.z, b.w);
+                    }
                 }
             }
         }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < c * kt * W; e += blockDim.x) {
-        const int cl = e / (kt * W), rem = e % (kt * W);
-        const int kk = rem / W, b = rem % W;
-        if (kk < kn) {
-            const uint32_t val = sc[cl * stride + rem];
-            if (val) atomicAdd(&bits[(cl * v + k0 + kk) * W + b], val);
+        // lane (g, t) holds centroids 2t, 2t+1 of each tile for rows g, g+8 of each 16 rows
+#pragma unroll
+        for (int x = 0; x < 16; ++x) {
+            const int m = x >> 3, nt = (x >> 2) & 1, e = x & 3;
+            const int q = 2 * m + (e >> 1), j = 16 * p + 8 * nt + 2 * t + (e & 1);
+            const int d = pcs[j] - (acc[m][nt][e] >> 6);  // popc(c) - 2 * (acc / 128)
+            if (j < c && d <= bestd[q]) {  // j rises: the highest centroid wins ties
+                bestd[q] = d;
+                bestj[q] = j;
+            }
         }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            const int d = __shfl_xor_sync(0xffffffffu, bestd[q], o);
+            const int j = __shfl_xor_sync(0xffffffffu, bestj[q], o);
+            if (d < bestd[q] || (d == bestd[q] && j > bestj[q])) {
+                bestd[q] = d;
+                bestj[q] = j;
+            }
+        }
+    }
+    // lane (g, t) writes row g + 8t
+    const int cl = t == 0 ? bestj[0] : (t == 1 ? bestj[1] : (t == 2 ? bestj[2] : bestj[3]));
+    const int64_t r = r0 + g + 8 * t;
+    if (r < rend) {
+        scl[r - base] = (uint16_t)cl;
+        assign[r] = cl;
+        atomicAdd(&hist[cl], 1u);
     }
 }
 
-// cnt[cl] = members of cluster cl
-__global__ void cluster_sizes_kernel(const int32_t *__restrict__ clusters, int64_t n, int c,
-                                     uint32_t *__restrict__ cnt) {
-    extern __shared__ uint32_t hist[];
-    for (int e = threadIdx.x; e < c; e += blockDim.x) hist[e] = 0;
-    __syncthreads();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int cl = clusters[i];
-        if (cl >= 0 && cl < c) atomicAdd(&hist[cl], 1u);
+// bits[cl][u * 32 + b] += rows of one task (up to kTaskRows rows of cluster cl) with bit b of
+// unit u set, for the units of one slice of 32 / R lanes x VEC units: every lane counts its
+// units' bits over its rows in bit planes (BitPlanes), the planes become byte counts, and the
+// warp adds those, 32 consecutive counters at a time, to the global ones.
+template <int VEC>
+__device__ __forceinline__ void count_task(const uint32_t *__restrict__ data, int64_t base,
+                                           const uint16_t *list, int rows, int units, int u0,
+                                           int lanes, uint32_t *flush, uint32_t *bits) {
+    const int lane = threadIdx.x & 31;
+    const int slot = lane / lanes, R = 32 / lanes;
+    const int u = u0 + (lane % lanes) * VEC;
+    const bool in = u < units;  // VEC divides units
+    BitPlanes<VEC> bp;
+    bp.clear();
+    constexpr int N = 8;
+    for (int k = slot; k < rows + slot; k += N * R) {  // same trips in every lane
+        uint32_t x[N][VEC];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const int kk = k + q * R;
+            const bool ok = in && kk < rows;
+            const uint32_t *p = data + (base + (ok ? list[kk] : 0)) * units + u;
+            if constexpr (VEC == 2) {
+                const uint2 y = ok ? *reinterpret_cast<const uint2 *>(p) : make_uint2(0, 0);
+                x[q][0] = y.x, x[q][1] = y.y;
+            } else {
+                x[q][0] = ok ? *p : 0u;
+            }
+        }
+        bp.add8(x);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < c; e += blockDim.x)
-        if (hist[e]) atomicAdd(&cnt[e], hist[e]);
+    // byte counts: word s of unit w holds bits s, s + 8, s + 16, s + 24
+#pragma unroll
+    for (int w = 0; w < VEC; ++w)
+#pragma unroll
+        for (int s = 0; s < 8; ++s) flush[lane * kFlushStride + w * 8 + s] = bp.bytes(w, s);
+    __syncwarp();
+    const int n = min(lanes * VEC, units - u0);
+    for (int w = 0; w < n; ++w) {
+        uint32_t cntb = 0;
+        for (int r = 0; r < R; ++r)
+            cntb += (flush[(r * lanes + w / VEC) * kFlushStride + (w % VEC) * 8 + (lane & 7)] >>
+                     (8 * (lane >> 3))) & 0xffu;
+        if (cntb) atomicAdd(&bits[(int64_t)(u0 + w) * 32 + lane], cntb);
+    }
+    __syncwarp();
+}
+
+// One round over the rows of a tile at a time: clusters (assign_rows), then the tile's rows
+// listed by cluster (a counting sort of row numbers in shared memory), then the set bits of
+// each cluster's rows (count_task).  The reference, and this kernel's predecessor, formed a
+// ballot per bit of every word (200k rows of 32 64-bit words, 16 clusters: 777 us for the
+// two phases); here a word costs ~3 logic operations per 32 bits.
+// Block: 16 warps, one block per SM, tiles of n / SMs rows, so that a cluster's rows of a
+// tile make a task long enough to pay for its flush.
+template <bool V16, int VEC>
+__global__ void __launch_bounds__(kRoundThreads, 1)
+kmeans_round_kernel(const uint32_t *__restrict__ data, int64_t n, const uint32_t *__restrict__ cent,
+                    int c, RoundShape sh, int tile, int32_t *__restrict__ assign,
+                    uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint4 *expanded = reinterpret_cast<uint4 *>(smem);
+    int32_t *pcs = reinterpret_cast<int32_t *>(smem + sh.expanded());
+    uint32_t *hist = reinterpret_cast<uint32_t *>(pcs + 16 * sh.pairs);
+    uint32_t *first = hist + c;       // next list entry of each cluster
+    uint32_t *task0 = first + c;      // first task of each cluster, then the number of tasks
+    uint16_t *scl = reinterpret_cast<uint16_t *>(
+        smem + sh.expanded() + align_up(sizeof(int32_t) * 16 * (size_t)sh.pairs, 16) +
+        align_up(sizeof(uint32_t) * (3 * (size_t)c + 2), 16));
+    uint16_t *list = scl + kTileRows;
+    uint32_t *flush = reinterpret_cast<uint32_t *>(list + kTileRows);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int units = sh.units;
+    grid_dep_wait();
+    grid_dep_release();
+    if (sh.assign) {
+        const int total = sh.pairs * sh.groups * 512;
+        for (int e = threadIdx.x; e < total; e += kRoundThreads) {
+            const int ln = e & 31, s = (e >> 5) & 3, i = (e >> 7) & 3;
+            const int k = (e >> 9) % sh.groups, p = (e >> 9) / sh.groups;
+            const int u = 16 * k + 4 * (ln & 3) + i, j = 16 * p + (ln >> 2);
+            uint32_t x0 = 0, x1 = 0;
+            if (u < units) {
+                if (j < c) x0 = cent[(int64_t)j * units + u];
+                if (j + 8 < c) x1 = cent[(int64_t)(j + 8) * units + u];
+            }
+            auto spread = [](uint32_t x, int b) { return ((x >> b) & 0x01010101u) << (7 - b); };
+            expanded[e] = make_uint4(spread(x0, 2 * s), spread(x0, 2 * s + 1), spread(x1, 2 * s),
+                                     spread(x1, 2 * s + 1));
+        }
+        for (int j = warp; j < 16 * sh.pairs; j += kRoundWarps) {
+            int pc = 0;
+            if (j < c)
+                for (int u = lane; u < units; u += 32) pc += __popc(cent[(int64_t)j * units + u]);
+            pc = __reduce_add_sync(0xffffffffu, pc);
+            if (lane == 0) pcs[j] = pc;
+        }
+    }
+    // lanes of a warp per row in count_task: a power of two that covers the row's units
+    int lanes = 32;
+    while (lanes > 1 && (lanes / 2) * VEC >= units) lanes >>= 1;
+    const int slices = (units + lanes * VEC - 1) / (lanes * VEC);
+    for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
+        const int64_t rend = min(base + tile, n);
+        const int rows = (int)(rend - base);
+        for (int j = threadIdx.x; j < c; j += kRoundThreads) hist[j] = 0;
+        __syncthreads();
+        if (sh.assign) {
+            for (int r = warp * 32; r < rows; r += kRoundThreads)
+                assign_rows<V16>(data, base + r, rend, base, sh, c, expanded, pcs, scl, hist,
+                                 assign);
+        } else {
+            for (int r = threadIdx.x; r < rows; r += kRoundThreads) {
+                const int cl = assign[base + r];
+                scl[r] = (uint16_t)cl;
+                atomicAdd(&hist[cl], 1u);
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {  // list entries and tasks before each cluster
+            uint32_t at = 0, tk = 0;
+            for (int j0 = 0; j0 < c; j0 += 32) {
+                const int j = j0 + lane;
+                const uint32_t h = j < c ? hist[j] : 0u;
+                const uint32_t th = (h + kTaskRows - 1) / kTaskRows;
+                uint32_t ih = h, it = th;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, ih, o);
+                    const uint32_t z = __shfl_up_sync(0xffffffffu, it, o);
+                    if (lane >= o) {
+                        ih += y;
+                        it += z;
+                    }
+                }
+                if (j < c) {
+                    first[j] = at + ih - h;
+                    task0[j] = tk + it - th;
+                }
+                at += __shfl_sync(0xffffffffu, ih, 31);
+                tk += __shfl_sync(0xffffffffu, it, 31);
+            }
+            if (lane == 0) task0[c] = tk;
+        }
+        __syncthreads();
+        for (int r = threadIdx.x; r < rows; r += kRoundThreads)
+            list[atomicAdd(&first[scl[r]], 1u)] = (uint16_t)r;
+        for (int j = threadIdx.x; j < c; j += kRoundThreads)
+            if (hist[j]) atomicAdd(&cnt[j], hist[j]);
+        __syncthreads();  // first[j] is now the end of cluster j's entries
+        const int jobs = (int)task0[c] * slices;
+        for (int job = warp; job < jobs; job += kRoundWarps) {
+            const int tk = job / slices, sl = job % slices;
+            int lo = 0, hi = c - 1;  // the last cluster whose first task is at most tk
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if ((int)task0[mid] <= tk) lo = mid; else hi = mid - 1;
+            }
+            const int part = tk - (int)task0[lo];
+            const int h = (int)hist[lo];
+            count_task<VEC>(data, base, list + (first[lo] - h) + part * kTaskRows,
+                            min(kTaskRows, h - part * kTaskRows), units, sl * lanes * VEC, lanes,
+                            flush + warp * 32 * kFlushStride, bits + (int64_t)lo * units * 32);
+        }
+        __syncthreads();
+    }
 }
 
 // Majority centroids with the reference's per-lane OR accumulation
 // (include/preproc/ibp_preproc_kmeans.cuh:219-236): bit set when count > size/2 (int div).
+// One block per cluster: a warp per word, a lane per bit (coalesced counts, one ballot per
+// 32 bits), then the accumulation over every 32nd word.  The counters are cleared for the
+// next round on the way.
 template <typename U>
-__global__ void majority_kernel(const uint32_t *__restrict__ bits, const uint32_t *__restrict__ cnt,
-                                int64_t v, int c, U *__restrict__ cent) {
+__global__ void __launch_bounds__(256)
+majority_kernel(uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt, int64_t v,
+                U *__restrict__ cent) {
     constexpr int W = 8 * sizeof(U);
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (tid >= (int64_t)c * 32) return;
-    const int cl = (int)(tid / 32), lane = (int)(tid % 32);
-    const uint32_t half = (uint32_t)((int32_t)cnt[cl] / 2);
-    uint64_t acc = 0;
-    for (int64_t id = lane; id < v; id += 32) {
-        const uint32_t *bb = bits + ((int64_t)cl * v + id) * W;
-        for (int b = 0; b < W; ++b)
-            if ((int32_t)bb[b] > (int32_t)half) acc |= 1ull << b;
-        cent[(int64_t)cl * v + id] = (U)acc;
+    grid_dep_wait();
+    grid_dep_release();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t *bb = bits + (int64_t)blockIdx.x * v * W;
+    U *cc = cent + (int64_t)blockIdx.x * v;
+    const int32_t half = (int32_t)cnt[blockIdx.x] / 2;
+    for (int64_t id = warp; id < v; id += 8) {
+        uint64_t m = 0;
+#pragma unroll
+        for (int h = 0; h < W; h += 32) {
+            const bool on = (int32_t)bb[id * W + h + lane] > half;
+            m |= (uint64_t)__ballot_sync(0xffffffffu, on) << h;
+            bb[id * W + h + lane] = 0;
+        }
+        if (lane == 0) cc[id] = (U)m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) cnt[blockIdx.x] = 0;
+    if (threadIdx.x < 32) {
+        U acc = 0;
+        for (int64_t id = threadIdx.x; id < v; id += 32) {
+            acc |= cc[id];
+            cc[id] = acc;
+        }
     }
 }
 
 // Per-cluster masks (include/preproc/ibp_preproc_kmeans.cuh:238-297): counts accumulate in
 // float32 there (saturating at 2^24); `>= thr*count` in float32, `<= (1-thr)*count` in
-// float64; an empty cluster yields all-ones mask and bitval.
+// float64; an empty cluster yields all-ones mask and bitval.  A warp per word, a lane per bit.
 template <typename U>
-__global__ void cluster_masks_kernel(const uint32_t *__restrict__ bits,
-                                     const uint32_t *__restrict__ cnt, int64_t v, int c,
-                                     float thr, U *__restrict__ masks, U *__restrict__ bitvals) {
+__global__ void __launch_bounds__(256)
+cluster_masks_kernel(const uint32_t *__restrict__ bits, const uint32_t *__restrict__ cnt, int64_t v,
+                     int c, float thr, U *__restrict__ masks, U *__restrict__ bitvals) {
     constexpr int W = 8 * sizeof(U);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)c * v;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int cl = (int)(e / v);
-        const int32_t count = (int32_t)cnt[cl];
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = (int64_t)gridDim.x * 8;
+    for (int64_t e = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); e < (int64_t)c * v;
+         e += nwarps) {
+        const int32_t count = (int32_t)cnt[e / v];
         const float lim1 = __fmul_rn(thr, (float)count);
         const double lim0 = __dmul_rn(1.0 - (double)thr, (double)count);
-        const uint32_t *bb = bits + e * W;
         uint64_t m = 0, val = 0;
-        for (int b = 0; b < W; ++b) {
-            const uint32_t bs = bb[b];
+#pragma unroll
+        for (int h = 0; h < W; h += 32) {
+            const uint32_t bs = bits[e * W + h + lane];
             const float bsf = bs > 16777216u ? 16777216.0f : (float)bs;
-            if (bsf >= lim1) {
-                val |= 1ull << b;
-                m |= 1ull << b;
-            } else if ((double)bsf <= lim0) {
-                m |= 1ull << b;
-            }
+            const bool one = bsf >= lim1;
+            const bool inv = one || (double)bsf <= lim0;
+            val |= (uint64_t)__ballot_sync(0xffffffffu, one) << h;
+            m |= (uint64_t)__ballot_sync(0xffffffffu, inv) << h;
         }
-        masks[e] = (U)m;
-        bitvals[e] = (U)val;
+        if (lane == 0) {
+            masks[e] = (U)m;
+            bitvals[e] = (U)val;
+        }
     }
 }
 
@@ -207,13 +461,54 @@ size_t kmeans_workspace(int64_t n, int64_t v, int wb, int c) {
     return s.total();
 }
 
-static int kt_for(int64_t v, int c, int W, size_t &smem) {
-    const size_t budget = 96 * 1024;
-    int64_t kt = (int64_t)(budget / ((size_t)c * W * 4 + 4));
-    if (kt > v) kt = v;
-    if (kt < 1) kt = 1;
-    smem = (size_t)c * ((size_t)kt * W + 1) * 4;
-    return (int)kt;
+// The ten rounds: assignment, counts, and (but for the last round) the next centroids.
+template <typename U>
+static ibp_status kmeans_rounds(const U *rows, int64_t n, int64_t v, int c, U *cent, uint32_t *bits,
+                                uint32_t *cnt, int32_t *assign, cudaStream_t st) {
+    const int sms = device_sm_count();
+    const size_t maxs = (size_t)device_max_smem_optin();
+    RoundShape sh;
+    sh.units = (int)(v * (int64_t)sizeof(U) / 4);
+    sh.groups = (sh.units + 15) / 16;
+    sh.pairs = (c + 15) / 16;
+    sh.assign = true;
+    if (sh.bytes(c) > maxs) sh.assign = false;
+    const size_t smem = sh.bytes(c);
+    const uint32_t *data = reinterpret_cast<const uint32_t *>(rows);
+    const bool v16 = sh.units % 4 == 0 && (((uintptr_t)rows) & 15) == 0;
+    const bool v8 = sh.units % 2 == 0 && (((uintptr_t)rows) & 7) == 0;
+    auto rkern = v16 ? kmeans_round_kernel<true, 2>
+                     : (v8 ? kmeans_round_kernel<false, 2> : kmeans_round_kernel<false, 1>);
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)rkern, kRoundThreads, smem, &per_sm));
+    int64_t tile = ((n + sms - 1) / sms + 31) / 32 * 32;
+    if (tile > kTileRows) tile = kTileRows;
+    const int64_t blocks = std::min<int64_t>((n + tile - 1) / tile, sms);
+    // fallback assignment
+    const size_t cent_bytes = (size_t)c * v * sizeof(U);
+    const bool cent_smem = cent_bytes <= 64 * 1024;
+    auto akern = assign_kernel<U>;
+    if (!sh.assign && cent_smem && cent_bytes > 48 * 1024)
+        IBP_CUDA(cudaFuncSetAttribute(akern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)cent_bytes));
+    const int64_t ablocks = std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)sms * 8));
+    for (int it = 0; it < kKmRounds; ++it) {
+        if (!sh.assign) {
+            akern<<<(unsigned)ablocks, 256, cent_smem ? cent_bytes : 0, st>>>(rows, n, v, cent, c,
+                                                                              cent_smem, assign);
+            IBP_LAUNCHED("assign_kernel");
+        }
+        IBP_CUDA(launch_dependent(rkern, (unsigned)blocks, kRoundThreads, smem, st, data, n,
+                                  reinterpret_cast<const uint32_t *>(cent), c, sh, (int)tile,
+                                  assign, bits, cnt));
+        IBP_LAUNCHED("kmeans_round_kernel");
+        if (it + 1 < kKmRounds) {
+            IBP_CUDA(launch_dependent(majority_kernel<U>, (unsigned)c, 256, 0, st, bits, cnt, v,
+                                      cent));
+            IBP_LAUNCHED("majority_kernel");
+        }
+    }
+    return IBP_OK;
 }
 
 template <typename U>
@@ -251,7 +546,6 @@ ibp_status kmeans_impl(const U *data, int64_t n, int64_t v, int c, const int64_t
     std::vector<int64_t> h(c > 0 ? c : 1, 0);
     for (int64_t i = 1; i < seeded; ++i) h[i] = init_rows[i];
     IBP_CUDA(cudaMemcpyAsync(seed, h.data(), sizeof(int64_t) * c, cudaMemcpyHostToDevice, st));
-    const int sms = device_sm_count();
     {
         int64_t tot = (int64_t)c * v;
         int blocks = (int)std::min<int64_t>((tot + 255) / 256, 1024);
@@ -259,49 +553,21 @@ ibp_status kmeans_impl(const U *data, int64_t n, int64_t v, int c, const int64_t
         IBP_LAUNCHED("seed_centroids_kernel");
     }
     IBP_CUDA(cudaMemsetAsync(assign, 0, sizeof(int32_t) * n, st));
-    if (n == 0) {
-        IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
-        IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * W, st));
+    IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
+    IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * W, st));
+    // the most clusters a call may ask for (894 of 64-bit words, 1760 of 32-bit words)
+    if ((size_t)c * (W + 1) * 4 > (size_t)device_max_smem_optin()) {
+        set_error("preprocess_kmeans: %d clusters do not fit shared memory", c);
+        return IBP_ERR_CUDA;
     }
-    const size_t cent_bytes = (size_t)c * v * wb;
-    const bool cent_smem = cent_bytes <= 64 * 1024;
-    auto akern = assign_kernel<U>;
-    if (cent_smem && cent_bytes > 48 * 1024)
-        IBP_CUDA(cudaFuncSetAttribute(akern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cent_bytes));
-    size_t bsmem = 0;
-    const int kt = kt_for(v, c, W, bsmem);
-    auto bkern = cluster_bits_kernel<U>;
-    if (bsmem > 48 * 1024)
-        IBP_CUDA(cudaFuncSetAttribute(bkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
-    const int64_t tiles = (v + kt - 1) / kt;
-    int64_t gx = (n + 255) / 256;
-    const int64_t capx = std::max<int64_t>(1, (int64_t)sms * 2 / tiles);
-    if (gx > capx) gx = capx;
-    if (gx < 1) gx = 1;
-    int64_t ablocks = std::min<int64_t>((n + 7) / 8, (int64_t)sms * 8);
-    if (ablocks < 1) ablocks = 1;
-    for (int it = 0; it < kKmRounds && n > 0; ++it) {
-        akern<<<(unsigned)ablocks, 256, cent_smem ? cent_bytes : 0, st>>>(rows, n, v, cent, c,
-                                                                          cent_smem, assign);
-        IBP_LAUNCHED("assign_kernel");
-        IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
-        IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * W, st));
-        bkern<<<dim3((unsigned)gx, (unsigned)tiles), 256, bsmem, st>>>(rows, n, v, assign, c,
-                                                                        kt, bits);
-        IBP_LAUNCHED("cluster_bits_kernel");
-        cluster_sizes_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, sms * 4), 256,
-                               sizeof(uint32_t) * c, st>>>(assign, n, c, cnt);
-        IBP_LAUNCHED("cluster_sizes_kernel");
-        majority_kernel<U><<<(c * 32 + 255) / 256, 256, 0, st>>>(bits, cnt, v, c, cent);
-        IBP_LAUNCHED("majority_kernel");
-    }
+    if (n > 0 && v > 0) IBP_RET(kmeans_rounds<U>(rows, n, v, c, cent, bits, cnt, assign, st));
     if (n > 0)
         IBP_CUDA(cudaMemcpyAsync(clusters, assign, sizeof(int32_t) * n, cudaMemcpyDefault, st));
     // the reference's final sweep leaves the masks of its last step, thr = 1.0f
     const ThrList sweep = sweep_thresholds(-1.0f);
     const float last = sweep.v[sweep.count - 1];
     if (c > 0 && v > 0) {
-        int blocks = (int)std::min<int64_t>(((int64_t)c * v + 255) / 256, 1024);
+        int blocks = (int)std::min<int64_t>(((int64_t)c * v + 7) / 8, 4096);
         cluster_masks_kernel<U><<<blocks, 256, 0, st>>>(bits, cnt, v, c, last, masks, bitvals);
         IBP_LAUNCHED("cluster_masks_kernel");
     }
