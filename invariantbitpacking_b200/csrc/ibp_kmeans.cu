@@ -102,33 +102,38 @@ __device__ __forceinline__ void mma_u8(int32_t (&d)[4], const uint32_t (&a)[4], 
 constexpr int kRoundThreads = 512;
 constexpr int kRoundWarps = kRoundThreads / 32;
 constexpr int kTileRows = 4096;   // most rows of a tile (16-bit row numbers in shared memory)
-constexpr int kTaskRows = 255;    // rows a lane's eight bit planes can count
+constexpr int kTaskRows = 128;    // rows of a task (a lane's eight bit planes count to 255)
 constexpr int kFlushStride = 17;  // words per lane of a warp's flush buffer (16 + 1 of padding)
 
 // Shared memory of kmeans_round_kernel: expanded centroids, their set bits, three words per
-// cluster (histogram, first list entry, first task), the tile's clusters and row list, and a
-// flush buffer per warp.
+// list key (entries, first list entry, first task), the tile's new and old clusters and its
+// row list, and a flush buffer per warp.
 struct RoundShape {
     int units;    // 32-bit units per row
     int groups;   // 64-byte groups of a row
     int pairs;    // pairs of 8-centroid tiles
     bool assign;  // false: the clusters are already in `assign`
+    bool fresh;   // every row is added to zero counts; false: only rows that changed cluster
     __host__ __device__ size_t expanded() const { return assign ? (size_t)pairs * groups * 8192 : 0; }
     size_t bytes(int c) const {
         return expanded() + align_up(sizeof(int32_t) * 16 * (size_t)pairs, 16) +
-               align_up(sizeof(uint32_t) * (3 * (size_t)c + 2), 16) + 2 * 2 * (size_t)kTileRows +
+               align_up(sizeof(uint32_t) * (6 * (size_t)c + 2), 16) + 2 * 4 * (size_t)kTileRows +
                sizeof(uint32_t) * 32 * kFlushStride * kRoundWarps;
     }
 };
 
 // Nearest centroids of the 32 rows r0.. (highest centroid on ties), into scl[r - base] and
-// `assign`; hist counts them.  V16: rows are 16-byte aligned.
+// `assign` (and `out`, the caller's copy, in the last round); the clusters they had go to
+// sold[r - base].  hist counts the list entries: key cl for a row added to cluster cl, key
+// c + cl for one taken from it.  V16: rows are 16-byte aligned.
 template <bool V16>
 __device__ __forceinline__ void assign_rows(const uint32_t *__restrict__ data, int64_t r0,
                                             int64_t rend, int64_t base, const RoundShape &sh,
                                             int c, const uint4 *__restrict__ expanded,
                                             const int32_t *__restrict__ pcs, uint16_t *scl,
-                                            uint32_t *hist, int32_t *__restrict__ assign) {
+                                            uint16_t *sold, uint32_t *hist,
+                                            int32_t *__restrict__ assign,
+                                            int32_t *__restrict__ out) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     int bestd[4], bestj[4];
 #pragma unroll
@@ -207,20 +212,27 @@ __device__ __forceinline__ void assign_rows(const uint32_t *__restrict__ data, i
     const int cl = t == 0 ? bestj[0] : (t == 1 ? bestj[1] : (t == 2 ? bestj[2] : bestj[3]));
     const int64_t r = r0 + g + 8 * t;
     if (r < rend) {
+        const int old = sh.fresh ? -1 : assign[r];
         scl[r - base] = (uint16_t)cl;
         assign[r] = cl;
-        atomicAdd(&hist[cl], 1u);
+        if (out) out[r] = cl;
+        if (!sh.fresh) sold[r - base] = (uint16_t)old;
+        if (old != cl) {
+            atomicAdd(&hist[cl], 1u);
+            if (old >= 0) atomicAdd(&hist[c + old], 1u);
+        }
     }
 }
 
-// bits[cl][u * 32 + b] += rows of one task (up to kTaskRows rows of cluster cl) with bit b of
-// unit u set, for the units of one slice of 32 / R lanes x VEC units: every lane counts its
-// units' bits over its rows in bit planes (BitPlanes), the planes become byte counts, and the
-// warp adds those, 32 consecutive counters at a time, to the global ones.
+// bits[u * 32 + b] += (or -=) rows of one task (up to kTaskRows list entries of one key) with
+// bit b of unit u set, for the units of one slice of 32 / R lanes x VEC units: every lane
+// counts its units' bits over its rows in bit planes (BitPlanes), the planes become byte
+// counts, and the warp adds those, 32 consecutive counters at a time, to the global ones.
 template <int VEC>
 __device__ __forceinline__ void count_task(const uint32_t *__restrict__ data, int64_t base,
                                            const uint16_t *list, int rows, int units, int u0,
-                                           int lanes, uint32_t *flush, uint32_t *bits) {
+                                           int lanes, bool minus, uint32_t *flush,
+                                           uint32_t *bits) {
     const int lane = threadIdx.x & 31;
     const int slot = lane / lanes, R = 32 / lanes;
     const int u = u0 + (lane % lanes) * VEC;
@@ -250,40 +262,65 @@ __device__ __forceinline__ void count_task(const uint32_t *__restrict__ data, in
 #pragma unroll
         for (int s = 0; s < 8; ++s) flush[lane * kFlushStride + w * 8 + s] = bp.bytes(w, s);
     __syncwarp();
-    const int n = min(lanes * VEC, units - u0);
-    for (int w = 0; w < n; ++w) {
-        uint32_t cntb = 0;
-        for (int r = 0; r < R; ++r)
-            cntb += (flush[(r * lanes + w / VEC) * kFlushStride + (w % VEC) * 8 + (lane & 7)] >>
-                     (8 * (lane >> 3))) & 0xffu;
-        if (cntb) atomicAdd(&bits[(int64_t)(u0 + w) * 32 + lane], cntb);
+    // lane b adds bit b's counter of each unit (the slots of a unit first, where a warp holds
+    // several rows at once)
+    const int nl = min(lanes, (units - u0) / VEC), sh = 8 * (lane >> 3);
+    const uint32_t *f = flush + (lane & 7);
+    uint32_t *to = bits + (int64_t)u0 * 32 + lane;
+    const uint32_t sign = minus ? ~0u : 1u;
+    auto put = [&](uint32_t count, int unit) {
+        if (count) atomicAdd(to + unit * 32, count * sign);
+    };
+    if (R == 1) {
+#pragma unroll 4
+        for (int l = 0; l < nl; ++l) {
+#pragma unroll
+            for (int w = 0; w < VEC; ++w)
+                put((f[l * kFlushStride + w * 8] >> sh) & 0xffu, l * VEC + w);
+        }
+    } else {
+        for (int l = 0; l < nl; ++l) {
+#pragma unroll
+            for (int w = 0; w < VEC; ++w) {
+                uint32_t count = 0;
+                for (int r = 0; r < R; ++r)
+                    count += (f[(r * lanes + l) * kFlushStride + w * 8] >> sh) & 0xffu;
+                put(count, l * VEC + w);
+            }
+        }
     }
     __syncwarp();
 }
 
 // One round over the rows of a tile at a time: clusters (assign_rows), then the tile's rows
 // listed by cluster (a counting sort of row numbers in shared memory), then the set bits of
-// each cluster's rows (count_task).  The reference, and this kernel's predecessor, formed a
-// ballot per bit of every word (200k rows of 32 64-bit words, 16 clusters: 777 us for the
-// two phases); here a word costs ~3 logic operations per 32 bits.
+// each cluster's rows (count_task).  The counts live on from round to round: after the first
+// only rows that changed cluster are listed, once to add and once to take away (a fifth of
+// the rows in the second round of a 16-cluster mixture, a fiftieth in the last).  The
+// reference issues an atomic per set bit, and this kernel's predecessors formed a ballot per
+// bit of every word (200k rows of 32 64-bit words, 16 clusters: 777 us a round; this kernel 38 us, 12 of them the
+// products at the rate mma.sync reaches, 8 cycles each per scheduler).
 // Block: 16 warps, one block per SM, tiles of n / SMs rows, so that a cluster's rows of a
 // tile make a task long enough to pay for its flush.
 template <bool V16, int VEC>
 __global__ void __launch_bounds__(kRoundThreads, 1)
 kmeans_round_kernel(const uint32_t *__restrict__ data, int64_t n, const uint32_t *__restrict__ cent,
                     int c, RoundShape sh, int tile, int32_t *__restrict__ assign,
-                    uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt) {
+                    int32_t *__restrict__ out, uint32_t *__restrict__ bits,
+                    uint32_t *__restrict__ cnt) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint4 *expanded = reinterpret_cast<uint4 *>(smem);
     int32_t *pcs = reinterpret_cast<int32_t *>(smem + sh.expanded());
     uint32_t *hist = reinterpret_cast<uint32_t *>(pcs + 16 * sh.pairs);
-    uint32_t *first = hist + c;       // next list entry of each cluster
-    uint32_t *task0 = first + c;      // first task of each cluster, then the number of tasks
+    const int keys = sh.fresh ? c : 2 * c;
+    uint32_t *first = hist + keys;   // next list entry of each key
+    uint32_t *task0 = first + keys;  // first task of each key, then the number of tasks
     uint16_t *scl = reinterpret_cast<uint16_t *>(
         smem + sh.expanded() + align_up(sizeof(int32_t) * 16 * (size_t)sh.pairs, 16) +
-        align_up(sizeof(uint32_t) * (3 * (size_t)c + 2), 16));
-    uint16_t *list = scl + kTileRows;
-    uint32_t *flush = reinterpret_cast<uint32_t *>(list + kTileRows);
+        align_up(sizeof(uint32_t) * (6 * (size_t)c + 2), 16));
+    uint16_t *sold = scl + kTileRows;
+    uint16_t *list = sold + kTileRows;
+    uint32_t *flush = reinterpret_cast<uint32_t *>(list + 2 * kTileRows);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int units = sh.units;
     grid_dep_wait();
@@ -318,25 +355,26 @@ kmeans_round_kernel(const uint32_t *__restrict__ data, int64_t n, const uint32_t
     for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
         const int64_t rend = min(base + tile, n);
         const int rows = (int)(rend - base);
-        for (int j = threadIdx.x; j < c; j += kRoundThreads) hist[j] = 0;
+        for (int j = threadIdx.x; j < keys; j += kRoundThreads) hist[j] = 0;
         __syncthreads();
         if (sh.assign) {
             for (int r = warp * 32; r < rows; r += kRoundThreads)
-                assign_rows<V16>(data, base + r, rend, base, sh, c, expanded, pcs, scl, hist,
-                                 assign);
+                assign_rows<V16>(data, base + r, rend, base, sh, c, expanded, pcs, scl, sold,
+                                 hist, assign, out);
         } else {
             for (int r = threadIdx.x; r < rows; r += kRoundThreads) {
                 const int cl = assign[base + r];
                 scl[r] = (uint16_t)cl;
+                if (out) out[base + r] = cl;
                 atomicAdd(&hist[cl], 1u);
             }
         }
         __syncthreads();
-        if (warp == 0) {  // list entries and tasks before each cluster
+        if (warp == 0) {  // list entries and tasks before each key
             uint32_t at = 0, tk = 0;
-            for (int j0 = 0; j0 < c; j0 += 32) {
+            for (int j0 = 0; j0 < keys; j0 += 32) {
                 const int j = j0 + lane;
-                const uint32_t h = j < c ? hist[j] : 0u;
+                const uint32_t h = j < keys ? hist[j] : 0u;
                 const uint32_t th = (h + kTaskRows - 1) / kTaskRows;
                 uint32_t ih = h, it = th;
 #pragma unroll
@@ -348,34 +386,41 @@ kmeans_round_kernel(const uint32_t *__restrict__ data, int64_t n, const uint32_t
                         it += z;
                     }
                 }
-                if (j < c) {
+                if (j < keys) {
                     first[j] = at + ih - h;
                     task0[j] = tk + it - th;
                 }
                 at += __shfl_sync(0xffffffffu, ih, 31);
                 tk += __shfl_sync(0xffffffffu, it, 31);
             }
-            if (lane == 0) task0[c] = tk;
+            if (lane == 0) task0[keys] = tk;
         }
         __syncthreads();
-        for (int r = threadIdx.x; r < rows; r += kRoundThreads)
-            list[atomicAdd(&first[scl[r]], 1u)] = (uint16_t)r;
-        for (int j = threadIdx.x; j < c; j += kRoundThreads)
-            if (hist[j]) atomicAdd(&cnt[j], hist[j]);
-        __syncthreads();  // first[j] is now the end of cluster j's entries
-        const int jobs = (int)task0[c] * slices;
+        for (int r = threadIdx.x; r < rows; r += kRoundThreads) {
+            const int cl = scl[r];
+            if (sh.fresh || sold[r] != cl) {
+                list[atomicAdd(&first[cl], 1u)] = (uint16_t)r;
+                if (!sh.fresh) list[atomicAdd(&first[c + sold[r]], 1u)] = (uint16_t)r;
+            }
+        }
+        for (int j = threadIdx.x; j < keys; j += kRoundThreads)
+            if (hist[j]) atomicAdd(&cnt[j < c ? j : j - c], j < c ? hist[j] : 0u - hist[j]);
+        __syncthreads();  // first[j] is now the end of key j's entries
+        const int jobs = (int)task0[keys] * slices;
         for (int job = warp; job < jobs; job += kRoundWarps) {
             const int tk = job / slices, sl = job % slices;
-            int lo = 0, hi = c - 1;  // the last cluster whose first task is at most tk
+            int lo = 0, hi = keys - 1;  // the last key whose first task is at most tk
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
                 if ((int)task0[mid] <= tk) lo = mid; else hi = mid - 1;
             }
             const int part = tk - (int)task0[lo];
             const int h = (int)hist[lo];
+            const bool minus = lo >= c;
             count_task<VEC>(data, base, list + (first[lo] - h) + part * kTaskRows,
                             min(kTaskRows, h - part * kTaskRows), units, sl * lanes * VEC, lanes,
-                            flush + warp * 32 * kFlushStride, bits + (int64_t)lo * units * 32);
+                            minus, flush + warp * 32 * kFlushStride,
+                            bits + (int64_t)(minus ? lo - c : lo) * units * 32);
         }
         __syncthreads();
     }
@@ -384,17 +429,16 @@ kmeans_round_kernel(const uint32_t *__restrict__ data, int64_t n, const uint32_t
 // Majority centroids with the reference's per-lane OR accumulation
 // (include/preproc/ibp_preproc_kmeans.cuh:219-236): bit set when count > size/2 (int div).
 // One block per cluster: a warp per word, a lane per bit (coalesced counts, one ballot per
-// 32 bits), then the accumulation over every 32nd word.  The counters are cleared for the
-// next round on the way.
+// 32 bits), then the accumulation over every 32nd word.
 template <typename U>
 __global__ void __launch_bounds__(256)
-majority_kernel(uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt, int64_t v,
+majority_kernel(const uint32_t *__restrict__ bits, const uint32_t *__restrict__ cnt, int64_t v,
                 U *__restrict__ cent) {
     constexpr int W = 8 * sizeof(U);
     grid_dep_wait();
     grid_dep_release();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *bb = bits + (int64_t)blockIdx.x * v * W;
+    const uint32_t *bb = bits + (int64_t)blockIdx.x * v * W;
     U *cc = cent + (int64_t)blockIdx.x * v;
     const int32_t half = (int32_t)cnt[blockIdx.x] / 2;
     for (int64_t id = warp; id < v; id += 8) {
@@ -403,12 +447,10 @@ majority_kernel(uint32_t *__restrict__ bits, uint32_t *__restrict__ cnt, int64_t
         for (int h = 0; h < W; h += 32) {
             const bool on = (int32_t)bb[id * W + h + lane] > half;
             m |= (uint64_t)__ballot_sync(0xffffffffu, on) << h;
-            bb[id * W + h + lane] = 0;
         }
         if (lane == 0) cc[id] = (U)m;
     }
     __syncthreads();
-    if (threadIdx.x == 0) cnt[blockIdx.x] = 0;
     if (threadIdx.x < 32) {
         U acc = 0;
         for (int64_t id = threadIdx.x; id < v; id += 32) {
@@ -464,14 +506,15 @@ size_t kmeans_workspace(int64_t n, int64_t v, int wb, int c) {
 // The ten rounds: assignment, counts, and (but for the last round) the next centroids.
 template <typename U>
 static ibp_status kmeans_rounds(const U *rows, int64_t n, int64_t v, int c, U *cent, uint32_t *bits,
-                                uint32_t *cnt, int32_t *assign, cudaStream_t st) {
+                                uint32_t *cnt, int32_t *assign, int32_t *clusters,
+                                cudaStream_t st) {
     const int sms = device_sm_count();
     const size_t maxs = (size_t)device_max_smem_optin();
     RoundShape sh;
     sh.units = (int)(v * (int64_t)sizeof(U) / 4);
     sh.groups = (sh.units + 15) / 16;
     sh.pairs = (c + 15) / 16;
-    sh.assign = true;
+    sh.assign = sh.fresh = true;
     if (sh.bytes(c) > maxs) sh.assign = false;
     const size_t smem = sh.bytes(c);
     const uint32_t *data = reinterpret_cast<const uint32_t *>(rows);
@@ -493,6 +536,12 @@ static ibp_status kmeans_rounds(const U *rows, int64_t n, int64_t v, int c, U *c
                                       (int)cent_bytes));
     const int64_t ablocks = std::max<int64_t>(1, std::min<int64_t>((n + 7) / 8, (int64_t)sms * 8));
     for (int it = 0; it < kKmRounds; ++it) {
+        const bool last = it + 1 == kKmRounds;
+        sh.fresh = it == 0 || !sh.assign;
+        if (sh.fresh) {
+            IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
+            IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * 8 * sizeof(U), st));
+        }
         if (!sh.assign) {
             akern<<<(unsigned)ablocks, 256, cent_smem ? cent_bytes : 0, st>>>(rows, n, v, cent, c,
                                                                               cent_smem, assign);
@@ -500,9 +549,9 @@ static ibp_status kmeans_rounds(const U *rows, int64_t n, int64_t v, int c, U *c
         }
         IBP_CUDA(launch_dependent(rkern, (unsigned)blocks, kRoundThreads, smem, st, data, n,
                                   reinterpret_cast<const uint32_t *>(cent), c, sh, (int)tile,
-                                  assign, bits, cnt));
+                                  assign, last ? clusters : nullptr, bits, cnt));
         IBP_LAUNCHED("kmeans_round_kernel");
-        if (it + 1 < kKmRounds) {
+        if (!last) {
             IBP_CUDA(launch_dependent(majority_kernel<U>, (unsigned)c, 256, 0, st, bits, cnt, v,
                                       cent));
             IBP_LAUNCHED("majority_kernel");
@@ -552,17 +601,17 @@ ibp_status kmeans_impl(const U *data, int64_t n, int64_t v, int c, const int64_t
         seed_centroids_kernel<U><<<blocks, 256, 0, st>>>(rows, n, v, seed, c, cent, status);
         IBP_LAUNCHED("seed_centroids_kernel");
     }
-    IBP_CUDA(cudaMemsetAsync(assign, 0, sizeof(int32_t) * n, st));
-    IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
-    IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * W, st));
+    if (n == 0) {
+        IBP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * c, st));
+        IBP_CUDA(cudaMemsetAsync(bits, 0, sizeof(uint32_t) * c * v * W, st));
+    }
     // the most clusters a call may ask for (894 of 64-bit words, 1760 of 32-bit words)
     if ((size_t)c * (W + 1) * 4 > (size_t)device_max_smem_optin()) {
         set_error("preprocess_kmeans: %d clusters do not fit shared memory", c);
         return IBP_ERR_CUDA;
     }
-    if (n > 0 && v > 0) IBP_RET(kmeans_rounds<U>(rows, n, v, c, cent, bits, cnt, assign, st));
-    if (n > 0)
-        IBP_CUDA(cudaMemcpyAsync(clusters, assign, sizeof(int32_t) * n, cudaMemcpyDefault, st));
+    if (n > 0 && v > 0)
+        IBP_RET(kmeans_rounds<U>(rows, n, v, c, cent, bits, cnt, assign, clusters, st));
     // the reference's final sweep leaves the masks of its last step, thr = 1.0f
     const ThrList sweep = sweep_thresholds(-1.0f);
     const float last = sweep.v[sweep.count - 1];

@@ -132,7 +132,7 @@ def preprocess_kmeans(dataset, num_clusters, threshold_=None, *, seed_rows=None)
     with torch.cuda.device(dev):
         masks = torch.empty((c, v), dtype=_INT_DTYPE[wb], device=dev)
         bitvals = torch.empty((c, v), dtype=_INT_DTYPE[wb], device=dev)
-        clusters = torch.zeros(n, dtype=torch.int32, pin_memory=True)
+        clusters = torch.empty(n, dtype=torch.int32, pin_memory=True)  # every entry is written
         need = _lib.ibp_preprocess_kmeans_workspace_size(n, v, wb, c)
         if dataset.device.type != "cuda" and _stage_budget(n * v * wb, dev):
             need += (n * v * wb + 255) // 256 * 256
