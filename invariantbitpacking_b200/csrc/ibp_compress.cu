@@ -3,9 +3,9 @@
 // (packer and its launchers) and the size/offset glue of src/compress.cu.
 //
 // B200 design
-//  * sizes: G lanes per row (G = 8/16/32 by row length), a branch-free popc sum and
-//    a shuffle reduction; no shared-memory atomics (the reference uses one 256-thread
-//    block per row with smem atomics).
+//  * sizes: 8 or 32 lanes per row, 16 bytes a lane where rows allow it, 8 rows in flight, the
+//    columns' tables in registers; no shared-memory atomics (the reference uses one
+//    256-thread block per row with smem atomics).
 //  * packing: one warp per row.  The row is staged in shared memory once (so in-place
 //    compression of a pinned host row reads it over PCIe once), every lane gathers its
 //    word's non-invariant bits with the Hacker's Delight move masks, a warp prefix sum
@@ -16,44 +16,87 @@
 //    thereby blocks the host).
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+
 #include "ibp_codec.cuh"
 #include "ibp_internal.cuh"
+#include "ibp_match.cuh"
 
 namespace ibp200 {
 
 // ------------------------------------------------------------------ sizes
-template <typename U, int G>
-__global__ void __launch_bounds__(256)
+// Bound: reading the rows.  G lanes share a row (8, 16 or 32 by its chunks of A bytes) and
+// take 8 rows at a time, all loads before any use, so a warp has up to 4 KiB in
+// flight; the columns' mask, values and set bits stay in registers, loaded once when a group
+// covers the row and once per 8 rows when it does not (1M rows of 128 16-bit words: 239 us
+// with a 2-byte load and two table loads a word, 103 with half the lanes idle, 51 now, 5.2 TB/s).
+constexpr int kSizeRows = 8;
+
+template <typename U, int A, int G, bool INDEX>
+__global__ void __launch_bounds__(256, 2)
 compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
                      const U *__restrict__ mask, const U *__restrict__ bitval,
                      const int64_t *__restrict__ idx, int64_t nrows,
                      int64_t *__restrict__ sizes, unsigned long long *__restrict__ total,
-                     int32_t *__restrict__ status) {
-    // groups of G lanes; the row loop advances a whole warp at a time so every lane
-    // reaches the shuffles of every iteration
-    constexpr int RPW = 32 / G;
-    const int sub = threadIdx.x & (G - 1);
-    const int gin = (threadIdx.x & 31) / G;
+                     int32_t *__restrict__ status, uint32_t one) {
+    using C = Chunk<U, A>;
+    constexpr int RPW = 32 / G, Q = kSizeRows;
+    __shared__ unsigned long long block_sum;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), gin = lane / G;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t row_bytes = v * (int64_t)sizeof(U);
+    const int64_t chunks = row_bytes / A;
+    if (threadIdx.x == 0) block_sum = 0;
+    __syncthreads();
     unsigned long long acc = 0;
-    for (int64_t wbase = warp * RPW; wbase < nrows; wbase += nwarps * RPW) {
-        const int64_t i = wbase + gin;
-        const bool live = i < nrows;
-        const int64_t r = live ? (idx ? idx[i] : i) : 0;
-        const bool ok = live && r >= 0 && r < n;
-        uint32_t s = 0;
-        if (ok) {
-            const U *row = data + r * v;
-            for (int64_t j = sub; j < v; j += G) {
-                const U m = __ldg(&mask[j]);
-                if ((U)(row[j] & m) == __ldg(&bitval[j])) s += popc_w(m);
+    uint32_t m[C::NR], b[C::NR], pc[C::NW];
+    auto tables = [&](int64_t c) {
+        C::load_words(mask + c * (A / (int)sizeof(U)), m);
+        C::load_words(bitval + c * (A / (int)sizeof(U)), b);
+        C::set_bits(m, pc);
+    };
+    const bool once = chunks <= G;
+    if (once && sub < chunks) tables(sub);
+    for (int64_t base = warp * RPW * Q; base < nrows; base += nwarps * RPW * Q) {
+        // positions i0 + q * RPW; consecutive rows without an index
+        const int64_t i0 = base + gin;
+        const char *row[INDEX ? Q : 1];
+        unsigned okm = 0;
+        if constexpr (INDEX) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int64_t r = i0 + q * RPW < nrows ? idx[i0 + q * RPW] : -1;
+                const bool ok = r >= 0 && r < n;
+                okm |= (unsigned)ok << q;
+                row[q] = reinterpret_cast<const char *>(data) + (ok ? r : 0) * row_bytes;
             }
+        } else {
+            row[0] = reinterpret_cast<const char *>(data) + i0 * row_bytes;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) okm |= (unsigned)(i0 + q * RPW < nrows) << q;
         }
-        s = group_sum<G>(s);
-        if (sub == 0 && live) {
-            if (ok) {
-                const int64_t sz = compressed_bytes(v, (int)sizeof(U), s);
+        uint32_t s[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) s[q] = 0;
+        for (int64_t c = sub; c < chunks; c += G) {
+            uint32_t x[Q][C::NR];
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if ((okm >> q) & 1)
+                    C::load((INDEX ? row[INDEX ? q : 0] : row[0] + q * RPW * row_bytes) + c * A, x[q]);
+            if (!once) tables(c);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if ((okm >> q) & 1)
+                    C::matched(s[q], [&](int k) { return (x[q][k] & m[k]) ^ b[k]; }, pc, one);
+        }
+        group_sums<Q, G>(s, one);
+        const int q = group_sums_value<Q, G>(sub);
+        const int64_t i = base + q * RPW + gin;
+        if ((sub & (group_sums_copies<Q, G>() - 1)) == 0 && i < nrows) {
+            if ((okm >> q) & 1) {
+                const int64_t sz = compressed_bytes(v, (int)sizeof(U), s[0]);
                 sizes[i] = sz;
                 acc += (unsigned long long)sz;
             } else {
@@ -64,21 +107,34 @@ compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
     }
     if (total) {
         acc = group_sum<32>(acc);
-        if ((threadIdx.x & 31) == 0 && acc) atomicAdd(total, acc);
+        if (lane == 0 && acc) atomicAdd(&block_sum, acc);
+        __syncthreads();
+        if (threadIdx.x == 0 && block_sum) atomicAdd(total, block_sum);
     }
 }
 
-template <typename U, int G>
+template <typename U, int A>
 static ibp_status launch_sizes(const U *data, int64_t n, int64_t v, const U *mask,
                                const U *bitval, const int64_t *idx, int64_t nrows,
                                int64_t *sizes, int64_t *total, int32_t *status,
                                cudaStream_t st) {
-    const int rows_per_block = 256 / G;
-    int64_t blocks = (nrows + rows_per_block - 1) / rows_per_block;
-    const int64_t cap = (int64_t)device_sm_count() * 8;
-    if (blocks > cap) blocks = cap;
-    compress_size_kernel<U, G><<<(unsigned)blocks, 256, 0, st>>>(
-        data, n, v, mask, bitval, idx, nrows, sizes, (unsigned long long *)total, status);
+    const int64_t chunks = v * (int64_t)sizeof(U) / A;
+    auto kern = idx ? compress_size_kernel<U, A, 32, true> : compress_size_kernel<U, A, 32, false>;
+    int lanes = 32;
+    if (chunks <= 8) {
+        kern = idx ? compress_size_kernel<U, A, 8, true> : compress_size_kernel<U, A, 8, false>;
+        lanes = 8;
+    } else if (chunks <= 16) {
+        kern = idx ? compress_size_kernel<U, A, 16, true> : compress_size_kernel<U, A, 16, false>;
+        lanes = 16;
+    }
+    const int64_t per_block = 8 * kSizeRows * (32 / lanes);
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, 256, 0, &per_sm));
+    const int64_t blocks = std::min<int64_t>((nrows + per_block - 1) / per_block,
+                                             (int64_t)device_sm_count() * per_sm);
+    kern<<<(unsigned)blocks, 256, 0, st>>>(data, n, v, mask, bitval, idx, nrows, sizes,
+                                           (unsigned long long *)total, status, 1u);
     IBP_LAUNCHED("compress_size_kernel");
     return IBP_OK;
 }
@@ -89,9 +145,15 @@ ibp_status compress_size_impl(const U *data, int64_t n, int64_t v, const U *mask
                               int64_t *sizes, int64_t *total, int32_t *status,
                               cudaStream_t st) {
     if (nrows <= 0) return IBP_OK;
-    if (v >= 32) return launch_sizes<U, 32>(data, n, v, mask, bitval, idx, nrows, sizes, total, status, st);
-    if (v >= 16) return launch_sizes<U, 16>(data, n, v, mask, bitval, idx, nrows, sizes, total, status, st);
-    return launch_sizes<U, 8>(data, n, v, mask, bitval, idx, nrows, sizes, total, status, st);
+    const int a = row_chunk_bytes(data, v, sizeof(U));
+    if (a == 16)
+        return launch_sizes<U, 16>(data, n, v, mask, bitval, idx, nrows, sizes, total, status, st);
+    if constexpr (sizeof(U) < 4)
+        if (a == 4)
+            return launch_sizes<U, 4>(data, n, v, mask, bitval, idx, nrows, sizes, total, status,
+                                      st);
+    return launch_sizes<U, sizeof(U)>(data, n, v, mask, bitval, idx, nrows, sizes, total, status,
+                                      st);
 }
 
 // ------------------------------------------------------------------ packing

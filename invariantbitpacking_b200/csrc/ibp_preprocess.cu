@@ -3,183 +3,322 @@
 // include/preproc/ibp_preproc_kernels.cuh:7-77).
 //
 // B200 design
-//  * census: each thread owns one word column and keeps 8 bit-sliced vertical counters
-//    (a ripple-carry adder in registers, 16 logic ops per word) that it flushes into
-//    per-thread shared-memory counters every 255 rows; one global atomic per
-//    (column, bit) per block at the end.  Reads are coalesced 32-word row slices.
-//    A host-resident dataset is optionally staged into HBM during this pass so the
-//    second pass reads HBM instead of PCIe.
+//  * census: rows are taken in 16-byte pieces whatever the word size (a group of up to 16 rows
+//    is a whole number of them), each thread counting the set bits of one piece's positions in
+//    bit planes (ibp_bitcount.cuh), 8 pieces in flight; shared counters per block, one global
+//    atomic per (position, block) at the end.  A host-resident dataset is optionally staged
+//    into HBM during this pass so the second pass reads HBM instead of PCIe.
 //  * all sweep thresholds are checked in ONE pass over the data (the reference makes one
 //    PCIe pass and one host round trip per threshold) and the winning mask is selected
 //    by a one-block kernel, so preprocess never blocks the host.
+#include <algorithm>
+
+#include "ibp_bitcount.cuh"
 #include "ibp_common.cuh"
 #include "ibp_internal.cuh"
+#include "ibp_match.cuh"
 
 namespace ibp200 {
 
 constexpr int kCensusThreads = 256;
-constexpr int kCensusDepth = 8;  // bit-sliced counter levels: flush every 255 rows
+constexpr int kCensusCols = 64;   // most 16-byte pieces a block covers side by side
 
-template <typename U>
-using Reg = typename std::conditional<(sizeof(U) < 4), uint32_t, U>::type;
-
-// counts[col * W + b] += number of rows whose word `col` has bit b set.
-// Block (bx, tile) covers columns [tile*cpb, tile*cpb + cpb) and rows bx*R + r_local + k*gx*R.
-template <typename U>
-__global__ void __launch_bounds__(kCensusThreads)
-census_kernel(const U *__restrict__ data, int64_t n, int64_t v, int cpb, int R,
-              uint32_t *__restrict__ counts, U *__restrict__ stage) {
-    constexpr int W = WordBits<U>::value;
-    extern __shared__ uint32_t sc[];  // [W][kCensusThreads]
-    const int t = threadIdx.x;
-    const int c_local = t % cpb, r_local = t / cpb;
-    const int64_t col = (int64_t)blockIdx.y * cpb + c_local;
-    const bool active = (r_local < R) && (col < v);
-    for (int b = 0; b < W; ++b) sc[b * kCensusThreads + t] = 0;
-
-    Reg<U> s[kCensusDepth];
-#pragma unroll
-    for (int d = 0; d < kCensusDepth; ++d) s[d] = 0;
-
-    auto flush = [&]() {
-#pragma unroll
-        for (int b = 0; b < W; ++b) {
-            uint32_t c = 0;
-#pragma unroll
-            for (int d = 0; d < kCensusDepth; ++d) c |= (uint32_t)((s[d] >> b) & 1u) << d;
-            sc[b * kCensusThreads + t] += c;
-        }
-#pragma unroll
-        for (int d = 0; d < kCensusDepth; ++d) s[d] = 0;
-    };
-    auto add = [&](Reg<U> x) {
-#pragma unroll
-        for (int d = 0; d < kCensusDepth; ++d) {
-            Reg<U> carry = s[d] & x;
-            s[d] ^= x;
-            x = carry;
-        }
-    };
-
-    if (active) {
-        const int64_t rstride = (int64_t)gridDim.x * R;
-        int64_t r = (int64_t)blockIdx.x * R + r_local;
+// counts[p] += rows whose bit p (word p / W, bit p % W) is set, over groups of k rows that
+// make up `pieces` 16-byte pieces each (bit p of a group is bit p % row_bits of a row).
+// Block bx * tiles + tile covers pieces [tile * cpb, tile * cpb + cpb) of every group; the R =
+// kCensusThreads / cpb row slots of a tile's blocks take the groups in turn.
+// Bound: HBM (600k rows of 512 bytes: 126 -> 54 us, 5.7 TB/s; a thread per word, a
+// ripple-carry add into 8 planes and 64 KiB of counters per block before).
+__global__ void __launch_bounds__(kCensusThreads, 2)
+census_kernel(const uint4 *__restrict__ data, int64_t groups, int64_t pieces, int cpb, int tiles,
+              int64_t row_bits, bool folded, uint32_t *__restrict__ counts,
+              uint4 *__restrict__ stage) {
+    extern __shared__ uint32_t sc[];  // [128][cpb | 1]
+    const int stride = cpb | 1;
+    const int R = kCensusThreads / cpb;
+    const int c = threadIdx.x % cpb, slot = threadIdx.x / cpb;
+    const int64_t col0 = (int64_t)(blockIdx.x % tiles) * cpb, col = col0 + c;
+    for (int e = threadIdx.x; e < 128 * stride; e += kCensusThreads) sc[e] = 0;
+    __syncthreads();
+    BitPlanes<4> bp;
+    bp.clear();
+    if (slot < R && col < pieces) {
+        const int64_t rstride = (int64_t)(gridDim.x / tiles) * R;
         int pending = 0;
-        constexpr int UNR = 4;
-        for (; r + (UNR - 1) * rstride < n; r += UNR * rstride) {
-            U x[UNR];
+        constexpr int N = 8;
+        for (int64_t r = (int64_t)(blockIdx.x / tiles) * R + slot; r < groups; r += N * rstride) {
+            uint32_t x[N][4];
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) x[u] = data[(r + u * rstride) * v + col];
-#pragma unroll
-            for (int u = 0; u < UNR; ++u) {
-                if (stage) stage[(r + u * rstride) * v + col] = x[u];
-                add((Reg<U>)x[u]);
+            for (int q = 0; q < N; ++q) {
+                const int64_t rr = r + q * rstride;
+                uint4 y = make_uint4(0, 0, 0, 0);
+                if (rr < groups) y = data[rr * pieces + col];
+                x[q][0] = y.x, x[q][1] = y.y, x[q][2] = y.z, x[q][3] = y.w;
             }
-            pending += UNR;
-            if (pending > 255 - UNR) {
-                flush();
+            if (stage) {
+#pragma unroll
+                for (int q = 0; q < N; ++q)
+                    if (r + q * rstride < groups)
+                        stage[(r + q * rstride) * pieces + col] =
+                            make_uint4(x[q][0], x[q][1], x[q][2], x[q][3]);
+            }
+            bp.add8(x);
+            pending += N;
+            if (pending > 255 - N || r + N * rstride >= groups) {  // full, or the last rows
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+#pragma unroll 1
+                    for (int s = 0; s < 8; ++s) {
+                        const uint32_t y = bp.bytes(w, s);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            atomicAdd(&sc[(w * 32 + s + 8 * q) * stride + c], (y >> (8 * q)) & 0xffu);
+                    }
+                }
+                bp.clear();
                 pending = 0;
             }
         }
-        for (; r < n; r += rstride) {
-            U x = data[r * v + col];
-            if (stage) stage[r * v + col] = x;
-            add((Reg<U>)x);
-            if (++pending == 255) {
-                flush();
-                pending = 0;
-            }
-        }
-        flush();
     }
     __syncthreads();
-    // reduce the R row slots of each column, one global atomic per (column, bit)
-    if (r_local == 0 && col < v) {
+    for (int e = threadIdx.x; e < 128 * cpb; e += kCensusThreads) {
+        const int cc = e >> 7, b = e & 127;  // consecutive threads: consecutive positions
+        const int64_t piece = col0 + cc;
+        const uint32_t x = sc[b * stride + cc];
+        if (piece < pieces && x) {
+            const int64_t p = piece * 128 + b;
+            atomicAdd(&counts[folded ? p % row_bits : p], x);
+        }
+    }
+}
+
+// The rows the 16-byte pieces leave over (fewer than a group), or all of them when the dataset
+// does not start on a 16-byte boundary: a thread per word and 32 rows, an atomic per set bit.
+template <typename U>
+__global__ void __launch_bounds__(kCensusThreads)
+census_rest_kernel(const U *__restrict__ data, int64_t n, int64_t v, uint32_t *__restrict__ counts,
+                   U *__restrict__ stage) {
+    constexpr int W = WordBits<U>::value;
+    const int64_t total = (n + 31) / 32 * v;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t col = e % v, r0 = e / v * 32;
+        const int rows = (int)min((int64_t)32, n - r0);
+        BitPlanes<sizeof(U) == 8 ? 2 : 1> bp;
+        bp.clear();
+        for (int r = 0; r < rows; r += 8) {
+            uint32_t x[8][sizeof(U) == 8 ? 2 : 1];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const bool in = r + q < rows;
+                const U y = in ? data[(r0 + r + q) * v + col] : (U)0;
+                if (in && stage) stage[(r0 + r + q) * v + col] = y;
+                x[q][0] = (uint32_t)y;
+                if constexpr (sizeof(U) == 8) x[q][1] = (uint32_t)(y >> 32);
+            }
+            bp.add8(x);
+        }
+#pragma unroll
         for (int b = 0; b < W; ++b) {
-            uint32_t tot = 0;
-            for (int k = 0; k < R; ++k) tot += sc[b * kCensusThreads + t + k * cpb];
-            if (tot) atomicAdd(&counts[col * W + b], tot);
+            const uint32_t x = (bp.bytes(b / 32, b % 8) >> (8 * (b % 32 / 8))) & 0xffu;
+            if (x) atomicAdd(&counts[col * W + b], x);
         }
     }
 }
 
 // One mask/bitval pair per threshold: include/preproc/ibp_preproc_kernels.cuh:33-51.
 // `count > thr * N` is a float32 product and compare, `count < (1 - thr) * N` float64.
+// A lane per bit: 32 consecutive counts make 4 bytes of every mask with two ballots.
 template <typename U>
-__global__ void masks_from_counts_kernel(const uint32_t *__restrict__ counts, int64_t n,
-                                         int64_t v, ThrList thr, U *__restrict__ masks,
-                                         U *__restrict__ bitvals) {
-    constexpr int W = WordBits<U>::value;
-    const int64_t total = v * thr.count;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int ti = (int)(e / v);
-        const int64_t j = e % v;
-        const float t = thr.v[ti];
-        const float lim1 = __fmul_rn(t, (float)(unsigned long long)n);
-        const double lim0 = __dmul_rn(1.0 - (double)t, (double)(unsigned long long)n);
-        uint64_t m = 0, val = 0;
-        for (int b = 0; b < W; ++b) {
-            const int32_t c = (int32_t)counts[j * W + b];
-            if ((float)c > lim1) {
-                val |= 1ull << b;
-                m |= 1ull << b;
-            } else if ((double)c < lim0) {
-                m |= 1ull << b;
+__global__ void __launch_bounds__(256)
+masks_from_counts_kernel(const uint32_t *__restrict__ counts, int64_t n, int64_t v, ThrList thr,
+                         U *__restrict__ masks, U *__restrict__ bitvals) {
+    grid_dep_wait();
+    grid_dep_release();
+    const int lane = threadIdx.x & 31;
+    const int64_t bits = v * WordBits<U>::value, row_bytes = v * (int64_t)sizeof(U);
+    const int64_t nwarps = (int64_t)gridDim.x * 8;
+    for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g * 32 < bits; g += nwarps) {
+        const bool in = g * 32 + lane < bits;
+        const int32_t c = in ? (int32_t)counts[g * 32 + lane] : 0;
+        for (int t = 0; t < thr.count; ++t) {
+            const float lim1 = __fmul_rn(thr.v[t], (float)(unsigned long long)n);
+            const double lim0 =
+                __dmul_rn(1.0 - (double)thr.v[t], (double)(unsigned long long)n);
+            const bool one = (float)c > lim1;
+            const unsigned val = __ballot_sync(0xffffffffu, in && one);
+            const unsigned m = __ballot_sync(0xffffffffu, in && (one || (double)c < lim0));
+            const int64_t at = g * 4 + lane;
+            if (lane < 4 && at < row_bytes) {
+                reinterpret_cast<uint8_t *>(masks)[t * row_bytes + at] = (uint8_t)(m >> (8 * lane));
+                reinterpret_cast<uint8_t *>(bitvals)[t * row_bytes + at] =
+                    (uint8_t)(val >> (8 * lane));
             }
         }
-        masks[e] = (U)m;
-        bitvals[e] = (U)val;
     }
 }
 
 // saved[t] += sum over rows of max(0, S_t(row) - v), S_t = sum of popc(mask_t[j]) over the
 // words with (x & mask_t[j]) == bitval_t[j]: include/preproc/ibp_preproc_kernels.cuh:53-77,
-// for every threshold of the sweep in one pass.  One warp per row.
-template <typename U>
-__global__ void __launch_bounds__(256)
+// for every threshold of the sweep in one pass (T == 7), or for one threshold (T == 1).
+// In the sweep the masks are nested: thr * N rises and (1 - thr) * N falls with thr, so a bit
+// invariant at one threshold is so at every lower one, with the same value (all thresholds are
+// above one half); a word matches at threshold t exactly when (x ^ bitval_0) & mask_t is 0.
+// Rows as in the size pass (G lanes, chunks of A bytes, Q rows in flight), tables in registers.
+// PACK: S_t of a row fits 16 bits, two thresholds to a register in the sums over lanes.
+// Bound: the integer pipe, 3 operations per word and threshold there and one on the
+// multiply-add pipe (600k rows of 64 64-bit words, 7 thresholds: 550 us with 14 table loads per
+// word, 119 with the adds on the integer pipe as well, 100 now, 3.1 TB/s).
+template <typename U, int A, int G, int T, bool PACK>
+__global__ void __launch_bounds__(256, 2)
 check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
                    const U *__restrict__ masks, const U *__restrict__ bitvals,
-                   unsigned long long *__restrict__ saved) {
+                   unsigned long long *__restrict__ saved, uint32_t one) {
+    using C = Chunk<U, A>;
+    constexpr int RPW = 32 / G;
+    constexpr int Q = T > 1 ? 4 : 8;
+    constexpr int S = T > 1 ? (PACK ? 4 : 8) : 1;  // sums per row
+    constexpr int L = Q * S > G ? Q * S / G : 1;   // sums a lane ends with
     __shared__ unsigned long long blk[kMaxThresholds];
     if (threadIdx.x < kMaxThresholds) blk[threadIdx.x] = 0;
     __syncthreads();
-    const int lane = threadIdx.x & 31;
+    grid_dep_wait();
+    grid_dep_release();
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), gin = lane / G;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    unsigned long long acc[kMaxThresholds];
+    const int64_t row_bytes = v * (int64_t)sizeof(U);
+    const int64_t chunks = row_bytes / A;
+    uint32_t b[C::NR], m[T][C::NR], pc[T][C::NW];
+    auto tables = [&](int64_t c) {
+        C::load_words(bitvals + c * (A / (int)sizeof(U)), b);
 #pragma unroll
-    for (int t = 0; t < kMaxThresholds; ++t) acc[t] = 0;
-    for (int64_t r = warp; r < n; r += nwarps) {
-        uint32_t s[kMaxThresholds];
+        for (int t = 0; t < T; ++t) {
+            if (t < nthr) {
+                C::load_words(masks + t * v + c * (A / (int)sizeof(U)), m[t]);
+            } else {
 #pragma unroll
-        for (int t = 0; t < kMaxThresholds; ++t) s[t] = 0;
-        const U *row = data + r * v;
-        for (int64_t j = lane; j < v; j += 32) {
-            const U x = row[j];
+                for (int i = 0; i < C::NR; ++i) m[t][i] = 0;  // saves nothing
+            }
+            if (PACK && (t & 1))
+                C::template set_bits<16>(m[t], pc[t]);
+            else
+                C::set_bits(m[t], pc[t]);
+        }
+    };
+    const int64_t steps = (chunks + G - 1) / G;  // per row
+    if (steps == 1 && sub < chunks) tables(sub);
+    unsigned long long acc[L][PACK ? 2 : 1];
 #pragma unroll
-            for (int t = 0; t < kMaxThresholds; ++t) {
-                if (t < nthr) {
-                    const U m = __ldg(&masks[t * v + j]);
-                    if ((U)(x & m) == __ldg(&bitvals[t * v + j])) s[t] += popc_w(m);
-                }
+    for (int l = 0; l < L; ++l) {
+        acc[l][0] = 0;
+        if (PACK) acc[l][PACK ? 1 : 0] = 0;
+    }
+    // Batches of RPW * Q rows from the last to the first: the census ended with the last rows,
+    // so they are still in L2.  Each step's rows are loaded while the step before is counted.
+    const int64_t batches = (n + RPW * Q - 1) / (RPW * Q);
+    auto load = [&](int64_t batch, int64_t c, uint32_t (&x)[Q][C::NR]) {
+        const int64_t r0 = batch * (RPW * Q) + gin;
+        const char *p = reinterpret_cast<const char *>(data) + r0 * row_bytes + c * A;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            if (c < chunks && r0 + q * RPW < n) {
+                C::load(p + q * RPW * row_bytes, x[q]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < C::NR; ++i) x[q][i] = 0;
             }
         }
+    };
+    uint32_t x[Q][C::NR];
+    int64_t batch = batches - 1 - warp;
+    if (batch >= 0) load(batch, sub, x);
+    for (; batch >= 0; batch -= nwarps) {
+        uint32_t f[Q * S];
 #pragma unroll
-        for (int t = 0; t < kMaxThresholds; ++t) {
-            if (t < nthr) {
-                const uint32_t tot = __reduce_add_sync(0xffffffffu, s[t]);
-                if (tot > (uint64_t)v) acc[t] += tot - (uint64_t)v;
+        for (int i = 0; i < Q * S; ++i) f[i] = 0;
+        const int64_t left = n - (batch * (RPW * Q) + gin);  // rows of this group's, every RPW-th
+        for (int64_t k = 0; k < steps; ++k) {
+            const int64_t c = k * G + sub;
+            uint32_t y[Q][C::NR];
+            const bool more = k + 1 < steps;
+            if (more || batch >= nwarps) load(more ? batch : batch - nwarps, more ? c + G : sub, y);
+            if (steps > 1 && c < chunks) tables(c);
+            if (c < chunks) {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    if (q * RPW < left) {
+                        if constexpr (T > 1) {
+#pragma unroll
+                            for (int i = 0; i < C::NR; ++i) x[q][i] ^= b[i];
+#pragma unroll
+                            for (int t = 0; t < T; ++t) {
+                                auto e = [&](int i) { return x[q][i] & m[t][i]; };
+                                if (PACK && (t & 1))
+                                    C::template matched<16>(f[q * S + t / 2], e, pc[t], one);
+                                else
+                                    C::matched(f[q * S + (PACK ? t / 2 : t)], e, pc[t], one);
+                            }
+                        } else {
+                            C::matched(f[q], [&](int i) { return (x[q][i] & m[0][i]) ^ b[i]; },
+                                       pc[0], one);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int i = 0; i < C::NR; ++i) x[q][i] = y[q][i];
+        }
+        group_sums<Q * S, G>(f, one);
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            if constexpr (PACK) {
+                const uint32_t lo = f[l] & 0xffffu, hi = f[l] >> 16;
+                if (lo > (uint64_t)v) acc[l][0] += lo - (uint32_t)v;
+                if (hi > (uint64_t)v) acc[l][1] += hi - (uint32_t)v;
+            } else {
+                if (f[l] > (uint64_t)v) acc[l][0] += f[l] - (uint64_t)v;
             }
         }
     }
-    if (lane == 0) {
+    if ((sub & (group_sums_copies<Q * S, G>() - 1)) == 0) {
+        const int first = group_sums_value<Q * S, G>(sub);
 #pragma unroll
-        for (int t = 0; t < kMaxThresholds; ++t)
-            if (t < nthr && acc[t]) atomicAdd(&blk[t], acc[t]);
+        for (int l = 0; l < L; ++l) {
+            const int t = (first + l) % S;
+            if constexpr (PACK) {
+                if (acc[l][0]) atomicAdd(&blk[2 * t], acc[l][0]);
+                if (acc[l][1]) atomicAdd(&blk[2 * t + 1], acc[l][1]);
+            } else {
+                if (acc[l][0]) atomicAdd(&blk[t], acc[l][0]);
+            }
+        }
     }
     __syncthreads();
     if (threadIdx.x < nthr && blk[threadIdx.x]) atomicAdd(&saved[threadIdx.x], blk[threadIdx.x]);
+}
+
+template <typename U, int A>
+static ibp_status launch_check(const U *data, int64_t n, int64_t v, int nthr, const U *masks,
+                               const U *bitvals, unsigned long long *saved, cudaStream_t st) {
+    const bool narrow = v * (int64_t)sizeof(U) <= 8 * A;
+    const bool pack = v * 8 * (int64_t)sizeof(U) < 65536;
+    auto kern = nthr == 1 ? (narrow ? check_saved_kernel<U, A, 8, 1, false>
+                                    : check_saved_kernel<U, A, 32, 1, false>)
+                          : (narrow ? check_saved_kernel<U, A, 8, 7, true>
+                                    : (pack ? check_saved_kernel<U, A, 32, 7, true>
+                                            : check_saved_kernel<U, A, 32, 7, false>));
+    const int64_t per_block = 8 * (nthr == 1 ? 8 : 4) * (narrow ? 4 : 1);
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, 256, 0, &per_sm));
+    const int64_t blocks =
+        std::min<int64_t>((n + per_block - 1) / per_block, (int64_t)device_sm_count() * per_sm);
+    IBP_CUDA(launch_dependent(kern, (unsigned)blocks, 256, 0, st, data, n, v, nthr, masks, bitvals,
+                              saved, 1u));
+    IBP_LAUNCHED("check_saved_kernel");
+    return IBP_OK;
 }
 
 // First threshold with strictly more saved bits than every earlier one (and > 0) wins;
@@ -190,6 +329,7 @@ __global__ void select_mask_kernel(const unsigned long long *__restrict__ saved,
                                    int64_t v, const U *__restrict__ masks,
                                    const U *__restrict__ bitvals, U *__restrict__ mask_out,
                                    U *__restrict__ bitval_out, int32_t *__restrict__ selected) {
+    grid_dep_wait();
     int sel = -1;
     double best = 0.0;
     for (int t = 0; t < nthr; ++t) {
@@ -217,27 +357,51 @@ ThrList sweep_thresholds(float threshold) {
     return l;
 }
 
-static void census_geometry(int64_t n, int64_t v, int &cpb, int &R, dim3 &grid) {
-    cpb = (int)(v < kCensusThreads ? v : kCensusThreads);
-    R = kCensusThreads / cpb;
-    const int64_t tiles = (v + cpb - 1) / cpb;
+// Counts of the whole dataset: groups of k rows as 16-byte pieces, then the rows left over.
+template <typename U>
+static ibp_status launch_census(const U *data, int64_t n, int64_t v, uint32_t *counts, U *stage,
+                                cudaStream_t st) {
+    const int64_t row_bytes = v * (int64_t)sizeof(U);
+    int64_t k = 1;
+    while (k * row_bytes % 16) k *= 2;
+    const bool aligned = ((((uintptr_t)data) | ((uintptr_t)stage)) & 15) == 0;
+    const int64_t groups = aligned ? n / k : 0;
     const int sms = device_sm_count();
-    int64_t gx = (n + (int64_t)R * 512 - 1) / ((int64_t)R * 512);
-    int64_t cap = (int64_t)sms * 8 / tiles;
-    if (cap < 1) cap = 1;
-    if (gx > cap) gx = cap;
-    if (gx < 1) gx = 1;
-    grid = dim3((unsigned)gx, (unsigned)tiles);
+    if (groups > 0) {
+        const int64_t pieces = k * row_bytes / 16;
+        const int cpb = (int)std::min<int64_t>(pieces, kCensusCols);
+        const int R = kCensusThreads / cpb;
+        const size_t smem = sizeof(uint32_t) * 128 * (size_t)(cpb | 1);
+        int per_sm = 0;
+        IBP_RET(kernel_blocks_per_sm((const void *)census_kernel, kCensusThreads, smem, &per_sm));
+        const int64_t tiles = (pieces + cpb - 1) / cpb;
+        // at least 32 groups per row slot (a block's counters cost 128 x cpb global atomics)
+        const int64_t gx = std::max<int64_t>(
+            1, std::min<int64_t>((groups + R * 32 - 1) / (R * 32), (int64_t)sms * per_sm / tiles));
+        census_kernel<<<(unsigned)(gx * tiles), kCensusThreads, smem, st>>>(
+            reinterpret_cast<const uint4 *>(data), groups, pieces, cpb, (int)tiles, row_bytes * 8, k > 1, counts, reinterpret_cast<uint4 *>(stage));
+        IBP_LAUNCHED("census_kernel");
+    }
+    const int64_t done = groups * k;
+    if (done < n) {
+        const int64_t threads = (n - done + 31) / 32 * v;
+        const int64_t blocks = std::min<int64_t>((threads + kCensusThreads - 1) / kCensusThreads,
+                                                 (int64_t)sms * 8);
+        census_rest_kernel<U><<<(unsigned)blocks, kCensusThreads, 0, st>>>(
+            data + done * v, n - done, v, counts, stage ? stage + done * v : nullptr);
+        IBP_LAUNCHED("census_rest_kernel");
+    }
+    return IBP_OK;
 }
 
 size_t preprocess_workspace(int64_t n, int64_t v, int wb, float threshold, bool staged) {
     Sizer s;
     s.take<char>(kStatusBytes);
     const ThrList l = sweep_thresholds(threshold);
+    s.take<unsigned long long>(kMaxThresholds);          // saved bits
     s.take<uint32_t>((size_t)(v * 8 * wb));              // counts
     s.take<char>((size_t)(l.count > 0 ? l.count : 1) * v * wb);  // masks
     s.take<char>((size_t)(l.count > 0 ? l.count : 1) * v * wb);  // bitvals
-    s.take<unsigned long long>(kMaxThresholds);          // saved bits
     s.take<int32_t>(4);                                  // selected step
     if (staged) s.take<char>((size_t)(n * v * wb));
     return s.total();
@@ -247,14 +411,14 @@ template <typename U>
 ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold, U *mask,
                            U *bitval, void *ws, size_t ws_bytes, bool data_on_host,
                            cudaStream_t st) {
-    const int wb = sizeof(U);
+    constexpr int wb = sizeof(U);
     const ThrList thr = sweep_thresholds(threshold);
     Carver c{(char *)ws, 0, ws_bytes};
     c.take<char>(kStatusBytes);
+    unsigned long long *saved = c.take<unsigned long long>(kMaxThresholds);
     uint32_t *counts = c.take<uint32_t>((size_t)(v * 8 * wb));
     U *masks = c.take<U>((size_t)(thr.count > 0 ? thr.count : 1) * v);
     U *bitvals = c.take<U>((size_t)(thr.count > 0 ? thr.count : 1) * v);
-    unsigned long long *saved = c.take<unsigned long long>(kMaxThresholds);
     int32_t *selected = c.take<int32_t>(4);
     if (!selected) {
         set_error("preprocess: workspace of %zu bytes is below the required %zu", ws_bytes,
@@ -263,38 +427,31 @@ ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold,
     }
     U *stage = nullptr;
     if (data_on_host && thr.count > 0) stage = c.take<U>((size_t)(n * v));  // null if it does not fit
-    IBP_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * v * 8 * wb, st));
-    IBP_CUDA(cudaMemsetAsync(saved, 0, sizeof(unsigned long long) * kMaxThresholds, st));
-    if (n > 0 && v > 0) {
-        int cpb, R;
-        dim3 grid;
-        census_geometry(n, v, cpb, R, grid);
-        const size_t smem = sizeof(uint32_t) * 8 * wb * kCensusThreads;
-        auto kern = census_kernel<U>;
-        if (smem > 48 * 1024)
-            IBP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-        kern<<<grid, kCensusThreads, smem, st>>>(data, n, v, cpb, R, counts, stage);
-        IBP_LAUNCHED("census_kernel");
-    }
+    // the saved bits and the counts follow one another
+    IBP_CUDA(cudaMemsetAsync(saved, 0, (size_t)((char *)(counts + v * 8 * wb) - (char *)saved), st));
+    if (n > 0 && v > 0) IBP_RET(launch_census<U>(data, n, v, counts, stage, st));
     if (thr.count > 0 && v > 0) {
-        const int64_t tot = v * thr.count;
-        const int blocks = (int)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096);
-        masks_from_counts_kernel<U><<<blocks, 256, 0, st>>>(counts, n, v, thr, masks, bitvals);
+        const int64_t warps = (v * 8 * wb + 31) / 32;
+        const unsigned blocks = (unsigned)std::min<int64_t>((warps + 7) / 8, 4096);
+        IBP_CUDA(launch_dependent(masks_from_counts_kernel<U>, blocks, 256, 0, st, counts, n, v,
+                                  thr, masks, bitvals));
         IBP_LAUNCHED("masks_from_counts_kernel");
         if (n > 0) {
-            const int sms = device_sm_count();
-            int64_t blocks2 = (n + 7) / 8;
-            if (blocks2 > (int64_t)sms * 8) blocks2 = (int64_t)sms * 8;
-            check_saved_kernel<U><<<(unsigned)blocks2, 256, 0, st>>>(
-                stage ? stage : data, n, v, thr.count, masks, bitvals, saved);
-            IBP_LAUNCHED("check_saved_kernel");
+            const U *rows = stage ? stage : data;
+            const int a = row_chunk_bytes(rows, v, wb);
+            if (a == 16)
+                IBP_RET((launch_check<U, 16>(rows, n, v, thr.count, masks, bitvals, saved, st)));
+            else if (a == 4 && wb < 4)
+                IBP_RET((launch_check<U, wb < 4 ? 4 : 16>(rows, n, v, thr.count, masks, bitvals,
+                                                          saved, st)));
+            else
+                IBP_RET((launch_check<U, wb>(rows, n, v, thr.count, masks, bitvals, saved, st)));
         }
     }
     if (v > 0) {
         const int blocks = (int)((v + 255) / 256 < 1024 ? (v + 255) / 256 : 1024);
-        select_mask_kernel<U><<<blocks, 256, 0, st>>>(saved, thr.count, v, masks, bitvals, mask,
-                                                      bitval, selected);
+        IBP_CUDA(launch_dependent(select_mask_kernel<U>, (unsigned)blocks, 256, 0, st, saved,
+                                  thr.count, v, masks, bitvals, mask, bitval, selected));
         IBP_LAUNCHED("select_mask_kernel");
     }
     return IBP_OK;
