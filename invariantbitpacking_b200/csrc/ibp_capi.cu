@@ -199,7 +199,7 @@ static ibp_status compress_inplace_t(U *data, int64_t n, int64_t v, const U *mas
     int32_t *status = c.take<int32_t>(kStatusBytes / 4);
     ColTables<U> t = carve_tables<U>(c, v);
     IBP_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), st));
-    if (v > 0) IBP_RET(build_tables<U>(mask, bitval, v, t, st));
+    if (v > 0) IBP_RET((build_tables<U, false>(mask, bitval, v, t, st)));
     if (has_index) {
         // every source row is read before any row is overwritten
         U *stage = c.take<U>((size_t)(nidx * v));
@@ -491,16 +491,16 @@ ibp_status ibp_compress_condensed(const void *dataset, int64_t num_vecs, int64_t
     if (word_bytes == 4) {
         ColTables<uint32_t> t = carve_tables<uint32_t>(c, vec_size);
         if (vec_size > 0)
-            IBP_RET(build_tables<uint32_t>((const uint32_t *)mask, (const uint32_t *)bitval,
-                                           vec_size, t, st));
+            IBP_RET((build_tables<uint32_t, false>((const uint32_t *)mask, (const uint32_t *)bitval,
+                                                   vec_size, t, st)));
         return compress_condensed_rows<uint32_t>((const uint32_t *)dataset, num_vecs, vec_size,
                                                  t, index, nrows, offsets, (uint32_t *)out,
                                                  status, st);
     }
     ColTables<uint64_t> t = carve_tables<uint64_t>(c, vec_size);
     if (vec_size > 0)
-        IBP_RET(build_tables<uint64_t>((const uint64_t *)mask, (const uint64_t *)bitval,
-                                       vec_size, t, st));
+        IBP_RET((build_tables<uint64_t, false>((const uint64_t *)mask, (const uint64_t *)bitval,
+                                               vec_size, t, st)));
     return compress_condensed_rows<uint64_t>((const uint64_t *)dataset, num_vecs, vec_size, t,
                                              index, nrows, offsets, (uint64_t *)out, status, st);
 }

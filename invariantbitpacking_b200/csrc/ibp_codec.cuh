@@ -8,13 +8,17 @@
 //                  all W bits;
 //   then zeros up to v words.
 //
-// Bit gather/scatter (x -> bits of x under `sel`, packed right; and the inverse) uses the
+// Bit gather/scatter (x -> bits of x under `sel`, packed; and the inverse) uses the
 // parallel-suffix method of H. S. Warren, "Hacker's Delight", 2nd ed., sections 7-4
-// (compress) and 7-5 (expand): log2(W) steps, each moving bits right by 2^i under a
+// (compress) and 7-5 (expand): five steps per 32-bit half, each moving bits by 2^i under a
 // per-column "move" mask.  The move masks depend only on the column's mask, so they are
-// built once per call (build_tables_kernel) and every word then costs log2(W) branch-free
-// steps instead of a data-dependent loop over mask runs.
+// built once per call (build_tables_kernel) and every word then costs a few branch-free
+// steps instead of a data-dependent loop over mask runs.  64-bit words are moved as two
+// 32-bit halves: five steps of one shift each (which can run as a multiplication on the other
+// pipe) in place of six of two.
 #pragma once
+
+#include <type_traits>
 
 #include "ibp_common.cuh"
 
@@ -23,19 +27,35 @@ namespace ibp200 {
 template <typename U>
 struct LogW { static constexpr int value = sizeof(U) == 8 ? 6 : 5; };
 
+constexpr int kMoves = 5;  // move masks per 32-bit half
+
+// Kept bits of a column: of the word (low byte) and, for 64-bit words, of its low half (high
+// byte).
+template <typename U>
+using KeptBits = typename std::conditional<sizeof(U) == 8, uint16_t, uint8_t>::type;
+
+template <typename U>
+__device__ __forceinline__ KeptBits<U> kept_bits(U mask) {
+    const int nb = 8 * (int)sizeof(U) - popc_w(mask);
+    if constexpr (sizeof(U) == 8)
+        return (KeptBits<U>)(nb | (32 - __popc((uint32_t)mask)) << 8);
+    else
+        return (KeptBits<U>)nb;
+}
+
 // Per-column decode/encode tables, structure-of-arrays in a workspace buffer.
 template <typename U>
 struct ColTables {
-    U *mask;       // [v]
-    U *bitval;     // [v]
-    U *mv;         // [LogW][v] move masks of sel = ~mask
-    uint8_t *nb;   // [v] bits a compressible word keeps = W - popc(mask)
+    U *mask;          // [v]
+    U *bitval;        // [v]
+    U *mv;            // [kMoves][v] move masks of sel = ~mask, each half's in its own half
+    KeptBits<U> *nb;  // [v] bits a compressible word keeps
 };
 
 template <typename U>
 size_t tables_bytes(int64_t v) {
-    return align_up((size_t)v * sizeof(U), kAlign) * (2 + LogW<U>::value) +
-           align_up((size_t)v, kAlign);
+    return align_up((size_t)v * sizeof(U), kAlign) * (2 + kMoves) +
+           align_up((size_t)v * sizeof(KeptBits<U>), kAlign);
 }
 
 template <typename U>
@@ -43,8 +63,8 @@ ColTables<U> carve_tables(Carver &c, int64_t v) {
     ColTables<U> t;
     t.mask = c.take<U>(v);
     t.bitval = c.take<U>(v);
-    t.mv = c.take<U>((size_t)v * LogW<U>::value);
-    t.nb = c.take<uint8_t>(v);
+    t.mv = c.take<U>((size_t)v * kMoves);
+    t.nb = c.take<KeptBits<U>>(v);
     return t;
 }
 
@@ -58,78 +78,105 @@ __device__ __forceinline__ U shr_w(U x, int s) {
     return s >= (int)(8 * sizeof(U)) ? (U)0 : (U)(x >> s);
 }
 
-// Move masks for gathering/scattering the bits of `sel` (Hacker's Delight 7-4 / 7-5).
-template <typename U>
-__device__ __forceinline__ void move_masks(U sel, U *mv, int stride) {
-    constexpr int LW = LogW<U>::value;
-    U m = sel;
-    U mk = (U)(~m << 1);
+// Move masks for scattering to (RIGHT: gathering from, packed right) the bits of `sel`
+// (Hacker's Delight 7-4 / 7-5), or, mirrored, for gathering them packed left.
+template <bool RIGHT>
+__device__ __forceinline__ void move_masks(uint32_t sel, uint32_t (&mv)[kMoves]) {
+    uint32_t m = sel;
+    uint32_t mk = RIGHT ? ~m << 1 : ~m >> 1;
 #pragma unroll
-    for (int i = 0; i < LW; ++i) {
-        U mp = (U)(mk ^ (mk << 1));
+    for (int i = 0; i < kMoves; ++i) {
+        uint32_t mp = mk;
 #pragma unroll
-        for (int k = 1; k < LW; ++k) mp = (U)(mp ^ (mp << (1 << k)));
-        const U v = (U)(mp & m);
-        mv[i * stride] = v;
-        m = (U)((m ^ v) | (v >> (1 << i)));
-        mk = (U)(mk & ~mp);
+        for (int k = 0; k < kMoves; ++k) mp ^= RIGHT ? mp << (1 << k) : mp >> (1 << k);
+        const uint32_t v = mp & m;
+        mv[i] = v;
+        m = (m ^ v) | (RIGHT ? v >> (1 << i) : v << (1 << i));
+        mk &= ~mp;
     }
 }
 
-// bits of x at the set positions of sel, packed to the right (pext)
-template <typename U>
-__device__ __forceinline__ U gather_bits(U x, U sel, const U *mv, int stride) {
-    constexpr int LW = LogW<U>::value;
-    x &= sel;
+// Bits of x at the set positions of ~mask, packed to the left (pext, left-aligned), with the
+// first LEVELS moves: the later masks are all zero where no kept bit has 2^LEVELS or more
+// dropped bits above it.
+template <int LEVELS>
+__device__ __forceinline__ uint32_t gather_left(uint32_t x, uint32_t mask,
+                                                const uint32_t (&mv)[kMoves]) {
+    x &= ~mask;
 #pragma unroll
-    for (int i = 0; i < LW; ++i) {
-        const U v = mv[i * stride];
-        const U t = (U)(x & v);
-        x = (U)((x ^ t) | (t >> (1 << i)));
+    for (int i = 0; i < LEVELS; ++i) {
+        const uint32_t t = x & mv[i];
+        x = (x ^ t) | (t << (1 << i));
     }
     return x;
 }
 
-// inverse of gather_bits: the low bits of y placed at the set positions of sel (pdep)
-template <typename U>
-__device__ __forceinline__ U scatter_bits(U y, U sel, const U *mv, int stride) {
-    constexpr int LW = LogW<U>::value;
+// The low bits of y placed at the set positions of sel (pdep), for move masks of
+// move_masks<true>; `keep` is the value outside sel.
+__device__ __forceinline__ uint32_t scatter_half(uint32_t y, uint32_t sel, uint32_t keep,
+                                                 const uint32_t (&mv)[kMoves]) {
 #pragma unroll
-    for (int i = LW - 1; i >= 0; --i) {
-        const U v = mv[i * stride];
-        const U t = (U)(y << (1 << i));
-        y = (U)((y & ~v) | (t & v));
-    }
-    return (U)(y & sel);
+    for (int i = kMoves - 1; i >= 0; --i) y = (y & ~mv[i]) | ((y << (1 << i)) & mv[i]);
+    return (y & sel) | keep;
 }
 
-// Column j of the tables.
+// The word whose kept bits are the low bits of y: scattered per half (the low half takes the
+// last nbl of them), with the invariant bits bv.
 template <typename U>
+__device__ __forceinline__ U scatter_word(U y, U mask, U bv, int nbl, const U (&mv)[kMoves]) {
+    uint32_t lo[kMoves];
+#pragma unroll
+    for (int i = 0; i < kMoves; ++i) lo[i] = (uint32_t)mv[i];
+    const uint32_t l = scatter_half((uint32_t)y, ~(uint32_t)mask, (uint32_t)bv, lo);
+    if constexpr (sizeof(U) == 8) {
+        uint32_t hi[kMoves];
+#pragma unroll
+        for (int i = 0; i < kMoves; ++i) hi[i] = (uint32_t)(mv[i] >> 32);
+        const uint32_t yh = __funnelshift_rc((uint32_t)y, (uint32_t)(y >> 32), nbl);
+        const uint32_t h = scatter_half(yh, ~(uint32_t)(mask >> 32), (uint32_t)(bv >> 32), hi);
+        return (uint64_t)h << 32 | l;
+    } else {
+        return l;
+    }
+}
+
+// Column j of the tables (RIGHT: for decoding; else for packing).
+template <typename U, bool RIGHT = true>
 __device__ __forceinline__ void build_table_column(const U *__restrict__ mask,
                                                    const U *__restrict__ bitval, int64_t v,
                                                    const ColTables<U> &t, int64_t j) {
     const U m = mask[j];
     t.mask[j] = m;
     t.bitval[j] = bitval[j];
-    t.nb[j] = (uint8_t)(8 * sizeof(U) - popc_w(m));
-    move_masks<U>((U)~m, t.mv + j, (int)v);
+    t.nb[j] = kept_bits<U>(m);
+    uint32_t mv[kMoves];
+    move_masks<RIGHT>(~(uint32_t)m, mv);
+    if constexpr (sizeof(U) == 8) {
+        uint32_t hv[kMoves];
+        move_masks<RIGHT>(~(uint32_t)(m >> 32), hv);
+#pragma unroll
+        for (int i = 0; i < kMoves; ++i) t.mv[i * v + j] = (uint64_t)hv[i] << 32 | mv[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < kMoves; ++i) t.mv[i * v + j] = mv[i];
+    }
 }
 
-template <typename U>
+template <typename U, bool RIGHT>
 __global__ void build_tables_kernel(const U *__restrict__ mask, const U *__restrict__ bitval,
                                     int64_t v, ColTables<U> t) {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < v;
          j += (int64_t)gridDim.x * blockDim.x)
-        build_table_column<U>(mask, bitval, v, t, j);
+        build_table_column<U, RIGHT>(mask, bitval, v, t, j);
 }
 
-template <typename U>
+template <typename U, bool RIGHT = true>
 inline ibp_status build_tables(const U *mask, const U *bitval, int64_t v, ColTables<U> t,
                                cudaStream_t st) {
     if (v <= 0) return IBP_OK;
     int blocks = (int)((v + 255) / 256);
     if (blocks > 1024) blocks = 1024;
-    build_tables_kernel<U><<<blocks, 256, 0, st>>>(mask, bitval, v, t);
+    build_tables_kernel<U, RIGHT><<<blocks, 256, 0, st>>>(mask, bitval, v, t);
     IBP_LAUNCHED("build_tables_kernel");
     return IBP_OK;
 }
@@ -142,22 +189,17 @@ __device__ __forceinline__ int unit_slot(int64_t q) {
     return sizeof(U) == 8 ? (int)(q ^ 1) : (int)q;
 }
 
-// OR the L (0..64) low bits of val into the stream at bit offset s (shared memory units).
+// OR a word's bits (left-aligned in hi:lo, the rest zero; hi alone for 32-bit words) into a
+// shared-memory image at bit s.  The image's units are in stream order.
+__device__ __forceinline__ void or_shared(uint32_t addr, uint32_t x) {
+    asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
+}
 template <typename U>
-__device__ __forceinline__ void put_bits(uint32_t *units, int64_t s, uint64_t val, int L) {
-    if (L <= 0) return;
-    const int64_t q = s >> 5;
-    const int off = (int)(s & 31);
-    // left-align the L bits in 64 bits
-    const uint64_t a = (L >= 64) ? val : (val << (64 - L));
-    // unit q takes the top (32 - off) bits of a
-    atomicOr(&units[unit_slot<U>(q)], (uint32_t)(a >> (32 + off)));
-    const int used = 32 - off;
-    if (L > used) {
-        const uint64_t b = a << used;  // used in [1, 32]
-        atomicOr(&units[unit_slot<U>(q + 1)], (uint32_t)(b >> 32));
-        if (L > used + 32) atomicOr(&units[unit_slot<U>(q + 2)], (uint32_t)(b & 0xffffffffu));
-    }
+__device__ __forceinline__ void put_bits(uint32_t image, uint32_t s, uint32_t hi, uint32_t lo) {
+    const uint32_t at = image + ((s >> 3) & ~3u), off = s & 31;
+    or_shared(at, hi >> off);
+    or_shared(at + 4, __funnelshift_r(lo, hi, off));
+    if constexpr (sizeof(U) == 8) or_shared(at + 8, __funnelshift_r(0, lo, off));
 }
 
 // Read L (0..W) bits at stream offset s from W-bit words (MSB-first); needs word s/W + 1.

@@ -3,15 +3,14 @@
 // (packer and its launchers) and the size/offset glue of src/compress.cu.
 //
 // B200 design
-//  * sizes: 8 or 32 lanes per row, 16 bytes a lane where rows allow it, 8 rows in flight, the
+//  * sizes: 8, 16 or 32 lanes per row, 16 bytes a lane where rows allow it, 8 rows in flight, the
 //    columns' tables in registers; no shared-memory atomics (the reference uses one
 //    256-thread block per row with smem atomics).
-//  * packing: one warp per row.  The row is staged in shared memory once (so in-place
-//    compression of a pinned host row reads it over PCIe once), every lane gathers its
-//    word's non-invariant bits with the Hacker's Delight move masks, a warp prefix sum
-//    gives bit offsets, and bits are ORed into a shared-memory copy of the output row
-//    (32-bit shared atomics, at most 3 per word).  The finished row goes back with one
-//    coalesced pass; an incompressible row compressed in place is not written at all.
+//  * packing: a warp per row and 4 rows in flight; words go from memory to registers once,
+//    each lane gathers its words' non-invariant bits with the Hacker's Delight move masks (in
+//    registers for rows of up to 64 words) and ORs them into a shared-memory image of the
+//    output row (32-bit shared atomics, at most 3 per word).  The finished row goes back with
+//    one coalesced pass; an incompressible row compressed in place is not written at all.
 //    No global workspace is cudaMalloc'd or freed per call (the reference does both and
 //    thereby blocks the host).
 #include <cub/device/device_scan.cuh>
@@ -25,11 +24,12 @@
 namespace ibp200 {
 
 // ------------------------------------------------------------------ sizes
-// Bound: reading the rows.  G lanes share a row (8, 16 or 32 by its chunks of A bytes) and
+// Bound: reading the rows.  G lanes share a row (8, 16 or 32 by its pieces of A bytes) and
 // take 8 rows at a time, all loads before any use, so a warp has up to 4 KiB in
 // flight; the columns' mask, values and set bits stay in registers, loaded once when a group
 // covers the row and once per 8 rows when it does not (1M rows of 128 16-bit words: 239 us
-// with a 2-byte load and two table loads a word, 103 with half the lanes idle, 51 now, 5.2 TB/s).
+// with a 2-byte load and two table loads a word, 103 with half the lanes idle, 51 now, 5.2 TB/s;
+// 200k rows of 99 32-bit words, in 4-byte pieces: 70 us, 78 with one piece a lane, 28 with four).
 constexpr int kSizeRows = 8;
 
 template <typename U, int A, int G, bool INDEX>
@@ -39,7 +39,7 @@ compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
                      const int64_t *__restrict__ idx, int64_t nrows,
                      int64_t *__restrict__ sizes, unsigned long long *__restrict__ total,
                      int32_t *__restrict__ status, uint32_t one) {
-    using C = Chunk<U, A>;
+    using C = Chunk<U, A, G>;
     constexpr int RPW = 32 / G, Q = kSizeRows;
     __shared__ unsigned long long block_sum;
     const int lane = threadIdx.x & 31, sub = lane & (G - 1), gin = lane / G;
@@ -52,11 +52,12 @@ compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
     unsigned long long acc = 0;
     uint32_t m[C::NR], b[C::NR], pc[C::NW];
     auto tables = [&](int64_t c) {
-        C::load_words(mask + c * (A / (int)sizeof(U)), m);
-        C::load_words(bitval + c * (A / (int)sizeof(U)), b);
+        C::load_words(mask, c, chunks, m);
+        C::load_words(bitval, c, chunks, b);
         C::set_bits(m, pc);
     };
-    const bool once = chunks <= G;
+    constexpr int SP = G * C::NS;  // pieces of a step
+    const bool once = chunks <= SP;
     if (once && sub < chunks) tables(sub);
     for (int64_t base = warp * RPW * Q; base < nrows; base += nwarps * RPW * Q) {
         // positions i0 + q * RPW; consecutive rows without an index
@@ -79,12 +80,12 @@ compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
         uint32_t s[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) s[q] = 0;
-        for (int64_t c = sub; c < chunks; c += G) {
+        for (int64_t c = sub; c < chunks; c += SP) {
             uint32_t x[Q][C::NR];
 #pragma unroll
             for (int q = 0; q < Q; ++q)
                 if ((okm >> q) & 1)
-                    C::load((INDEX ? row[INDEX ? q : 0] : row[0] + q * RPW * row_bytes) + c * A, x[q]);
+                    C::load(INDEX ? row[INDEX ? q : 0] : row[0] + q * RPW * row_bytes, c, chunks, x[q]);
             if (!once) tables(c);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
@@ -121,10 +122,10 @@ static ibp_status launch_sizes(const U *data, int64_t n, int64_t v, const U *mas
     const int64_t chunks = v * (int64_t)sizeof(U) / A;
     auto kern = idx ? compress_size_kernel<U, A, 32, true> : compress_size_kernel<U, A, 32, false>;
     int lanes = 32;
-    if (chunks <= 8) {
+    if (chunks <= 8 * Chunk<U, A, 8>::NS) {
         kern = idx ? compress_size_kernel<U, A, 8, true> : compress_size_kernel<U, A, 8, false>;
         lanes = 8;
-    } else if (chunks <= 16) {
+    } else if (chunks <= 16 * Chunk<U, A, 8>::NS) {
         kern = idx ? compress_size_kernel<U, A, 16, true> : compress_size_kernel<U, A, 16, false>;
         lanes = 16;
     }
@@ -145,7 +146,7 @@ ibp_status compress_size_impl(const U *data, int64_t n, int64_t v, const U *mask
                               int64_t *sizes, int64_t *total, int32_t *status,
                               cudaStream_t st) {
     if (nrows <= 0) return IBP_OK;
-    const int a = row_chunk_bytes(data, v, sizeof(U));
+    const int a = row_piece_bytes(data, v, sizeof(U));
     if (a == 16)
         return launch_sizes<U, 16>(data, n, v, mask, bitval, idx, nrows, sizes, total, status, st);
     if constexpr (sizeof(U) < 4)
@@ -157,48 +158,6 @@ ibp_status compress_size_impl(const U *data, int64_t n, int64_t v, const U *mask
 }
 
 // ------------------------------------------------------------------ packing
-// Packs row `in` (v words in shared memory) into `out_units` (shared, zeroed, v words +
-// pad) with a warp.  Returns nothing; bitmap + stream land in out_units.
-template <typename U>
-__device__ __forceinline__ void pack_row_warp(const U *in, int64_t v, ColTables<U> t,
-                                              uint32_t *out_units) {
-    constexpr int W = 8 * sizeof(U);
-    const int lane = threadIdx.x & 31;
-    const int64_t mw = meta_bytes(v, (int)sizeof(U)) / (int64_t)sizeof(U);
-    const int64_t stream0 = mw * W;  // stream bit 0 in row bits
-    int64_t base = 0;
-    for (int64_t c0 = 0; c0 < v; c0 += 32) {
-        const int64_t j = c0 + lane;
-        bool cj = false;
-        int L = 0;
-        uint64_t val = 0;
-        if (j < v) {
-            const U x = in[j];
-            const U m = __ldg(&t.mask[j]);
-            cj = (U)(x & m) == __ldg(&t.bitval[j]);
-            if (cj) {
-                L = __ldg(&t.nb[j]);
-                val = (uint64_t)gather_bits<U>(x, (U)~m, t.mv + j, (int)v);
-            } else {
-                L = W;
-                val = (uint64_t)x;
-            }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, cj);
-        if (lane == 0) out_units[c0 >> 5] = bal;  // bitmap unit (j/32), LSB-first
-        // exclusive prefix of L across the warp
-        int incl = L;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int64_t off = base + incl - L;
-        put_bits<U>(out_units, stream0 + off, val, L);
-        base += __shfl_sync(0xffffffffu, incl, 31);
-    }
-}
-
 template <typename U>
 struct PackArgs {
     const U *src;
@@ -212,95 +171,327 @@ struct PackArgs {
     bool in_place;      // out rows alias src rows one to one
     int32_t *bitmask;
     int32_t *status;
-    int64_t row_words;  // smem words per staged row buffer
+    int64_t buf_words;  // shared-memory words per output row
 };
 
+// A lane's tables for NC columns (32 * c + lane of a group of 32 * NC), and where each column's
+// bits start, and the group's end, when all of it is compressible.
+template <typename U, int NC>
+struct PackTables {
+    static constexpr int H = sizeof(U) / 4;  // 32-bit halves, high first
+    uint32_t m[NC][H], bv[NC][H], mv[NC][H][kMoves];
+    uint32_t nb[NC], nbh[NC];  // kept bits of the word, of its high half
+    uint32_t before[NC], all, valid[NC];
+    int levels;  // moves the group's columns need (gather_left)
+
+    __device__ __forceinline__ static void split(U x, uint32_t (&h)[H]) {
+        if constexpr (H == 2) {
+            h[0] = (uint32_t)(x >> 32);
+            h[1] = (uint32_t)x;
+        } else {
+            h[0] = x;
+        }
+    }
+
+    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t j0) {
+        const int lane = threadIdx.x & 31;
+        uint32_t moves[kMoves] = {};
+        all = 0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int64_t j = j0 + 32 * c + lane;
+            const bool in = j < v;  // a column past the end: no bits, always compressible
+            valid[c] = __ballot_sync(0xffffffffu, in);
+            split(in ? __ldg(&t.mask[j]) : (U)0, m[c]);
+            split(in ? __ldg(&t.bitval[j]) : (U)0, bv[c]);
+            const uint32_t k = in ? (uint32_t)__ldg(&t.nb[j]) : 0u;
+            nb[c] = k & 0xffu;
+            nbh[c] = nb[c] - (k >> 8);
+#pragma unroll
+            for (int i = 0; i < kMoves; ++i) {
+                uint32_t h[H];
+                split(in ? __ldg(&t.mv[i * v + j]) : (U)0, h);
+#pragma unroll
+                for (int x = 0; x < H; ++x) {
+                    mv[c][x][i] = h[x];
+                    moves[i] |= h[x];
+                }
+            }
+            uint32_t incl = nb[c];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            before[c] = all + incl - nb[c];
+            all += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        levels = 0;
+#pragma unroll
+        for (int i = 0; i < kMoves; ++i)
+            if (__any_sync(0xffffffffu, moves[i] != 0)) levels = i + 1;
+    }
+};
+
+// Moves `words` words of a row image (units in stream order: a 64-bit word's high half first)
+// to global memory and leaves zeros in their place.
 template <typename U>
-__global__ void __launch_bounds__(256) pack_rows_kernel(PackArgs<U> a) {
+__device__ __forceinline__ void write_image(U *__restrict__ dst, uint32_t *image, int words) {
+    const int lane = threadIdx.x & 31;
+    int done = 0;
+    if ((((uintptr_t)dst) & 15) == 0) {
+        uint4 *d4 = reinterpret_cast<uint4 *>(dst), *b4 = reinterpret_cast<uint4 *>(image);
+        const int n16 = words * (int)sizeof(U) / 16;
+        for (int k = lane; k < n16; k += 32) {
+            const uint4 x = b4[k];
+            b4[k] = make_uint4(0, 0, 0, 0);
+            d4[k] = sizeof(U) == 8 ? make_uint4(x.y, x.x, x.w, x.z) : x;
+        }
+        done = n16 * (16 / (int)sizeof(U));
+    }
+    for (int k = done + lane; k < words; k += 32) {
+        if constexpr (sizeof(U) == 8) {
+            dst[k] = (uint64_t)image[2 * k] << 32 | image[2 * k + 1];
+            image[2 * k] = image[2 * k + 1] = 0;
+        } else {
+            dst[k] = image[k];
+            image[k] = 0;
+        }
+    }
+}
+
+// A warp takes Q consecutive positions at a time.  Each row goes through registers once: a
+// lane gathers its words' kept bits (left-aligned) and ORs them into the row's zeroed
+// shared-memory image at the word's bit offset, the row's length falls out of the last offset,
+// and only then is it known whether the row is stored compressed; the image is written (or, for
+// a row that stays raw, dropped) and zeroed for the next.  Offsets come from the tables where
+// a group is all compressible, else from a prefix sum.  Rows of up to 32 * NC words keep their
+// tables in registers (ONE); longer ones load them per group of columns, for Q rows at once.
+// The words of the next step are loaded while this one is packed.  LEVELS: moves per gather.
+template <typename U, int NC, int Q, bool ONE, bool INDEX, int LEVELS>
+__device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC> &t) {
+    constexpr int W = 8 * sizeof(U), H = sizeof(U) / 4;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    U *in = reinterpret_cast<U *>(smem) + (int64_t)wib * 2 * a.row_words;
-    U *outw = in + a.row_words;
-    uint32_t *out_units = reinterpret_cast<uint32_t *>(outw);
-    const int64_t v = a.v;
-    const int64_t vb = v * (int64_t)sizeof(U);
+    uint32_t *images = reinterpret_cast<uint32_t *>(smem) +
+                       (int64_t)(threadIdx.x >> 5) * Q * a.buf_words * H;
+    const int image_units = (int)a.buf_words * H;
+    const uint32_t images_at = (uint32_t)__cvta_generic_to_shared(images);
+    const int v = (int)a.v;
+    const uint32_t stream0 = (uint32_t)meta_bytes(v, (int)sizeof(U)) * 8;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = warp; i < a.nrows; i += nwarps) {
-        const int64_t r = a.idx ? a.idx[i] : i;
-        if (r < 0 || r >= a.n) {
-            if (lane == 0) atomicOr(a.status, kStatusBadIndex);
-            continue;
+    const int64_t batches = (a.nrows + Q - 1) / Q;
+    const int groups = ONE ? 1 : (v + 32 * NC - 1) / (32 * NC);
+    for (int k = lane; k < Q * image_units; k += 32) images[k] = 0;
+    __syncwarp();
+    // source row of position batch * Q + q (-1: none)
+    auto source = [&](int64_t batch, int q) -> int64_t {
+        const int64_t i = batch * Q + q;
+        if (i >= a.nrows) return -1;
+        if (!INDEX) return i;
+        const int64_t r = a.idx[i];
+        return r >= 0 && r < a.n ? r : -1;
+    };
+    auto load = [&](int64_t batch, int g, U (&x)[Q][NC]) {
+        const int j = g * 32 * NC + lane;
+        if (!INDEX && (batch + 1) * Q <= a.nrows) {  // Q rows one after the other
+            const U *p = a.src + batch * Q * v + j;
+#pragma unroll
+            for (int q = 0; q < Q; ++q, p += v)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) x[q][c] = j + 32 * c < v ? p[32 * c] : (U)0;
+            return;
         }
-        const U *srow = a.src + r * v;
-        warp_copy<U>(in, srow, v);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int64_t r = source(batch, q);
+            const U *p = a.src + (r < 0 ? 0 : r) * v + j;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) x[q][c] = r >= 0 && j + 32 * c < v ? p[32 * c] : (U)0;
+        }
+    };
+    // fixed-stride rows of whole 16-byte blocks, at most one per lane
+    const int n16 = v * (int)sizeof(U) / 16;
+    const bool blocks = ONE && a.out && n16 <= 32 && v * (int)sizeof(U) % 16 == 0 &&
+                        (((uintptr_t)a.out) & 15) == 0;
+    U x[Q][NC];
+    if (warp < batches) load(warp, 0, x);
+    for (int64_t batch = warp; batch < batches; batch += nwarps) {
+        uint32_t at[Q];  // stream bits so far
+#pragma unroll
+        for (int q = 0; q < Q; ++q) at[q] = stream0;
+        for (int g = 0; g < groups; ++g) {
+            U y[Q][NC];
+            const bool more = g + 1 < groups;
+            if (more || batch + nwarps < batches)
+                load(more ? batch : batch + nwarps, more ? g + 1 : 0, y);
+            if (!ONE) t.load(a.t, v, (int64_t)g * 32 * NC);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                uint32_t hi[NC], lo[NC], off[NC], bal[NC];
+                bool cj[NC];
+                uint32_t every = 0xffffffffu;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    uint32_t h[H];
+                    PackTables<U, NC>::split(x[q][c], h);
+                    uint32_t e = (h[0] & t.m[c][0]) ^ t.bv[c][0];
+                    if (H == 2) e |= (h[H - 1] & t.m[c][H - 1]) ^ t.bv[c][H - 1];
+                    cj[c] = e == 0;
+                    bal[c] = __ballot_sync(0xffffffffu, cj[c]);
+                    every &= bal[c];
+                    hi[c] = gather_left<LEVELS>(h[0], t.m[c][0], t.mv[c][0]);
+                    lo[c] = 0;
+                    if (H == 2) {
+                        const uint32_t l =
+                            gather_left<LEVELS>(h[H - 1], t.m[c][H - 1], t.mv[c][H - 1]);
+                        hi[c] |= __funnelshift_rc(l, 0, t.nbh[c]);
+                        lo[c] = __funnelshift_rc(0, l, t.nbh[c]);
+                    }
+                    off[c] = at[q] + t.before[c];
+                }
+                if (every == 0xffffffffu) {
+                    at[q] += t.all;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const uint32_t len = cj[c] ? t.nb[c] : (uint32_t)W;
+                        uint32_t incl = len;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t z = __shfl_up_sync(0xffffffffu, incl, o);
+                            if (lane >= o) incl += z;
+                        }
+                        off[c] = at[q] + incl - len;
+                        at[q] += __shfl_sync(0xffffffffu, incl, 31);
+                        uint32_t h[H];
+                        PackTables<U, NC>::split(x[q][c], h);
+                        hi[c] = cj[c] ? hi[c] : h[0];
+                        if (H == 2) lo[c] = cj[c] ? lo[c] : h[H - 1];
+                    }
+                }
+                // the group's bitmap units, LSB-first, in memory order (units past the row's
+                // last are zero and belong to the stream, where an OR of nothing does no harm)
+                uint32_t mine = 0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (lane == c) mine = bal[c] & t.valid[c];
+                const uint32_t image = images_at + q * image_units * 4;
+                or_shared(image + (uint32_t)((g * NC + (lane & (NC - 1))) ^ (H - 1)) * 4, mine);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) put_bits<U>(image, off[c], hi[c], lo[c]);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) x[q][c] = y[q][c];
+        }
         __syncwarp();
-        uint32_t s = 0;
-        for (int64_t j = lane; j < v; j += 32) {
-            const U m = __ldg(&a.t.mask[j]);
-            if ((U)(in[j] & m) == __ldg(&a.t.bitval[j])) s += popc_w(m);
+        unsigned packed = 0;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int64_t i = batch * Q + q;
+            if (i >= a.nrows) break;
+            const int64_t r = source(batch, q);
+            uint32_t *image = images + q * image_units;
+            // bitmap and stream in whole words; stored compressed only when below the raw row
+            const int words = (int)((at[q] + W - 1) / W);
+            if (r >= 0 && words < v) {
+                packed |= 1u << q;
+                if (blocks) {
+                    if (lane < n16) {
+                        uint4 *b4 = reinterpret_cast<uint4 *>(image) + lane;
+                        const uint4 x = *b4;
+                        *b4 = make_uint4(0, 0, 0, 0);
+                        reinterpret_cast<uint4 *>(a.out + i * v)[lane] =
+                            H == 2 ? make_uint4(x.y, x.x, x.w, x.z) : x;
+                    }
+                } else if (a.out)
+                    write_image<U>(a.out + i * v, image, v);
+                else
+                    write_image<U>(reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
+                                                         (i ? a.offsets[i - 1] : 0)),
+                                   image, words);
+                continue;
+            }
+            if (r >= 0) {
+                if (!a.out)
+                    warp_copy<U>(reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
+                                                       (i ? a.offsets[i - 1] : 0)),
+                                 a.src + r * v, v);
+                else if (!a.in_place)
+                    warp_copy<U>(a.out + i * v, a.src + r * v, v);
+            } else if (lane == 0) {
+                atomicOr(a.status, kStatusBadIndex);
+            }
+            for (int k = lane; k < words * H; k += 32) image[k] = 0;
         }
-        s = __reduce_add_sync(0xffffffffu, s);
-        const int64_t size = compressed_bytes(v, (int)sizeof(U), s);
-        const bool comp = size < vb;
-        if (comp) {
-            for (int64_t k = lane; k < a.row_words; k += 32) outw[k] = 0;
-            __syncwarp();
-            pack_row_warp<U>(in, v, a.t, out_units);
-            __syncwarp();
-        }
-        if (a.out) {
-            U *orow = a.out + i * v;
-            if (comp)
-                warp_copy<U>(orow, outw, v);
-            else if (!a.in_place)
-                warp_copy<U>(orow, in, v);
-            if (lane == 0 && comp) atomicOr(&a.bitmask[i >> 5], (int32_t)(1u << (i & 31)));
-        } else {
-            const int64_t start = i ? a.offsets[i - 1] : 0;
-            U *orow = reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) + start);
-            if (comp)
-                warp_copy<U>(orow, outw, size / (int64_t)sizeof(U));
-            else
-                warp_copy<U>(orow, in, v);
-        }
+        // Q divides 32 and the batch starts at a multiple of Q: one bitmask word
+        if (a.out && packed && lane == 0)
+            atomicOr(&a.bitmask[batch * Q >> 5], (int32_t)(packed << (batch * Q & 31)));
         __syncwarp();
     }
 }
 
-template <typename U>
-static int pack_warps_per_block(int64_t row_words, size_t &smem) {
-    const size_t per_warp = 2 * (size_t)row_words * sizeof(U);
-    const size_t budget = 96 * 1024;
-    int w = (int)(budget / per_warp);
-    if (w > 8) w = 8;
-    if (w < 1) w = 1;
-    smem = per_warp * w;
-    return w;
+// Bound: the integer pipe (three operations per move and 32-bit half) and the shared atomics,
+// then HBM.  600k rows of 64 64-bit words: 459 us with tables read through L1 and the row staged
+// and packed in two passes; 317 with tables in registers; 207 with 32-bit indices and images in
+// stream order; 188 with the moves chosen once; 163 without a test per atomic (its branches cost
+// more than the atomics of zeros); 140 now with the 16-byte epilogue, 4.0 TB/s.  Rows whose
+// tables stay in registers choose their moves once (LEVELS 2 covers masks that drop at most
+// three bits above any kept one, as quantised floats do).
+template <typename U, int NC, int Q, bool ONE, bool INDEX>
+__global__ void __launch_bounds__(256, 2) pack_rows_kernel(PackArgs<U> a) {
+    PackTables<U, NC> t;
+    if (ONE) {
+        t.load(a.t, a.v, 0);
+        if (t.levels <= 2) {
+            pack_rows<U, NC, Q, ONE, INDEX, 2>(a, t);
+            return;
+        }
+    }
+    pack_rows<U, NC, Q, ONE, INDEX, kMoves>(a, t);
+}
+
+template <typename U, int NC, int Q, bool ONE>
+static ibp_status launch_pack_q(const PackArgs<U> &a, int warps, size_t smem, cudaStream_t st) {
+    auto kern = a.idx ? pack_rows_kernel<U, NC, Q, ONE, true> : pack_rows_kernel<U, NC, Q, ONE, false>;
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, warps * 32, smem, &per_sm));
+    const int64_t batches = (a.nrows + Q - 1) / Q;
+    const int64_t blocks =
+        std::min<int64_t>((batches + warps - 1) / warps, (int64_t)device_sm_count() * per_sm);
+    kern<<<(unsigned)blocks, warps * 32, smem, st>>>(a);
+    IBP_LAUNCHED("pack_rows_kernel");
+    return IBP_OK;
 }
 
 template <typename U>
 static ibp_status launch_pack(PackArgs<U> a, cudaStream_t st) {
     if (a.nrows <= 0) return IBP_OK;
-    a.row_words = (int64_t)align_up((size_t)a.v + 4, 4);
-    size_t smem = 0;
-    const int wpb = pack_warps_per_block<U>(a.row_words, smem);
     const int maxs = device_max_smem_optin();
-    if ((int64_t)smem > maxs) {
+    // the longest rows packed: two raw rows of shared memory (an image can grow past the raw
+    // row by its bitmap before it is found incompressible)
+    if ((int64_t)(2 * align_up((size_t)a.v + 4, 4) * sizeof(U)) > maxs) {
         set_error("rows of %lld words do not fit the packer's shared-memory staging",
                   (long long)a.v);
         return IBP_ERR_UNSUPPORTED;
     }
-    auto kern = pack_rows_kernel<U>;
-    int per_sm = 0;
-    IBP_RET(kernel_blocks_per_sm((const void *)kern, wpb * 32, smem, &per_sm));
-    int64_t blocks = (a.nrows + wpb - 1) / wpb;
-    const int64_t cap = (int64_t)device_sm_count() * per_sm;
-    if (blocks > cap) blocks = cap;
-    kern<<<(unsigned)blocks, wpb * 32, smem, st>>>(a);
-    IBP_LAUNCHED("pack_rows_kernel");
-    return IBP_OK;
+    // bitmap and stream, and the units past them that an OR of no bits may touch
+    a.buf_words = (int64_t)align_up(
+        (size_t)(a.v + meta_bytes(a.v, sizeof(U)) / (int64_t)sizeof(U)) + 16 / sizeof(U),
+        16 / sizeof(U));
+    const size_t row = (size_t)a.buf_words * sizeof(U);
+    constexpr int NC = 16 / sizeof(U);  // 64 64-bit words or 128 32-bit words: 512 bytes
+    if (a.v <= 32) return launch_pack_q<U, 1, 4, true>(a, 8, 4 * 8 * row, st);
+    if (a.v <= 64) return launch_pack_q<U, 2, 4, true>(a, 8, 4 * 8 * row, st);
+    if (a.v <= 32 * NC) return launch_pack_q<U, NC, 4, true>(a, 8, 4 * 8 * row, st);
+    // longer rows: 4 rows share a load of the tables while two blocks of 8 warps fit an SM,
+    // else 1 row and as many warps as fit
+    if (4 * 8 * row <= 100 * 1024) return launch_pack_q<U, NC, 4, false>(a, 8, 4 * 8 * row, st);
+    const int warps = (int)std::min<size_t>(8, (size_t)maxs / row);
+    return launch_pack_q<U, NC, 1, false>(a, warps, (size_t)warps * row, st);
 }
 
 template <typename U>

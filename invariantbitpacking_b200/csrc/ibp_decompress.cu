@@ -416,7 +416,7 @@ __device__ __forceinline__ void hbm_decode_group(const U *__restrict__ buf, int 
             if (j < v) {
                 const bool cj = (cjm >> (q * NC + c)) & 1u;
                 const U y = stream_bits_ending<U>(stream, (int32_t)((c ? t0 : 0u) + incl[q][c]));
-                o[j] = cj ? (U)(lt.bv[c] | scatter_regs<U>(y, (U)~lt.m[c], lt.mv[c])) : y;
+                o[j] = cj ? lt.word(y, c) : y;
             }
         }
     }

@@ -56,9 +56,9 @@ __device__ __forceinline__ void issue_words(U *__restrict__ slot, const U *__res
 // through L1 from the workspace copy (NC = 0, any row length).
 template <typename U, int NC>
 struct LaneTables {
-    static constexpr int LW = LogW<U>::value;
-    U m[NC > 0 ? NC : 1], bv[NC > 0 ? NC : 1], mv[NC > 0 ? NC : 1][LW];
-    int nb[NC > 0 ? NC : 1];
+    static constexpr int N = NC > 0 ? NC : 1;
+    U m[N], bv[N], mv[N][kMoves];
+    int nb[N], nbl[N];  // kept bits of the word, of its low half
 
     __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v) {
         const int lane = threadIdx.x & 31;
@@ -68,23 +68,19 @@ struct LaneTables {
             const bool in = j < v;
             m[c] = in ? t.mask[j] : (U)0;
             bv[c] = in ? t.bitval[j] : (U)0;
-            nb[c] = in ? (int)t.nb[j] : 0;
+            const int k = in ? (int)t.nb[j] : 0;
+            nb[c] = k & 0xff;
+            nbl[c] = k >> 8;
 #pragma unroll
-            for (int i = 0; i < LW; ++i) mv[c][i] = in ? t.mv[i * v + j] : (U)0;
+            for (int i = 0; i < kMoves; ++i) mv[c][i] = in ? t.mv[i * v + j] : (U)0;
         }
     }
-};
 
-template <typename U>
-__device__ __forceinline__ U scatter_regs(U y, U sel, const U *mv) {
-    constexpr int LW = LogW<U>::value;
-#pragma unroll
-    for (int i = LW - 1; i >= 0; --i) {
-        const U t = (U)(y << (1 << i));
-        y = (U)((y & ~mv[i]) | (t & mv[i]));
+    // the word of column 32 * c + lane whose kept bits are the low bits of y
+    __device__ __forceinline__ U word(U y, int c) const {
+        return scatter_word<U>(y, m[c], bv[c], nbl[c], mv[c]);
     }
-    return (U)(y & sel);
-}
+};
 
 // Decode one compressed row from its shared-memory slot (bitmap at word 0, stream at word
 // mw, zero words after the stream) into the output row.  Lane j of a 32-word chunk takes
@@ -118,7 +114,7 @@ __device__ __forceinline__ void decode_row(const U *__restrict__ buf, int64_t v,
             }
             if (in) {
                 const U y = get_bits<U>(stream, base + incl - L, L);
-                orow[j] = cj ? (U)(lt.bv[c] | scatter_regs<U>(y, (U)~lt.m[c], lt.mv[c])) : y;
+                orow[j] = cj ? lt.word(y, c) : y;
             }
             base += __shfl_sync(0xffffffffu, incl, 31);
         }
@@ -139,7 +135,7 @@ __device__ __forceinline__ void decode_row(const U *__restrict__ buf, int64_t v,
                 in[c] = j < v;
                 m[c] = in[c] ? __ldg(&t.mask[j]) : (U)0;
                 bv[c] = in[c] ? __ldg(&t.bitval[j]) : (U)0;
-                const int nb = in[c] ? (int)__ldg(&t.nb[j]) : 0;
+                const int nb = in[c] ? (int)__ldg(&t.nb[j]) & 0xff : 0;
                 maxnb = max(maxnb, nb);
                 cj[c] = in[c] && ((units[j >> 5] >> (j & 31)) & 1u);
                 incl[c] = in[c] ? (cj[c] ? nb : W) : 0;
@@ -185,8 +181,14 @@ __device__ __forceinline__ void decode_row(const U *__restrict__ buf, int64_t v,
                     const int64_t j = g0 + 32 * c + lane;
                     if (in[c]) {
                         const U y = stream_bits_ending<U>(gs, off + incl[c]);
-                        orow[j] = cj[c] ? (U)(bv[c] | scatter_bits<U>(y, (U)~m[c], t.mv + j, (int)v))
-                                        : y;
+                        U x = y;
+                        if (cj[c]) {
+                            U mv[kMoves];
+#pragma unroll
+                            for (int i = 0; i < kMoves; ++i) mv[i] = __ldg(&t.mv[i * v + j]);
+                            x = scatter_word<U>(y, m[c], bv[c], (int)__ldg(&t.nb[j]) >> 8, mv);
+                        }
+                        orow[j] = x;
                     }
                     off += __shfl_sync(0xffffffffu, incl[c], 31);
                 }
@@ -248,7 +250,7 @@ __device__ __forceinline__ void decode_rows_multi(const U *__restrict__ slots,
             const int L = in ? (cj ? lt.nb[c] : W) : 0;
             if (in) {
                 const U y = get_bits<U>(stream, base + incl[q][c] - L, L);
-                o[q][j] = cj ? (U)(lt.bv[c] | scatter_regs<U>(y, (U)~lt.m[c], lt.mv[c])) : y;
+                o[q][j] = cj ? lt.word(y, c) : y;
             }
             base += __shfl_sync(0xffffffffu, incl[q][c], 31);
         }
@@ -272,7 +274,8 @@ __device__ __forceinline__ int64_t row_words(const U *__restrict__ buf, int64_t 
         }
     } else {
         for (int64_t j = lane; j < v; j += 32)
-            bits += ((units[j >> 5] >> (j & 31)) & 1u) ? (uint32_t)__ldg(&t.nb[j]) : (uint32_t)W;
+            bits += ((units[j >> 5] >> (j & 31)) & 1u) ? (uint32_t)__ldg(&t.nb[j]) & 0xffu
+                                                        : (uint32_t)W;
     }
     bits = __reduce_add_sync(0xffffffffu, bits);
     return mw + (bits + W - 1) / W;

@@ -1,8 +1,9 @@
 // ibp_match.cuh -- which words of a row match the invariant bits, and how many bits that
 // saves: the inner loop of the size pass and of the threshold check.
 //
-// A lane takes A bytes of a row at a time (16 where rows allow it) and keeps the mask, the
-// values and the masks' set bits of those columns in registers while several rows pass by.
+// A lane takes pieces of A bytes of a row (16 where rows allow it, else several smaller ones,
+// each G pieces after the last) and keeps the mask, the values and the masks' set bits of those
+// columns in registers while several rows pass by.
 // Words of 1 and 2 bytes are compared four and two to a register: a byte (or half) of
 // e = (x & mask) ^ value is zero exactly where its top bit stays clear in
 // ((e & 0x7f..) + 0x7f..) | e, and a byte dot product adds up the set bits of the matches.
@@ -21,41 +22,61 @@ __device__ __forceinline__ void add_if_zero(uint32_t &s, uint32_t d, uint32_t pc
         : "r"(d), "r"(pc), "r"(one));
 }
 
-template <typename U, int A>
+template <typename U, int A, int G>
 struct Chunk {
     static constexpr int WB = sizeof(U);
-    static constexpr int NR = A >= 4 ? A / 4 : 1;           // registers of A bytes
-    static constexpr int NW = WB == 8 ? NR / 2 : NR;        // set-bit counts (bytes of one for WB < 4)
-    static_assert(A >= WB && (A & (A - 1)) == 0 && A <= 16, "chunk size");
+    static constexpr int NS = A == 16 ? 1 : (A == 8 ? 2 : 4);  // pieces
+    static constexpr int PR = A >= 4 ? A / 4 : 1;              // registers of a piece
+    static constexpr int NR = NS * PR;
+    static constexpr int NW = WB == 8 ? NR / 2 : NR;  // set-bit counts (bytes of one for WB < 4)
+    static_assert(A >= WB && (A & (A - 1)) == 0 && A <= 16, "piece size");
 
-    static __device__ __forceinline__ void load(const void *p, uint32_t (&x)[NR]) {
-        if constexpr (A == 16) {
-            const uint4 y = *reinterpret_cast<const uint4 *>(p);
-            x[0] = y.x, x[1] = y.y, x[2] = y.z, x[3] = y.w;
-        } else if constexpr (A == 8) {
-            const uint2 y = *reinterpret_cast<const uint2 *>(p);
-            x[0] = y.x, x[1] = y.y;
-        } else if constexpr (A == 4) {
-            x[0] = *reinterpret_cast<const uint32_t *>(p);
-        } else if constexpr (A == 2) {
-            x[0] = *reinterpret_cast<const uint16_t *>(p);
-        } else {
-            x[0] = *reinterpret_cast<const uint8_t *>(p);
+    // Pieces c, c + G, ... of a row of `pieces`; those past the end are zero.
+    static __device__ __forceinline__ void load(const char *row, int64_t c, int64_t pieces,
+                                                uint32_t (&x)[NR]) {
+        const char *p = row + c * A;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            uint32_t *y = x + k * PR;
+#pragma unroll
+            for (int i = 0; i < PR; ++i) y[i] = 0;
+            if (c + k * G < pieces) {
+                if constexpr (A == 16) {
+                    const uint4 z = *reinterpret_cast<const uint4 *>(p);
+                    y[0] = z.x, y[1] = z.y, y[2] = z.z, y[3] = z.w;
+                } else if constexpr (A == 8) {
+                    const uint2 z = *reinterpret_cast<const uint2 *>(p + k * G * A);
+                    y[0] = z.x, y[1] = z.y;
+                } else if constexpr (A == 4) {
+                    y[0] = *reinterpret_cast<const uint32_t *>(p + k * G * A);
+                } else if constexpr (A == 2) {
+                    y[0] = *reinterpret_cast<const uint16_t *>(p + k * G * A);
+                } else {
+                    y[0] = *reinterpret_cast<const uint8_t *>(p + k * G * A);
+                }
+            }
         }
     }
 
-    // masks, values and the like start at any multiple of the word size
-    static __device__ __forceinline__ void load_words(const U *p, uint32_t (&x)[NR]) {
+    // the same columns' masks or values, which start at any multiple of the word size
+    static __device__ __forceinline__ void load_words(const U *p, int64_t c, int64_t pieces,
+                                                      uint32_t (&x)[NR]) {
 #pragma unroll
-        for (int i = 0; i < NR; ++i) x[i] = 0;
+        for (int k = 0; k < NS; ++k) {
+            uint32_t *y = x + k * PR;
 #pragma unroll
-        for (int j = 0; j < A / WB; ++j) {
-            const U w = __ldg(p + j);
-            if constexpr (WB == 8) {
-                x[2 * j] = (uint32_t)w;
-                x[2 * j + 1] = (uint32_t)(w >> 32);
-            } else {
-                x[j * WB / 4] |= (uint32_t)w << (8 * (j * WB % 4));
+            for (int i = 0; i < PR; ++i) y[i] = 0;
+            if (c + k * G < pieces) {
+#pragma unroll
+                for (int j = 0; j < A / WB; ++j) {
+                    const U w = __ldg(p + (c + k * G) * (A / WB) + j);
+                    if constexpr (WB == 8) {
+                        y[2 * j] = (uint32_t)w;
+                        y[2 * j + 1] = (uint32_t)(w >> 32);
+                    } else {
+                        y[j * WB / 4] |= (uint32_t)w << (8 * (j * WB % 4));
+                    }
+                }
             }
         }
     }
@@ -148,8 +169,8 @@ constexpr int group_sums_copies() {
     return G > N ? G / N : 1;
 }
 
-// Largest chunk (16, 4 or the word itself; 8 for 64-bit words) that divides every row's start.
-inline int row_chunk_bytes(const void *base, int64_t v, int wb) {
+// Largest piece (16, 4 or the word itself; 8 for 64-bit words) that divides every row's start.
+inline int row_piece_bytes(const void *base, int64_t v, int wb) {
     const uint64_t a = (uint64_t)(uintptr_t)base | (uint64_t)(v * wb);
     if ((a & 15) == 0) return 16;
     if (wb == 8) return (a & 7) == 0 ? 8 : 0;

@@ -164,7 +164,7 @@ masks_from_counts_kernel(const uint32_t *__restrict__ counts, int64_t n, int64_t
 // In the sweep the masks are nested: thr * N rises and (1 - thr) * N falls with thr, so a bit
 // invariant at one threshold is so at every lower one, with the same value (all thresholds are
 // above one half); a word matches at threshold t exactly when (x ^ bitval_0) & mask_t is 0.
-// Rows as in the size pass (G lanes, chunks of A bytes, Q rows in flight), tables in registers.
+// Rows as in the size pass (G lanes, pieces of A bytes, Q rows in flight), tables in registers.
 // PACK: S_t of a row fits 16 bits, two thresholds to a register in the sums over lanes.
 // Bound: the integer pipe, 3 operations per word and threshold there and one on the
 // multiply-add pipe (600k rows of 64 64-bit words, 7 thresholds: 550 us with 14 table loads per
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256, 2)
 check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
                    const U *__restrict__ masks, const U *__restrict__ bitvals,
                    unsigned long long *__restrict__ saved, uint32_t one) {
-    using C = Chunk<U, A>;
+    using C = Chunk<U, A, G>;
     constexpr int RPW = 32 / G;
     constexpr int Q = T > 1 ? 4 : 8;
     constexpr int S = T > 1 ? (PACK ? 4 : 8) : 1;  // sums per row
@@ -191,11 +191,11 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
     const int64_t chunks = row_bytes / A;
     uint32_t b[C::NR], m[T][C::NR], pc[T][C::NW];
     auto tables = [&](int64_t c) {
-        C::load_words(bitvals + c * (A / (int)sizeof(U)), b);
+        C::load_words(bitvals, c, chunks, b);
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             if (t < nthr) {
-                C::load_words(masks + t * v + c * (A / (int)sizeof(U)), m[t]);
+                C::load_words(masks + t * v, c, chunks, m[t]);
             } else {
 #pragma unroll
                 for (int i = 0; i < C::NR; ++i) m[t][i] = 0;  // saves nothing
@@ -206,7 +206,8 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
                 C::set_bits(m[t], pc[t]);
         }
     };
-    const int64_t steps = (chunks + G - 1) / G;  // per row
+    constexpr int SP = G * C::NS;  // pieces of a step
+    const int64_t steps = (chunks + SP - 1) / SP;  // per row
     if (steps == 1 && sub < chunks) tables(sub);
     unsigned long long acc[L][PACK ? 2 : 1];
 #pragma unroll
@@ -219,16 +220,10 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
     const int64_t batches = (n + RPW * Q - 1) / (RPW * Q);
     auto load = [&](int64_t batch, int64_t c, uint32_t (&x)[Q][C::NR]) {
         const int64_t r0 = batch * (RPW * Q) + gin;
-        const char *p = reinterpret_cast<const char *>(data) + r0 * row_bytes + c * A;
+        const char *p = reinterpret_cast<const char *>(data) + r0 * row_bytes;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            if (c < chunks && r0 + q * RPW < n) {
-                C::load(p + q * RPW * row_bytes, x[q]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < C::NR; ++i) x[q][i] = 0;
-            }
-        }
+        for (int q = 0; q < Q; ++q)
+            C::load(p + q * RPW * row_bytes, c, r0 + q * RPW < n ? chunks : 0, x[q]);
     };
     uint32_t x[Q][C::NR];
     int64_t batch = batches - 1 - warp;
@@ -239,10 +234,10 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
         for (int i = 0; i < Q * S; ++i) f[i] = 0;
         const int64_t left = n - (batch * (RPW * Q) + gin);  // rows of this group's, every RPW-th
         for (int64_t k = 0; k < steps; ++k) {
-            const int64_t c = k * G + sub;
+            const int64_t c = k * SP + sub;
             uint32_t y[Q][C::NR];
             const bool more = k + 1 < steps;
-            if (more || batch >= nwarps) load(more ? batch : batch - nwarps, more ? c + G : sub, y);
+            if (more || batch >= nwarps) load(more ? batch : batch - nwarps, more ? c + SP : sub, y);
             if (steps > 1 && c < chunks) tables(c);
             if (c < chunks) {
 #pragma unroll
@@ -303,7 +298,7 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
 template <typename U, int A>
 static ibp_status launch_check(const U *data, int64_t n, int64_t v, int nthr, const U *masks,
                                const U *bitvals, unsigned long long *saved, cudaStream_t st) {
-    const bool narrow = v * (int64_t)sizeof(U) <= 8 * A;
+    const bool narrow = v * (int64_t)sizeof(U) <= 8 * A * Chunk<U, A, 8>::NS;
     const bool pack = v * 8 * (int64_t)sizeof(U) < 65536;
     auto kern = nthr == 1 ? (narrow ? check_saved_kernel<U, A, 8, 1, false>
                                     : check_saved_kernel<U, A, 32, 1, false>)
@@ -438,7 +433,7 @@ ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold,
         IBP_LAUNCHED("masks_from_counts_kernel");
         if (n > 0) {
             const U *rows = stage ? stage : data;
-            const int a = row_chunk_bytes(rows, v, wb);
+            const int a = row_piece_bytes(rows, v, wb);
             if (a == 16)
                 IBP_RET((launch_check<U, 16>(rows, n, v, thr.count, masks, bitvals, saved, st)));
             else if (a == 4 && wb < 4)

@@ -1,5 +1,5 @@
-"""preprocess and get_compress_size against the CPU oracle at the edges of their row chunks:
-every word size, rows of one chunk and of many, rows that are no whole number of 16- or 4-byte
+"""preprocess and get_compress_size against the CPU oracle at the edges of their row pieces:
+every word size, rows of one piece and of many, rows that are no whole number of 16- or 4-byte
 chunks, groups of rows that are and the rows left over, row sums past 16 bits, and datasets
 that do not start on a 16-byte boundary.  Outputs are integers and must be equal."""
 import numpy as np
