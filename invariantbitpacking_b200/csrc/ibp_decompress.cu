@@ -16,10 +16,11 @@
 //    slot decodes straight from its source.
 //  * decode: lane j of a 32-word chunk takes its bit length, a warp prefix sum gives its
 //    stream offset, a funnel read pulls its bits and the Hacker's Delight scatter places
-//    them at the non-invariant positions (log2(W) branch-free steps).  For rows of up to 64
-//    words the per-column tables (mask, bitval, kept bits, move masks) live in registers,
-//    loaded once per warp; longer rows read them through the L1 cache, four chunks at a
-//    time, and place the bits of columns that keep at most 4 directly from the mask.
+//    them at the non-invariant positions (five branch-free steps per 32-bit half).  For rows of
+//    up to 64 words the per-column tables (mask, bitval, kept bits, move masks) live in
+//    registers, loaded once per warp; longer host rows read them through the L1 cache, four
+//    chunks at a time, and place the bits of columns that keep at most 4 directly from the
+//    mask; longer device rows load them once for up to 16 rows decoded together.
 //  * index arrays: each distinct row crosses the link once.  Dense batches of host rows (a
 //    quarter of the rows or more) and raw gathers are fetched in sorted index order (cub
 //    radix sort on only the bits the row count needs) so concurrent warps read neighbouring
@@ -59,11 +60,10 @@ struct FetchArgs {
     int slots;            // row slots per warp (<= kRowsInFlight)
     int upos;             // positions per chunk the grid was sized for (unit_positions)
     int gmax;             // largest chunk a warp takes (positions); 0: its row slots
-    bool async_rows;      // rows in device memory: first reads as asynchronous copies
     bool device_rows;     // rows in device memory
     ClaimTable claims;    // in-fetch claims (keys == nullptr: none); repeats are copied
                           // inside the fetch
-    const int64_t *list;  // positions to fetch (claimed heads), or nullptr: all positions
+    const longlong2 *list;  // head records of the claim pass, or nullptr: all positions
     const unsigned long long *list_len;  // entries of `list` (device)
 };
 
@@ -75,18 +75,17 @@ constexpr uint64_t kRecordPacked = 1ull << 63;  // head record: the row is store
 // appended to `heads` (one atomic per block and pass, so the list's counter is not a hot
 // spot), and the fetch kernel then walks distinct rows only, 32 to a chunk.  Out-of-range
 // rows are flagged here and never claimed.  256 threads per block, P positions each.
-// bitmask != nullptr: each listed head is a record of two words, its position (bit 63 set
-// when the row is stored compressed) and its row, so that a fetch reads one 16-byte record
-// per row instead of a position, then the index entry it points to, then the bitmask word.
+// Each listed head is a record of two words, its position (bit 63 set when the row is stored
+// compressed; condensed rows have no bitmask) and its row, so that a fetch reads one 16-byte
+// record per row instead of a position, then the index entry it points to, then the bitmask word.
 // P positions per thread and pass: 2 when one position per thread would need more than one
 // wave of resident blocks (fewer block-wide rounds), else 1 (more blocks for small batches).
 template <int P>
 __global__ void __launch_bounds__(256)
 claim_heads_kernel(const int64_t *__restrict__ idx, int64_t nidx, int64_t n, int64_t *hkeys,
-                   int64_t *hpos, int64_t hslots, int64_t *__restrict__ heads,
+                   int64_t *hpos, int64_t hslots, longlong2 *__restrict__ heads,
                    unsigned long long *nheads, int32_t *status,
                    const int32_t *__restrict__ bitmask) {
-    const bool records = bitmask != nullptr;
     __shared__ unsigned counts[8];
     __shared__ unsigned long long block_base;
     // the block's own table of the rows its 256 x P positions hold (empty: ~0), so that a hot
@@ -120,7 +119,7 @@ claim_heads_kernel(const int64_t *__restrict__ idx, int64_t nidx, int64_t n, int
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             // the row's bitmask word, loaded before the claim so that the latencies overlap
-            bmw[p] = records && ok[p] ? __ldg(&bitmask[key[p] >> 5]) : 0;
+            bmw[p] = bitmask && ok[p] ? __ldg(&bitmask[key[p] >> 5]) : 0;
         }
         unsigned hm[P];
         unsigned total = 0;
@@ -166,10 +165,9 @@ claim_heads_kernel(const int64_t *__restrict__ idx, int64_t nidx, int64_t n, int
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const unsigned long long my = at + __popc(hm[p] & below);
-            if (head[p] && !records) heads[my] = k[p];
-            if (head[p] && records) {
+            if (head[p]) {
                 const bool packed = (bmw[p] >> (key[p] & 31)) & 1;
-                reinterpret_cast<longlong2 *>(heads)[my] = make_longlong2(
+                heads[my] = make_longlong2(
                     packed ? (int64_t)((uint64_t)k[p] | kRecordPacked) : k[p], key[p]);
             }
             at += __popc(hm[p]);
@@ -240,28 +238,25 @@ static ibp_status launch_fill_hashed(const int64_t *idx, int64_t nidx, int64_t n
 }
 
 // ------------------------------------------------------------------ fetch kernel
+// Rows in host memory, and raw gathers.
 // EXACT: condensed rows (byte ranges from a.s.offsets) instead of fixed-stride rows.
-// ASYNC: fixed-stride rows in device memory, first reads double-buffered (fetch_heads_async;
-// each warp owns two sets of a.slots slots).
 // RAW: rows stored raw may be staged with the first reads (rows of at most 1 KiB).
-template <typename U, int NC, bool EXACT, bool ASYNC, bool RAW>
+template <typename U, int NC, bool EXACT, bool RAW>
 __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<U> a) {
     extern __shared__ __align__(16) unsigned char smem[];
     // tables, counters, claim table and sorted keys come from the kernels before this one
     grid_dep_wait();
-    constexpr bool kClaims = !ASYNC;  // in-fetch claims: host rows (fixed-stride or condensed)
     const int lane = threadIdx.x & 31;
-    U *slots = reinterpret_cast<U *>(smem) +
-               (int64_t)(threadIdx.x >> 5) * a.slots * (ASYNC ? 2 : 1) * a.slot_words;
+    U *slots = reinterpret_cast<U *>(smem) + (int64_t)(threadIdx.x >> 5) * a.slots * a.slot_words;
     // in-fetch claims: 64 words per warp after all the row slots
     int64_t *claim = reinterpret_cast<int64_t *>(
-                         reinterpret_cast<U *>(smem) + (int64_t)(blockDim.x >> 5) * a.slots *
-                                                           (ASYNC ? 2 : 1) * a.slot_words) +
+                         reinterpret_cast<U *>(smem) +
+                         (int64_t)(blockDim.x >> 5) * a.slots * a.slot_words) +
                      (threadIdx.x >> 5) * 64;
     LaneTables<U, NC> lt;
     if (!a.raw_only) lt.load(a.s.t, a.s.v);
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
+    const int64_t nrows = a.nrows;
     int64_t seen = 0;  // positions handed out when this warp last took a chunk
     for (;;) {
         // guided self-scheduling: 32-position chunks while much work remains, shrinking to
@@ -276,9 +271,9 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
         const int64_t p0 = (int64_t)__shfl_sync(0xffffffffu, c, 0);
         if (p0 >= nrows) break;
         seen = p0 + g;
-        // lane-parallel metadata of the chunk's positions (list entries: claimed heads)
+        // lane-parallel metadata of the chunk's positions
         const bool valid = lane < g && p0 + lane < nrows;
-        const int64_t k = a.list ? (valid ? a.list[p0 + lane] : 0) : p0 + lane;
+        const int64_t k = p0 + lane;
         const int64_t k0 = p0;
         const int64_t key = valid ? (a.keys ? a.keys[k] : k) : -1;
         bool head = valid;
@@ -292,7 +287,7 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
         head = head && !bad;
         // in-fetch claims: one claim per distinct row of the chunk; the other lanes of that
         // row, and the lanes whose row was claimed earlier, are repeats
-        const bool claims = kClaims && a.claims.keys;
+        const bool claims = a.claims.keys != nullptr;
         bool rep = false;
         const bool out_row = head;  // lanes with an output row (heads before claiming)
         U *orow = a.out + (out_row ? (a.pos ? a.pos[k] : k) : 0) * a.s.v;
@@ -308,12 +303,8 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
             } else {
                 const bool packed = fetch_lane && !a.raw_only &&
                                     ((__ldg(&a.s.bitmask[key >> 5]) >> (key & 31)) & 1);
-                if constexpr (ASYNC)
-                    fetch_heads_async<U, NC>(a.s, lt, slots, a.slots, a.slot_words, key, orow,
-                                             fetch_lane, packed, a.status);
-                else
-                    fetch_heads<U, NC, RAW>(a.s, lt, slots, a.slots, a.slot_words, key, orow,
-                                       fetch_lane, packed, a.status);
+                fetch_heads<U, NC, RAW>(a.s, lt, slots, a.slots, a.slot_words, key, orow,
+                                        fetch_lane, packed, a.status);
             }
             if (!claims || pass > 0) break;
             fetch_lane = settle_chunk<U>(a.claims, claim, rep, a.s.v, a.status);
@@ -485,7 +476,7 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
         int64_t k = p0 + lane, key = k;
         int packed = 0;
         if (valid && a.list) {  // a head record of the claim pass: position and row
-            const longlong2 r = reinterpret_cast<const longlong2 *>(a.list)[p0 + lane];
+            const longlong2 r = a.list[p0 + lane];
             k = (int64_t)((uint64_t)r.x & ~kRecordPacked);
             key = r.y;
             packed = r.x < 0;
@@ -540,7 +531,7 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
 template <typename U>
 static bool hbm_rows_fit(const FetchArgs<U> &a) {
     return a.device_rows && !a.raw_only && !a.dedup && !a.pos && !a.s.offsets &&
-           !a.claims.keys && (!a.keys || a.list) && a.s.v <= 64 &&
+           (!a.keys || a.list) && a.s.v <= 64 &&
            (a.s.v * (int64_t)sizeof(U)) % 16 == 0 && (((uintptr_t)a.s.comp) & 15) == 0;
 }
 
@@ -563,6 +554,247 @@ static ibp_status launch_hbm_nc(FetchArgs<U> a, cudaStream_t st) {
     IBP_CUDA(launch_dependent(kern, (unsigned)blocks, threads, smem, st, a));
     IBP_LAUNCHED("hbm_rows_kernel");
     profile_end(slot, st);
+    return IBP_OK;
+}
+
+// ------------------------------------------------------------------ other HBM rows
+// Rows in device memory of any length and alignment, fixed-stride or condensed (EXACT): a warp
+// takes up to `slots` rows (the claim pass's head records, sorted positions, or rows p, p + 1,
+// ... of an unindexed fetch) at a time, lane q holding row q's metadata.  Their 16-byte
+// blocks go to shared-memory slots as asynchronous copies -- the first_words expected of a
+// fixed-stride row, all of a condensed one -- while the next rows' metadata is loaded; a
+// fixed-stride row that needs more gets its tail the same way, and the rows are decoded
+// together (decode_group).  One set of slots per warp: a decode takes several times a read's
+// latency and the SM's other warps hide that.  Rows of up to 512 bytes of columns (ONE) keep the
+// tables in registers for the whole kernel.
+// Bound: issue and the integer pipe (a 32-bit half takes five masked moves).  Whole sets: 100k
+// rows of 256 32-bit words at half the bits 174 -> 83 us, 40k rows of 512 64-bit words at a
+// quarter 254 -> 91 us; 50k condensed rows of 99 32-bit words 87 -> 45 us (a row at a time
+// before, with eight table loads a word).
+template <typename U, bool ONE, bool EXACT>
+__global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int W = 8 * sizeof(U), per16 = 16 / sizeof(U);
+    const int lane = threadIdx.x & 31;
+    const int64_t v = a.s.v, mw = a.s.mw;
+    const int sw = (int)a.slot_words;
+    U *slots = reinterpret_cast<U *>(smem) + (int64_t)(threadIdx.x >> 5) * a.slots * sw;
+    // tables, counters, head records and sorted keys come from the kernels before this one
+    grid_dep_wait();
+    grid_dep_release();
+    GroupTables<U> gt;
+    uint32_t packed_bits = 0;  // stream bits of a row whose words are all compressible
+    if constexpr (ONE) {
+        gt.load(a.s.t, v, 0);
+        packed_bits = gt.total;
+    } else {
+        for (int64_t j = lane; j < v; j += 32) packed_bits += (uint32_t)__ldg(a.s.t.nb + j) & 0xffu;
+        packed_bits = __reduce_add_sync(0xffffffffu, packed_bits);
+    }
+    const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
+    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    // rows at a time: fewer when the fetch does not fill every warp's slots
+    const int per = (int)max((int64_t)1, min((int64_t)a.slots, nrows / nwarps));
+    const int64_t units = (nrows + per - 1) / per;
+
+    // this lane's row of unit u: position and row ...
+    struct Head {
+        int64_t k, key;
+        bool ok, packed;
+    };
+    auto head_of = [&](int64_t u) {
+        Head h{0, -1, false, false};
+        const int64_t p = u * per + lane;
+        if (lane < per && p < nrows) {
+            h.k = h.key = p;
+            if (a.list) {
+                const longlong2 r = a.list[p];
+                h.k = (int64_t)((uint64_t)r.x & ~kRecordPacked);
+                h.packed = r.x < 0;
+                h.key = r.y;
+            } else if (a.keys) {
+                h.key = a.keys[p];
+                if (a.pos) h.k = a.pos[p];
+            }
+            h.ok = !(a.dedup && p > 0 && a.keys[p - 1] == h.key);
+        }
+        return h;
+    };
+    // ... then the bytes [lo, hi) of `comp` to read first
+    struct Bytes {
+        int64_t lo, hi;
+    };
+    auto bytes_of = [&](Head &h) {
+        Bytes b{0, 0};
+        if (!h.ok) return b;
+        if (h.key < 0 || h.key >= a.s.n) {
+            atomicOr(a.status, kStatusBadIndex);
+            h.ok = false;
+            return b;
+        }
+        if constexpr (EXACT) {
+            b.lo = h.key > 0 ? a.s.offsets[h.key - 1] : 0;
+            b.hi = a.s.offsets[h.key];
+            if (b.lo < 0 || b.hi < b.lo || b.hi > a.s.comp_bytes ||
+                b.hi - b.lo > v * (int64_t)sizeof(U) ||
+                ((b.lo | b.hi) % (int64_t)sizeof(U)) != 0) {
+                atomicOr(a.status, kStatusCorruptRow);  // not a row's range: no read leaves comp
+                h.ok = false;
+                return Bytes{0, 0};
+            }
+            h.packed = b.hi - b.lo != v * (int64_t)sizeof(U);
+        } else {
+            if (!a.list) h.packed = (__ldg(&a.s.bitmask[h.key >> 5]) >> (h.key & 31)) & 1;
+            b.lo = h.key * v * (int64_t)sizeof(U);
+            b.hi = b.lo + (h.packed ? a.s.first_words : v) * (int64_t)sizeof(U);
+        }
+        return b;
+    };
+    // the 16-byte blocks of [from, to) into the slot whose first block is that of `lo`
+    const uintptr_t comp = (uintptr_t)a.s.comp;
+    auto copy_blocks = [&](U *slot, uintptr_t lo, uintptr_t from, uintptr_t to) {
+        const uintptr_t b0 = from & ~(uintptr_t)15;
+        const int n = (int)((to + 15 - b0) >> 4);
+        const char *src = reinterpret_cast<const char *>(b0) + lane * 16;
+        char *dst = reinterpret_cast<char *>(slot) + (b0 - (lo & ~(uintptr_t)15)) + lane * 16;
+        for (int i = lane; i < n; i += 32, src += 512, dst += 512) cp_async16(dst, src);
+    };
+
+    int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    Head cur = head_of(u), next = head_of(u + nwarps);
+    Bytes cb = bytes_of(cur);
+    for (; u < units; u += nwarps) {
+        // this lane's row: output, first byte, words read, place in the slots
+        U *const out = a.out + cur.k * v;
+        const uintptr_t lo = comp + cb.lo;
+        const int64_t len = (cb.hi - cb.lo) / (int64_t)sizeof(U);
+        const int place = lane * sw + (int)((lo & 15) / sizeof(U));
+        const bool fits = len + 2 * per16 <= sw;
+        unsigned pm = __ballot_sync(0xffffffffu, cur.ok && cur.packed);
+        const unsigned rm = __ballot_sync(0xffffffffu, cur.ok && !cur.packed && fits);
+        unsigned wide = __ballot_sync(0xffffffffu, cur.ok && !cur.packed && !fits);
+#pragma unroll 1
+        for (unsigned m = pm | rm; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            const uintptr_t l = __shfl_sync(0xffffffffu, (unsigned long long)lo, q);
+            const int64_t n = __shfl_sync(0xffffffffu, len, q);
+            copy_blocks(slots + q * sw, l, l, l + n * (int64_t)sizeof(U));
+        }
+        cp_async_commit();
+        cur = next;
+        cb = bytes_of(cur);
+        next = head_of(u + 2 * nwarps);
+        for (; wide; wide &= wide - 1) {  // rows stored raw that are longer than a slot
+            const int q = __ffs(wide) - 1;
+            const uintptr_t l = __shfl_sync(0xffffffffu, (unsigned long long)lo, q);
+            U *o = reinterpret_cast<U *>(
+                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), q));
+            warp_copy<U>(o, reinterpret_cast<const U *>(l), v);
+        }
+        cp_async_wait_all();
+        __syncwarp();
+        // lengths
+        int64_t end = 0;
+#pragma unroll 1
+        for (unsigned m = pm; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            const uint32_t bits = row_stream_bits<U>(slots + __shfl_sync(0xffffffffu, place, q), v,
+                                                     a.s.t, packed_bits);
+            if (lane == q) end = mw + (int64_t)((bits + W - 1) / W);
+        }
+        // a bitmap whose stream does not fit its row cannot come from this mask: report it and
+        // leave the output row alone
+        const bool packed = (pm >> lane) & 1u;
+        const bool corrupt = packed && (EXACT ? end > len : end >= v);
+        if (corrupt) atomicOr(a.status, kStatusCorruptRow);
+        pm &= ~__ballot_sync(0xffffffffu, corrupt);
+        if constexpr (!EXACT) {
+            const bool more = packed && !corrupt && end > len;
+            const unsigned sm = __ballot_sync(0xffffffffu, more && end + 2 * per16 > sw);
+            unsigned tm = __ballot_sync(0xffffffffu, more) & ~sm;
+            if (tm) {
+#pragma unroll 1
+                for (; tm; tm &= tm - 1) {
+                    const int q = __ffs(tm) - 1;
+                    const uintptr_t l = __shfl_sync(0xffffffffu, (unsigned long long)lo, q);
+                    const int64_t n = __shfl_sync(0xffffffffu, len, q);
+                    const int64_t e = __shfl_sync(0xffffffffu, end, q);
+                    copy_blocks(slots + q * sw, l, l + n * (int64_t)sizeof(U),
+                                l + e * (int64_t)sizeof(U));
+                }
+                cp_async_commit();
+                cp_async_wait_all();
+                __syncwarp();
+            }
+            if constexpr (!ONE) {
+                if (sm) {
+                    pm &= ~sm;
+                    decode_source_rows<U>(a.s.comp, (int64_t)(lo - comp) / (int64_t)sizeof(U), out,
+                                          sm, v, mw, a.s.t);
+                }
+            }
+        }
+#pragma unroll 1
+        for (unsigned m = rm; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            const U *src = slots + __shfl_sync(0xffffffffu, place, q);
+            U *o = reinterpret_cast<U *>(
+                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), q));
+            for (int j = lane; j < (int)v; j += 32) o[j] = src[j];
+        }
+        if (pm) {
+            if constexpr (ONE) {
+                int64_t base = 0;
+                decode_group<U, int>(gt, slots, place, out, pm, 0, mw, base);
+            } else {
+                decode_rows_long<U, int>(slots, place, out, pm, v, mw, a.s.t);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// A row starts at any word of its first 16-byte block.  Condensed rows are read whole; slots of
+// longer fixed-stride rows hold twice the first read (rows beyond that decode from their
+// source), so that more warps fit an SM.
+template <typename U>
+static int64_t device_slot_words(const RowSet<U> &s) {
+    constexpr int per16 = 16 / sizeof(U);
+    int64_t words = s.v;
+    if (!s.offsets && s.v > 256)
+        words = std::min<int64_t>(words, std::max<int64_t>(2 * s.first_words, 256));
+    return (int64_t)align_up((size_t)words + 2 * per16 + 2, per16);
+}
+
+// Every fetch of device rows but raw gathers and rows too long for one slot per block.
+template <typename U>
+static bool device_fetch_fit(const FetchArgs<U> &a) {
+    return a.device_rows && !a.raw_only &&
+           device_slot_words<U>(a.s) * (int64_t)sizeof(U) <= device_max_smem_optin();
+}
+
+template <typename U>
+static ibp_status launch_device_fetch(FetchArgs<U> a, cudaStream_t st) {
+    a.slot_words = device_slot_words<U>(a.s);
+    const size_t slot = (size_t)a.slot_words * sizeof(U);
+    // up to 16 rows share a load of the tables as long as two blocks of 8 warps fit an SM
+    a.slots = 16;
+    while (a.slots > 1 && 8 * a.slots * slot > 110 * 1024) a.slots /= 2;
+    const int warps = (int)std::min<size_t>(8, (size_t)device_max_smem_optin() / (a.slots * slot));
+    const bool one = a.s.v * (int64_t)sizeof(U) <= 512;
+    auto kern = a.s.offsets
+                    ? (one ? device_fetch_kernel<U, true, true> : device_fetch_kernel<U, false, true>)
+                    : (one ? device_fetch_kernel<U, true, false>
+                           : device_fetch_kernel<U, false, false>);
+    const size_t smem = slot * a.slots * warps;
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, warps * 32, smem, &per_sm));
+    const int64_t blocks = std::min<int64_t>((a.nrows + warps - 1) / warps,
+                                             (int64_t)device_sm_count() * per_sm);
+    const int pslot = profile_begin(st);
+    IBP_CUDA(launch_dependent(kern, (unsigned)blocks, warps * 32, smem, st, a));
+    IBP_LAUNCHED("device_fetch_kernel");
+    profile_end(pslot, st);
     return IBP_OK;
 }
 
@@ -625,16 +857,15 @@ size_t decompress_workspace(int64_t nidx, int64_t v, int wb, bool has_index) {
         Sizer hsh;
         hsh.take<int64_t>(hash_slots(nidx));
         hsh.take<int64_t>(hash_slots(nidx));
-        hsh.take<int64_t>(2 * nidx);  // claimed heads (records of two words)
+        hsh.take<longlong2>(nidx);  // claimed heads
         s.take<char>(std::max(srt.total(), hsh.total()));
     }
     return s.total();
 }
 
-template <typename U, int NC, bool EXACT, bool ASYNC>
+template <typename U, int NC, bool EXACT>
 static ibp_status launch_fetch_nc(FetchArgs<U> a, int nblks, int nthreads, cudaStream_t st) {
-    // a warp's slots: one set, or two for the double-buffered reads of device rows
-    const size_t slot_bytes = (size_t)a.slot_words * sizeof(U) * (ASYNC ? 2 : 1);
+    const size_t slot_bytes = (size_t)a.slot_words * sizeof(U);
     int threads = nthreads > 0 ? nthreads : kFetchThreads;
     threads = threads < 32 ? 32 : (threads > kFetchThreads ? kFetchThreads : threads / 32 * 32);
     const int maxs = device_max_smem_optin();
@@ -656,9 +887,9 @@ static ibp_status launch_fetch_nc(FetchArgs<U> a, int nblks, int nthreads, cudaS
     // raw rows of over 1 KiB are never staged with the first reads: their kernel goes without
     // that code and its registers (whole-set fetches of 16 KiB rows at 97% invariant bits:
     // 2.85 -> 2.36 ms); rows of up to 1 KiB keep it
-    auto kern = (EXACT || ASYNC || a.s.v * (int64_t)sizeof(U) <= 1024)
-                    ? fetch_rows_kernel<U, NC, EXACT, ASYNC, true>
-                    : fetch_rows_kernel<U, NC, EXACT, ASYNC, false>;
+    auto kern = (EXACT || a.s.v * (int64_t)sizeof(U) <= 1024)
+                    ? fetch_rows_kernel<U, NC, EXACT, true>
+                    : fetch_rows_kernel<U, NC, EXACT, false>;
     int per_sm = 0;
     IBP_RET(kernel_blocks_per_sm((const void *)kern, threads, smem, &per_sm));
     int64_t blocks = nblks > 0 ? nblks : (int64_t)device_sm_count() * per_sm;
@@ -676,22 +907,24 @@ static ibp_status launch_fetch_nc(FetchArgs<U> a, int nblks, int nthreads, cudaS
     return IBP_OK;
 }
 
-template <typename U, bool EXACT, bool ASYNC>
+template <typename U, bool EXACT>
 static ibp_status launch_fetch_x(FetchArgs<U> a, int nblks, int nthreads, cudaStream_t st) {
-    if (a.raw_only || a.s.v > 64)
-        return launch_fetch_nc<U, 0, EXACT, ASYNC>(a, nblks, nthreads, st);
-    if (a.s.v > 32) return launch_fetch_nc<U, 2, EXACT, ASYNC>(a, nblks, nthreads, st);
-    return launch_fetch_nc<U, 1, EXACT, ASYNC>(a, nblks, nthreads, st);
+    if (a.raw_only || a.s.v > 64) return launch_fetch_nc<U, 0, EXACT>(a, nblks, nthreads, st);
+    if (a.s.v > 32) return launch_fetch_nc<U, 2, EXACT>(a, nblks, nthreads, st);
+    return launch_fetch_nc<U, 1, EXACT>(a, nblks, nthreads, st);
 }
 
 template <typename U>
 static ibp_status launch_fetch(FetchArgs<U> a, int nblks, int nthreads, cudaStream_t st) {
     if (a.nrows <= 0) return IBP_OK;
     constexpr int per16 = 16 / sizeof(U);
+    if (hbm_rows_fit(a))
+        return a.s.v > 32 ? launch_hbm_nc<U, 2>(a, st) : launch_hbm_nc<U, 1>(a, st);
+    if (device_fetch_fit(a)) return launch_device_fetch<U>(a, st);
     if (a.s.offsets) {
         // a condensed row starts at any word: room for the blocks around it and the padding
         a.slot_words = (int64_t)align_up((size_t)a.s.v + 2 * per16 + 2, per16);
-        return launch_fetch_x<U, true, false>(a, nblks, nthreads, st);
+        return launch_fetch_x<U, true>(a, nblks, nthreads, st);
     }
     if (a.raw_only) {
         a.slot_words = per16;  // raw rows are copied straight to the output
@@ -704,10 +937,7 @@ static ibp_status launch_fetch(FetchArgs<U> a, int nblks, int nthreads, cudaStre
     } else {
         a.slot_words = (int64_t)align_up((size_t)a.s.v + 2, per16);
     }
-    if (hbm_rows_fit(a))
-        return a.s.v > 32 ? launch_hbm_nc<U, 2>(a, st) : launch_hbm_nc<U, 1>(a, st);
-    if (a.async_rows && !a.raw_only) return launch_fetch_x<U, false, true>(a, nblks, nthreads, st);
-    return launch_fetch_x<U, false, false>(a, nblks, nthreads, st);
+    return launch_fetch_x<U, false>(a, nblks, nthreads, st);
 }
 
 // The first kernel of a fetch call, in place of two memsets and the table build (a per-call
@@ -776,10 +1006,6 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
     }
     FetchArgs<U> a{};
     a.gmax = on_device ? 32 : 0;
-    // HBM rows of 256 bytes and up: first reads double-buffered, and rows of up to 64 words
-    // decoded a group at a time (256-byte rows: 75 -> 61 us for 100k rows; smaller rows
-    // decode too quickly for the extra bookkeeping to pay)
-    a.async_rows = on_device && v * (int64_t)sizeof(U) >= 256;
     a.device_rows = on_device;
     a.s.comp = comp;
     a.s.n = n;
@@ -816,14 +1042,17 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
         const int64_t slots = hash_slots(nidx);
         int64_t *hkeys = c.take<int64_t>(slots);
         int64_t *hpos = c.take<int64_t>(slots);
-        int64_t *heads = c.take<int64_t>(2 * nidx);
+        longlong2 *heads = c.take<longlong2>(nidx);
         // keys -1 (empty); positions -1 (unpublished) for the in-fetch claims (a claim pass
         // writes the position of each slot it claims); hpos follows hkeys directly (slots is
         // a multiple of 64 words)
+        // a fetch of host rows, and the few of device rows that no device kernel takes (raw
+        // gathers, rows longer than shared memory), claim inside the fetch
+        const bool pass = hbm_rows_fit(a) || device_fetch_fit(a);
         IBP_RET(launch_prep<U>(status, mask, bitval, v, t, tables, hkeys,
-                               on_device ? slots : (int64_t)(hpos + slots - hkeys), st));
+                               pass ? slots : (int64_t)(hpos + slots - hkeys), st));
         a.keys = idx;
-        if (on_device) {
+        if (pass) {
             // HBM rows: claim in a pass of its own, so the fetch walks distinct rows only, 32
             // to a chunk (the fetch is latency-bound here and chunks of repeats cost it)
             auto *nheads =
@@ -834,15 +1063,12 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
                                                  wave);
             a.list = heads;
             a.list_len = nheads;
-            // the HBM-row kernel reads head records (position and stored-compressed flag, row)
-            const int32_t *records = hbm_rows_fit(a) ? bitmask : nullptr;
             IBP_CUDA(launch_dependent(two ? claim_heads_kernel<2> : claim_heads_kernel<1>,
                                       (unsigned)cb, 256, 0, st, idx, nidx, n, hkeys, hpos, slots,
-                                      heads, nheads, status, records));
+                                      heads, nheads, status, bitmask));
             IBP_LAUNCHED("claim_heads_kernel");
         } else {
-            // host rows: claims and repeat copies happen inside the fetch, hidden behind its
-            // PCIe reads
+            // claims and repeat copies happen inside the fetch, hidden behind its PCIe reads
             a.claims = ClaimTable{hkeys, hpos, slots, repeat_wait_polls()};
             return launch_fetch<U>(a, nblks, nthreads, st);
         }

@@ -198,65 +198,6 @@ __device__ __forceinline__ void decode_row(const U *__restrict__ buf, int64_t v,
     }
 }
 
-// decode_row for up to kRowsInFlight rows of at most 64 words at once (rows in slots
-// `slots + q * slot_words` for the q set in `qm`, outputs `o[q]`): the prefix sums of every
-// row's chunks are issued together, so their shuffle chains overlap instead of following
-// one another, then each row's bits are placed as in decode_row.
-template <typename U, int NC>
-__device__ __forceinline__ void decode_rows_multi(const U *__restrict__ slots,
-                                                  int64_t slot_words, unsigned qm, int64_t v,
-                                                  int64_t mw, const LaneTables<U, NC> &lt,
-                                                  U *const *o) {
-    static_assert(NC > 0, "register tables only");
-    constexpr int W = 8 * sizeof(U);
-    constexpr int Q = kRowsInFlight;
-    const int lane = threadIdx.x & 31;
-    int incl[Q][NC];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const uint32_t *units = reinterpret_cast<const uint32_t *>(slots + q * slot_words);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const int64_t j = 32 * c + lane;
-            const bool in = ((qm >> q) & 1) && j < v;
-            const bool cj = in && ((units[j >> 5] >> (j & 31)) & 1u);
-            incl[q][c] = in ? (cj ? lt.nb[c] : W) : 0;
-        }
-    }
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const int y = __shfl_up_sync(0xffffffffu, incl[q][c], off);
-                if (lane >= off) incl[q][c] += y;
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        if (!((qm >> q) & 1)) continue;
-        const U *buf = slots + q * slot_words;
-        const uint32_t *units = reinterpret_cast<const uint32_t *>(buf);
-        const U *stream = buf + mw;
-        int64_t base = 0;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            if (32 * c >= v) break;
-            const int64_t j = 32 * c + lane;
-            const bool in = j < v;
-            const bool cj = in && ((units[j >> 5] >> (j & 31)) & 1u);
-            const int L = in ? (cj ? lt.nb[c] : W) : 0;
-            if (in) {
-                const U y = get_bits<U>(stream, base + incl[q][c] - L, L);
-                o[q][j] = cj ? lt.word(y, c) : y;
-            }
-            base += __shfl_sync(0xffffffffu, incl[q][c], 31);
-        }
-    }
-}
-
 // Exact compressed words of the row whose bitmap is in the slot (bitmap + stream).
 template <typename U, int NC>
 __device__ __forceinline__ int64_t row_words(const U *__restrict__ buf, int64_t v, int64_t mw,
@@ -282,6 +223,168 @@ __device__ __forceinline__ int64_t row_words(const U *__restrict__ buf, int64_t 
 }
 
 
+// ------------------------------------------------------------------ rows decoded together
+// The tables of a group of 512 bytes of columns (64 64-bit or 128 32-bit words; column
+// g0 + 32 * c + lane) and the bits its rows hold up to each column's end when every word of
+// the group is compressible.
+template <typename U>
+struct GroupTables {
+    static constexpr int GC = 16 / sizeof(U);
+    U m[GC], bv[GC], mv[GC][kMoves];
+    int kept[GC];
+    uint32_t incl[GC], total;
+    unsigned absent[GC];  // columns past the row's end
+    int left;             // columns from this lane's first to the row's end
+
+    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t g0) {
+        const int lane = threadIdx.x & 31;
+        left = (int)min(v - g0, (int64_t)(32 * GC)) - lane;
+#pragma unroll
+        for (int c = 0; c < GC; ++c) {
+            const bool in = 32 * c < left;
+            const int64_t j = g0 + 32 * c + lane;
+            m[c] = in ? __ldg(t.mask + j) : (U)0;
+            bv[c] = in ? __ldg(t.bitval + j) : (U)0;
+            kept[c] = in ? (int)__ldg(t.nb + j) : 0;
+            const U *mvp = t.mv + j;
+#pragma unroll
+            for (int i = 0; i < kMoves; ++i, mvp += v) mv[c][i] = in ? __ldg(mvp) : (U)0;
+            absent[c] = ~__ballot_sync(0xffffffffu, in);
+            incl[c] = (uint32_t)kept[c] & 0xffu;
+        }
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl[c], off);
+                if (lane >= off) incl[c] += y;
+            }
+        }
+        total = 0;
+#pragma unroll
+        for (int c = 0; c < GC; ++c) {
+            incl[c] += total;
+            total = __shfl_sync(0xffffffffu, incl[c], 31);
+        }
+    }
+};
+
+// Decode the group's words of the rows of the lanes in `lanes`: each such lane holds its row's
+// place (words from `rows`, all in shared or all in global memory: bitmap, then the stream mw
+// words on), its output row and the bits of the stream in earlier groups (base, advanced).  A
+// word's bits are read as the stream bits that end at its end, which a group whose words are
+// all compressible takes from the tables and any other from a prefix sum; the words of a
+// group are then read, scattered and written without a branch between them.  (Columns past the
+// end read where the row's last word ends, and what they read is not written.)  One row at a
+// time in a loop that is not unrolled: four rows' code side by side missed the instruction
+// cache (device_fetch_kernel, 100k rows of 256 32-bit words: 139 us, with the loop 83).
+template <typename U, typename Place>
+__device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *rows, Place place,
+                                             U *out, unsigned lanes, int64_t g0, int64_t mw,
+                                             int64_t &base) {
+    constexpr int W = 8 * sizeof(U), GC = GroupTables<U>::GC;
+    constexpr int LW = LogW<U>::value;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    while (lanes) {
+        const int q = __ffs(lanes) - 1;
+        lanes &= lanes - 1;
+        const U *row = rows + __shfl_sync(0xffffffffu, place, q);
+        const int64_t at = __shfl_sync(0xffffffffu, base, q);
+        U *o = reinterpret_cast<U *>(
+                   __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), q)) +
+               g0 + lane;
+        const uint32_t *units = reinterpret_cast<const uint32_t *>(row) + (g0 >> 5);
+        const U *gs = row + mw + (at >> LW);
+        const int32_t off = (int32_t)(at & (W - 1));
+        uint32_t bits[GC], end[GC], every = 0xffffffffu;
+#pragma unroll
+        for (int c = 0; c < GC; ++c) {
+            bits[c] = units[c];
+            every &= bits[c] | t.absent[c];
+            end[c] = t.incl[c];
+        }
+        uint32_t all = t.total;
+        if (every != 0xffffffffu) {
+            all = 0;
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+                const bool cj = (bits[c] >> lane) & 1u;
+                end[c] = 32 * c < t.left ? (cj ? (uint32_t)t.kept[c] & 0xffu : (uint32_t)W) : 0u;
+            }
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+                for (int c = 0; c < GC; ++c) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, end[c], d);
+                    if (lane >= d) end[c] += y;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+                end[c] += all;
+                all = __shfl_sync(0xffffffffu, end[c], 31);
+            }
+        }
+        U x[GC];
+#pragma unroll
+        for (int c = 0; c < GC; ++c) {
+            const U y = stream_bits_ending<U>(gs, off + (int32_t)end[c]);
+            x[c] = scatter_word<U>(y, t.m[c], t.bv[c], t.kept[c] >> 8, t.mv[c]);
+            x[c] = (bits[c] >> lane) & 1u ? x[c] : y;
+        }
+#pragma unroll
+        for (int c = 0; c < GC; ++c)
+            if (32 * c < t.left) o[32 * c] = x[c];
+        if (lane == q) base += all;
+    }
+}
+
+// Decode the rows of the lanes in `lanes`, of any length, at once (each lane's place and output
+// row as above): the tables of a group of columns are loaded once and serve every row.  Device
+// rows only: in the host-row kernels, whose small fetches wait for one row's decode after its
+// link round trip, decode_row is shorter (2048 rows of 128 64-bit words: 48.2 against 51 us).
+template <typename U, typename Place>
+__device__ __forceinline__ void decode_rows_long(const U *rows, Place place, U *out,
+                                                 unsigned lanes, int64_t v, int64_t mw,
+                                                 const ColTables<U> &t) {
+    int64_t base = 0;
+    for (int64_t g0 = 0; g0 < v; g0 += 32 * GroupTables<U>::GC) {
+        GroupTables<U> gt;
+        gt.load(t, v, g0);
+        decode_group<U, Place>(gt, rows, place, out, lanes, g0, mw, base);
+    }
+}
+
+// The same from the rows' sources, for the few rows longer than their slots: a called function,
+// so that its registers do not add to the caller's.
+template <typename U>
+__device__ __noinline__ void decode_source_rows(const U *rows, int64_t place, U *out,
+                                                unsigned lanes, int64_t v, int64_t mw,
+                                                const ColTables<U> &t) {
+    decode_rows_long<U, int64_t>(rows, place, out, lanes, v, mw, t);
+}
+
+// Stream bits of the row whose bitmap is at `row`: `packed` when every word is compressible (the
+// usual row, seen from the bitmap alone), else the sum over the columns.
+template <typename U>
+__device__ __forceinline__ uint32_t row_stream_bits(const U *row, int64_t v, const ColTables<U> &t,
+                                                    uint32_t packed) {
+    constexpr int W = 8 * sizeof(U);
+    const int lane = threadIdx.x & 31;
+    const uint32_t *bitmap = reinterpret_cast<const uint32_t *>(row);
+    const int64_t units = (v + 31) / 32;
+    const uint32_t absent = v & 31 ? ~0u << (v & 31) : 0u;  // of the last unit
+    bool full = true;
+    for (int64_t i = lane; i < units; i += 32)
+        full = full && (bitmap[i] | (i == units - 1 ? absent : 0u)) == ~0u;
+    if (__all_sync(0xffffffffu, full)) return packed;
+    uint32_t bits = 0;
+    for (int64_t j = lane; j < v; j += 32)
+        bits += (bitmap[j >> 5] >> lane) & 1u ? (uint32_t)__ldg(t.nb + j) & 0xffu : (uint32_t)W;
+    return __reduce_add_sync(0xffffffffu, bits);
+}
+
 // Second half of a group of rows whose first reads are in their slots (slot q at
 // slots + q * slot_words for the rows of lanes lid[0..cnt)): exact lengths from the
 // bitmaps, the rest of every row that needs more than its first read (all issued before any
@@ -306,7 +409,7 @@ __device__ __forceinline__ void copy_raw_row(U *o, const U *slot, const U *src, 
     }
 }
 
-template <typename U, int NC, bool MULTI = false>
+template <typename U, int NC>
 __device__ __forceinline__ void finish_rows(const RowSet<U> &s, const LaneTables<U, NC> &lt,
                                             U *__restrict__ slots, int64_t slot_words,
                                             const int *lid, int cnt, int64_t key, U *orow,
@@ -349,67 +452,37 @@ __device__ __forceinline__ void finish_rows(const RowSet<U> &s, const LaneTables
                 reinterpret_cast<uint4 *>(slots + q * slot_words)[tb0[q] + lane] = tail[q];
     }
     __syncwarp();
-    if constexpr (MULTI && NC > 0) {
-        // rows of at most 64 words: copies and corrupt rows first, then every row of the
-        // group that decodes from its slot, all at once
-        U *o[kRowsInFlight];
-        unsigned qm = 0;
 #pragma unroll
-        for (int q = 0; q < kRowsInFlight; ++q) {
-            o[q] = nullptr;
-            if (q < cnt) {
-                const int64_t r = __shfl_sync(0xffffffffu, key, lid[q]);
-                o[q] = reinterpret_cast<U *>(
-                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(orow), lid[q]));
-                if (end[q] < 0) {
-                    copy_raw_row<U>(o[q], slots + q * slot_words, s.comp + r * v, v, raw_staged);
-                } else if (end[q] >= v) {
-                    if (lane == 0) atomicOr(status, kStatusCorruptRow);
-                } else if (end[q] + 2 > slot_words) {  // not with slots of v + 2 words
-                    decode_row<U, NC>(s.comp + r * v, v, s.mw, s.t, lt, o[q]);
-                    __syncwarp();
-                } else {
-                    if (lane < 2) slots[q * slot_words + end[q] + lane] = 0;
-                    qm |= 1u << q;
-                }
+    for (int q = 0; q < kRowsInFlight; ++q) {
+        if (q < cnt) {
+            const int64_t r = __shfl_sync(0xffffffffu, key, lid[q]);
+            U *o = reinterpret_cast<U *>(
+                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(orow), lid[q]));
+            if (end[q] < 0) {
+                copy_raw_row<U>(o, slots + q * slot_words, s.comp + r * v, v, raw_staged);
+                continue;
             }
-        }
-        __syncwarp();
-        if (qm) decode_rows_multi<U, NC>(slots, slot_words, qm, v, s.mw, lt, o);
-        __syncwarp();
-    } else {
-#pragma unroll
-        for (int q = 0; q < kRowsInFlight; ++q) {
-            if (q < cnt) {
-                const int64_t r = __shfl_sync(0xffffffffu, key, lid[q]);
-                U *o = reinterpret_cast<U *>(
-                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(orow), lid[q]));
-                if (end[q] < 0) {
-                    copy_raw_row<U>(o, slots + q * slot_words, s.comp + r * v, v, raw_staged);
-                    continue;
-                }
-                if (end[q] >= v) {
-                    // a bitmap claiming a stream as long as the raw row cannot come from this
-                    // mask: report it and leave the output row alone
-                    if (lane == 0) atomicOr(status, kStatusCorruptRow);
-                    continue;
-                }
-                if (end[q] + 2 > slot_words) {
-                    // longer than the slot (slots are sized for rows near the average length
-                    // when rows are long): decode from the source row, whose words after the
-                    // stream are its zero padding
-                    decode_row<U, NC>(s.comp + r * v, v, s.mw, s.t, lt, o);
-                    __syncwarp();
-                    continue;
-                }
-                U *buf = slots + q * slot_words;
-                // words past the stream read as zero (get_bits looks one word ahead; the
-                // value there never reaches an output bit)
-                if (lane < 2) buf[end[q] + lane] = 0;
-                __syncwarp();
-                decode_row<U, NC>(buf, v, s.mw, s.t, lt, o);
-                __syncwarp();
+            if (end[q] >= v) {
+                // a bitmap claiming a stream as long as the raw row cannot come from this
+                // mask: report it and leave the output row alone
+                if (lane == 0) atomicOr(status, kStatusCorruptRow);
+                continue;
             }
+            if (end[q] + 2 > slot_words) {
+                // longer than the slot (slots are sized for rows near the average length
+                // when rows are long): decode from the source row, whose words after the
+                // stream are its zero padding
+                decode_row<U, NC>(s.comp + r * v, v, s.mw, s.t, lt, o);
+                __syncwarp();
+                continue;
+            }
+            U *buf = slots + q * slot_words;
+            // words past the stream read as zero (get_bits looks one word ahead; the
+            // value there never reaches an output bit)
+            if (lane < 2) buf[end[q] + lane] = 0;
+            __syncwarp();
+            decode_row<U, NC>(buf, v, s.mw, s.t, lt, o);
+            __syncwarp();
         }
     }
 }
@@ -489,21 +562,6 @@ __device__ __forceinline__ void fetch_heads(const RowSet<U> &s, const LaneTables
     }
 }
 
-// The next up-to-`nslots` head lanes of `hm` (removed from it), in lane order.
-__device__ __forceinline__ int pick_rows(unsigned &hm, int nslots, int *lid) {
-    int cnt = 0;
-#pragma unroll
-    for (int q = 0; q < kRowsInFlight; ++q) {
-        lid[q] = 0;
-        if (q < nslots && hm) {
-            lid[q] = __ffs(hm) - 1;
-            hm &= hm - 1;
-            ++cnt;
-        }
-    }
-    return cnt;
-}
-
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(smem)),
@@ -513,62 +571,6 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// fetch_heads for rows in device memory: the first reads of the next group of rows are
-// issued as asynchronous copies into a second set of slots while the current group is
-// decoded, so a warp's HBM round trips overlap its decode instead of following it (the
-// warp owns 2 x nslots slots).  Not used for host rows: asynchronous copies from host
-// memory are slow on this part.
-template <typename U, int NC>
-__device__ __forceinline__ void fetch_heads_async(const RowSet<U> &s, const LaneTables<U, NC> &lt,
-                                                  U *__restrict__ slots, int nslots,
-                                                  int64_t slot_words, int64_t key, U *orow,
-                                                  bool head, bool packed, int32_t *status) {
-    constexpr int per16 = 16 / sizeof(U);
-    const int lane = threadIdx.x & 31;
-    const int64_t v = s.v;
-    const int64_t nq = (s.first_words + per16 - 1) / per16;
-    auto issue = [&](const int *lid, int cnt, U *base) {
-        for (int q = 0; q < cnt; ++q) {
-            const int64_t r = __shfl_sync(0xffffffffu, key, lid[q]);
-            const bool pk = __shfl_sync(0xffffffffu, (int)packed, lid[q]);
-            if (!pk) continue;
-            const U *row = s.comp + r * v;
-            U *buf = base + q * slot_words;
-            if ((((uintptr_t)row) & 15) == 0) {
-                for (int64_t b = lane; b < nq; b += 32)
-                    cp_async16(reinterpret_cast<uint4 *>(buf) + b,
-                               reinterpret_cast<const uint4 *>(row) + b);
-            } else {
-                issue_words<U>(buf, row, 0, s.first_words);
-            }
-        }
-        cp_async_commit();
-    };
-    unsigned hm = __ballot_sync(0xffffffffu, head);
-    int lid[kRowsInFlight], nlid[kRowsInFlight];
-    int cnt = pick_rows(hm, nslots, lid);
-    int cur = 0;
-    if (cnt) issue(lid, cnt, slots);
-    while (cnt) {
-        const int ncnt = pick_rows(hm, nslots, nlid);
-        U *nbase = slots + (int64_t)(cur ^ 1) * nslots * slot_words;
-        if (ncnt) {
-            issue(nlid, ncnt, nbase);
-            cp_async_wait_one();  // the current group's copies are done
-        } else {
-            cp_async_wait_all();
-        }
-        __syncwarp();
-        finish_rows<U, NC, true>(s, lt, slots + (int64_t)cur * nslots * slot_words, slot_words,
-                                 lid, cnt, key, orow, packed, status);
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kRowsInFlight; ++q) lid[q] = nlid[q];
-        cnt = ncnt;
-        cur ^= 1;
-    }
-}
 
 // Condensed rows (byte ranges known from the offsets): each head lane's row is read exactly,
 // its 16-byte blocks (at most 64 per row staged in registers, longer rows by a plain loop)
