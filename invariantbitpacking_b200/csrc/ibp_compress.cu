@@ -193,7 +193,8 @@ struct PackTables {
         }
     }
 
-    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t j0) {
+    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t j0,
+                                         bool count_levels = false) {
         const int lane = threadIdx.x & 31;
         uint32_t moves[kMoves] = {};
         all = 0;
@@ -226,10 +227,13 @@ struct PackTables {
             before[c] = all + incl - nb[c];
             all += __shfl_sync(0xffffffffu, incl, 31);
         }
-        levels = 0;
+        levels = kMoves;
+        if (count_levels) {
+            levels = 0;
 #pragma unroll
-        for (int i = 0; i < kMoves; ++i)
-            if (__any_sync(0xffffffffu, moves[i] != 0)) levels = i + 1;
+            for (int i = 0; i < kMoves; ++i)
+                if (__any_sync(0xffffffffu, moves[i] != 0)) levels = i + 1;
+        }
     }
 };
 
@@ -334,6 +338,11 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                 uint32_t every = 0xffffffffu;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
+                    if (!ONE && t.valid[c] == 0) {  // a chunk past the row's end
+                        cj[c] = true;
+                        hi[c] = lo[c] = off[c] = bal[c] = 0;
+                        continue;
+                    }
                     uint32_t h[H];
                     PackTables<U, NC>::split(x[q][c], h);
                     uint32_t e = (h[0] & t.m[c][0]) ^ t.bv[c][0];
@@ -380,7 +389,8 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                 const uint32_t image = images_at + q * image_units * 4;
                 or_shared(image + (uint32_t)((g * NC + (lane & (NC - 1))) ^ (H - 1)) * 4, mine);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) put_bits<U>(image, off[c], hi[c], lo[c]);
+                for (int c = 0; c < NC; ++c)
+                    if (ONE || t.valid[c]) put_bits<U>(image, off[c], hi[c], lo[c]);
             }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
@@ -445,7 +455,7 @@ template <typename U, int NC, int Q, bool ONE, bool INDEX>
 __global__ void __launch_bounds__(256, 2) pack_rows_kernel(PackArgs<U> a) {
     PackTables<U, NC> t;
     if (ONE) {
-        t.load(a.t, a.v, 0);
+        t.load(a.t, a.v, 0, true);
         if (t.levels <= 2) {
             pack_rows<U, NC, Q, ONE, INDEX, 2>(a, t);
             return;
