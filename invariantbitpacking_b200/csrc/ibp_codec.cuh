@@ -140,6 +140,22 @@ __device__ __forceinline__ U scatter_word(U y, U mask, U bv, int nbl, const U (&
     }
 }
 
+// The top bits of y placed at the set positions of sel, for the first LEVELS masks of
+// move_masks<false> (all of them, or the only ones that are not zero: see moves_left).
+template <int LEVELS>
+__device__ __forceinline__ uint32_t scatter_top(uint32_t y, uint32_t sel, uint32_t keep,
+                                                const uint32_t *mv) {
+#pragma unroll
+    for (int i = LEVELS - 1; i >= 0; --i) y = (y & ~mv[i]) | ((y >> (1 << i)) & mv[i]);
+    return (y & sel) | keep;
+}
+
+// Dropped bits above the lowest kept bit of sel: how far the farthest kept bit is from its place
+// when they are packed left, so that moves of 1, 2, ... up to this many places suffice.
+__device__ __forceinline__ int moves_left(uint32_t sel) {
+    return sel ? 33 - __ffs((int)sel) - __popc(sel) : 0;
+}
+
 // Column j of the tables (RIGHT: for decoding; else for packing).
 template <typename U, bool RIGHT = true>
 __device__ __forceinline__ void build_table_column(const U *__restrict__ mask,

@@ -318,140 +318,169 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
 // so this kernel keeps per-row bookkeeping to a minimum: a warp takes a chunk of listed rows
 // from a work counter (the claim pass's head records -- position with the row's
 // stored-compressed flag, and row -- or rows p, p+1, ... of an unindexed fetch; 4 to 32 rows
-// at a time by the batch's size), parks their keys and output rows in shared memory, and
+// at a time by the batch's size), parks their sources and output rows in shared memory, and
 // copies groups of G whole rows (one 16-byte cp.async per lane and row; rows must be 16-byte
 // aligned) into one of two shared buffers while it decodes the previous group from the
-// other.  A group whose words are all compressible (the usual case: a good mask leaves few
-// words whole) takes its stream offsets from a table made once per warp; otherwise its prefix
-// sums are issued together.  The row's stream length falls out of the offsets (no separate
-// length pass, no tail reads), and stream offsets are 32-bit.
+// other.
 //
-// Stream reads: stream_bits_ending (ibp_codec.cuh), a word read as the W stream bits that end
-// where its bits end.
-// `full[32 * c + lane]`: the inclusive prefix over the lanes of chunk c of the kept bits of
-// every column (the stream offsets of a row whose words are all compressible).
-template <typename U, int NC, int G>
-__device__ __forceinline__ void hbm_decode_group(const U *__restrict__ buf, int sw, int r0,
-                                                 int rows, unsigned okm, unsigned pm, int v,
-                                                 int mw, const LaneTables<U, NC> &lt,
-                                                 const uint32_t *full, U *const *mout,
-                                                 int32_t *status) {
-    constexpr int W = 8 * sizeof(U);
-    const int lane = threadIdx.x & 31;
-    uint32_t incl[G][NC];
-    unsigned cjm = 0;  // bit q * NC + c: this lane's column of chunk c in row q is compressible
-    bool mixed = false;  // a packed row of the group has a word stored whole
-#pragma unroll
-    for (int q = 0; q < G; ++q) {
-        const int r = r0 + q;
-        const bool pk = r < rows && ((pm >> r) & 1);
-        const uint32_t *units = reinterpret_cast<const uint32_t *>(buf + q * sw);
+// A row whose words are all compressible (the usual case: a good mask leaves few words whole)
+// has every word at the same place, so a lane's word is three reads at offsets fixed for the
+// whole kernel, funnel shifts by fixed amounts, the moves and a store (ShortTables::word);
+// any other row takes a prefix sum.  Moves: a word's halves are read either as the bits that
+// start where it starts and moved right into place (LEFT), or as the bits that end where it ends
+// and moved left; LEFT when two moves (three places) suffice for every column, as for masks
+// that drop little above what they keep, else five moves the other way.  The row's stream
+// length falls out of the offsets (no separate length pass, no tail reads), and stream offsets
+// are 32-bit.
+// Bound: issue, then HBM (whole rows are read: 512 + 512 bytes for a 64-word row).  200k rows of
+// 64 64-bit words at 264 stored bytes: 57 us with offsets and reads worked out per row, 53 with
+// 32-bit halves, 39.6 now (5.2 TB/s of the bytes it moves); the 79k distinct rows of a 400k-row
+// batch 34.1 -> 28.4 us.
+template <typename U, int NC>
+struct ShortColumns {
+    U mask[NC], val[NC];
+    int kept[NC];
+
+    __device__ __forceinline__ void load(const ColTables<U> &t, int v) {
+        const int lane = threadIdx.x & 31;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const bool in = 32 * c + lane < v;
-            const bool cj = pk && in && ((units[c] >> lane) & 1u);
-            cjm |= (unsigned)cj << (q * NC + c);
-            mixed |= pk && in && !cj;
-            incl[q][c] = pk ? full[c * 32 + lane] : 0u;
+            const int j = lane + 32 * c;
+            const bool in = j < v;
+            mask[c] = in ? t.mask[j] : (U)~(U)0;
+            val[c] = in ? t.bitval[j] : (U)0;
+            kept[c] = in ? (int)t.nb[j] : 0;
         }
     }
-    if (__any_sync(0xffffffffu, mixed)) {
-        // some word of the group is stored whole: offsets from a prefix sum per row and chunk
+
+    // two moves suffice for every column of the row
+    __device__ __forceinline__ bool left_fits() const {
+        bool fits = true;
 #pragma unroll
-        for (int q = 0; q < G; ++q) {
-            const bool pk = r0 + q < rows && ((pm >> (r0 + q)) & 1);
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const bool in = 32 * c + lane < v;
-                const bool cj = (cjm >> (q * NC + c)) & 1u;
-                incl[q][c] = (pk && in) ? (cj ? (uint32_t)lt.nb[c] : (uint32_t)W) : 0u;
-            }
+        for (int c = 0; c < NC; ++c) {
+            const U sel = (U)~mask[c];
+            fits = fits && moves_left((uint32_t)sel) < 4;
+            if (sizeof(U) == 8) fits = fits && moves_left((uint32_t)((uint64_t)sel >> 32)) < 4;
         }
+        return __all_sync(0xffffffffu, fits);
+    }
+};
+
+template <typename U, int NC, bool LEFT>
+struct ShortTables {
+    static constexpr int W = 8 * sizeof(U), H = sizeof(U) / 4;  // halves, high first
+    static constexpr int MV = LEFT ? 2 : kMoves;
+    uint32_t m[NC][H], bv[NC][H], mv[NC][H][MV];
+    int nb[NC], split[NC];  // kept bits; of the high half (LEFT) or the low half
+    uint32_t total;         // stream bits of a row whose words are all compressible
+    int at[NC][H + 1];      // byte offsets from the row of the units that row's word lies in
+    uint32_t shift[NC];
+
+    // unit `q` of the stream in bytes from the row's start (mw words of bitmap before it)
+    static __device__ __forceinline__ int unit_byte(int q, int mw) {
+        return mw * (int)sizeof(U) + 4 * (H == 2 ? q ^ 1 : q);
+    }
+
+    __device__ __forceinline__ void load(const ColTables<U> &t, const ShortColumns<U, NC> &cols,
+                                         int v, int mw) {
+        const int lane = threadIdx.x & 31;
+        total = 0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
+        for (int c = 0; c < NC; ++c) {
+            const int j = lane + 32 * c;
+            const bool in = j < v;
+            const U mask = cols.mask[c], val = cols.val[c];
+            nb[c] = cols.kept[c] & 0xff;
+            const int nbl = H == 2 ? cols.kept[c] >> 8 : 0;
+            split[c] = LEFT ? nb[c] - nbl : nbl;
 #pragma unroll
-            for (int q = 0; q < G; ++q) {
+            for (int h = 0; h < H; ++h) {
+                m[c][h] = (uint32_t)(H == 2 && h == 0 ? (uint64_t)mask >> 32 : mask);
+                bv[c][h] = (uint32_t)(H == 2 && h == 0 ? (uint64_t)val >> 32 : val);
+                if constexpr (LEFT) {
+                    uint32_t all[kMoves];
+                    move_masks<false>(~m[c][h], all);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl[q][c], off);
-                    if (lane >= off) incl[q][c] += y;
+                    for (int i = 0; i < MV; ++i) mv[c][h][i] = all[i];
                 }
             }
-        }
-    }
+            if constexpr (!LEFT) {
 #pragma unroll
-    for (int q = 0; q < G; ++q) {
-        const int r = r0 + q;
-        if (r >= rows || !((okm >> r) & 1)) continue;
-        U *o = mout[r];
-        const U *row = buf + q * sw;
-        if (!((pm >> r) & 1)) {  // stored raw
+                for (int i = 0; i < kMoves; ++i) {
+                    const U x = in ? t.mv[i * (int64_t)v + j] : (U)0;
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if (32 * c + lane < v) o[32 * c + lane] = row[32 * c + lane];
-            continue;
-        }
-        const uint32_t t0 = __shfl_sync(0xffffffffu, incl[q][0], 31);
-        uint32_t tot = t0;
-        if (NC > 1) tot += __shfl_sync(0xffffffffu, incl[q][NC - 1], 31);
-        if (mw + (int)((tot + W - 1) / W) >= v) {
-            // a bitmap claiming a stream as long as the raw row cannot come from this mask:
-            // report it and leave the output row alone
-            if (lane == 0) atomicOr(status, kStatusCorruptRow);
-            continue;
-        }
-        const U *stream = row + mw;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const int j = 32 * c + lane;
-            if (j < v) {
-                const bool cj = (cjm >> (q * NC + c)) & 1u;
-                const U y = stream_bits_ending<U>(stream, (int32_t)((c ? t0 : 0u) + incl[q][c]));
-                o[j] = cj ? lt.word(y, c) : y;
+                    for (int h = 0; h < H; ++h)
+                        mv[c][h][i] = (uint32_t)(H == 2 && h == 0 ? (uint64_t)x >> 32 : x);
+                }
             }
+            uint32_t incl = (uint32_t)nb[c];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const int32_t s = (int32_t)(total + incl) - (LEFT ? nb[c] : W);
+#pragma unroll
+            for (int i = 0; i <= H; ++i) at[c][i] = unit_byte((s >> 5) + i, mw);
+            shift[c] = (uint32_t)s & 31u;
+            total += __shfl_sync(0xffffffffu, incl, 31);
         }
     }
-}
 
-// Shared memory of hbm_rows_kernel per warp: keys, output rows and stored-compressed flags
-// of its (up to) 32 rows, the stream offsets of an all-compressible row (up to 64 words),
-// then two buffers of G row slots.
-constexpr size_t kHbmWarpMetaBytes = 512 + 128 + 256;
+    // The word of column 32 * c + lane from the H + 1 stream units u around it (the bits start,
+    // or the last unit's first 32 - r are those that follow, by r); raw: stored whole.
+    __device__ __forceinline__ U word(const uint32_t (&u)[H + 1], uint32_t r, int c, bool raw) const {
+        uint32_t w[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) w[h] = __funnelshift_l(u[h + 1], u[h], r);
+        uint32_t x[H];
+        if constexpr (H == 2) {
+            x[0] = LEFT ? w[0] : __funnelshift_rc(w[1], w[0], split[c]);
+            x[1] = LEFT ? __funnelshift_lc(w[1], w[0], split[c]) : w[1];
+        } else {
+            x[0] = w[0];
+        }
+        U y = 0;
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            if constexpr (LEFT)
+                x[h] = scatter_top<MV>(x[h], ~m[c][h], bv[c][h], mv[c][h]);
+            else
+                x[h] = scatter_half(x[h], ~m[c][h], bv[c][h], mv[c][h]);
+            x[h] = raw ? w[h] : x[h];
+            y = (U)(((uint64_t)y << 32) | x[h]);
+        }
+        return y;
+    }
+};
 
-template <typename U, int NC, int G>
-__global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int per16 = 16 / sizeof(U);
+// Shared memory of hbm_rows_kernel per warp: sources, output rows and stored-compressed flags
+// of its (up to) 32 rows, then two buffers of G row slots.
+constexpr size_t kHbmWarpMetaBytes = 512 + 128;
+
+template <typename U, int NC, int G, bool LEFT>
+__device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *smem,
+                                         const ShortColumns<U, NC> &cols, int64_t nrows,
+                                         longlong2 record0) {
+    using T = ShortTables<U, NC, LEFT>;
+    constexpr int per16 = 16 / sizeof(U), W = T::W, H = T::H;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char *meta = smem + warp * kHbmWarpMetaBytes;
-    int64_t *mkey = reinterpret_cast<int64_t *>(meta);
-    U **mout = reinterpret_cast<U **>(mkey + 32);
+    const U **msrc = reinterpret_cast<const U **>(meta);
+    U **mout = reinterpret_cast<U **>(meta + 256);
     int32_t *mpk = reinterpret_cast<int32_t *>(meta + 512);
     const int sw = (int)a.slot_words;
     U *bufs = reinterpret_cast<U *>(smem + (blockDim.x >> 5) * kHbmWarpMetaBytes) +
               (int64_t)warp * 2 * G * sw;
-    // the column tables, the claim pass's list, the work counter and the status words come
-    // from the kernels before this one
-    grid_dep_wait();
-    grid_dep_release();
-    LaneTables<U, NC> lt;
-    lt.load(a.s.t, a.s.v);
     const int v = (int)a.s.v, mw = (int)a.s.mw;
-    // stream offsets (inclusive) of a row whose words are all compressible, lane-major
-    uint32_t *full = reinterpret_cast<uint32_t *>(meta + 640);
+    T t;
+    t.load(a.s.t, cols, v, mw);
+    // no row of this mask is all compressible and yet not shorter than raw
+    const bool full_fits = mw + (int)((t.total + W - 1) / W) < v;
+    uint32_t absent[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        uint32_t f = 32 * c + lane < v ? (uint32_t)lt.nb[c] : 0u;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, f, off);
-            if (lane >= off) f += y;
-        }
-        full[c * 32 + lane] = f;
-    }
-    __syncwarp();
+    for (int c = 0; c < NC; ++c) absent[c] = ~__ballot_sync(0xffffffffu, 32 * c + lane < v);
     const int nq16 = v / per16;  // 16-byte blocks of a row (<= 32)
-    const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
     // chunks of 32 rows (double-buffered groups) when every warp gets several of them, of
     // 8 (two groups) when every warp gets two, otherwise one group per chunk, so that the
     // rows spread over all warps (each chunk costs an atomic on the one work counter)
@@ -476,7 +505,7 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
         int64_t k = p0 + lane, key = k;
         int packed = 0;
         if (valid && a.list) {  // a head record of the claim pass: position and row
-            const longlong2 r = a.list[p0 + lane];
+            const longlong2 r = first && chunk == G ? record0 : a.list[p0 + lane];
             k = (int64_t)((uint64_t)r.x & ~kRecordPacked);
             key = r.y;
             packed = r.x < 0;
@@ -490,23 +519,21 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
         const int rows = __popc(fm);
         if (ok) {
             const int slot = __popc(fm & below);
-            mkey[slot] = key;
+            msrc[slot] = a.s.comp + key * v;
             mout[slot] = a.out + k * (int64_t)v;
             mpk[slot] = packed;
         }
         __syncwarp();
-        const unsigned okm = rows == 32 ? 0xffffffffu : ((1u << rows) - 1u);
         const unsigned pm = __ballot_sync(0xffffffffu, lane < rows && mpk[lane]);
         const int ng = (rows + G - 1) / G;
         // groups of G whole rows: the next group is copied into the other buffer while this
         // one decodes
         auto issue = [&](int g) {
-            U *buf = bufs + (g & 1) * G * sw;
+            U *buf = bufs + (g & 1) * G * sw + lane * per16;
 #pragma unroll
             for (int q = 0; q < G; ++q) {
                 const int r = g * G + q;
-                if (r < rows && lane < nq16)
-                    cp_async16(buf + q * sw + lane * per16, a.s.comp + mkey[r] * v + lane * per16);
+                if (r < rows && lane < nq16) cp_async16(buf + q * sw, msrc[r] + lane * per16);
             }
             cp_async_commit();
         };
@@ -519,11 +546,107 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
                 cp_async_wait_all();
             }
             __syncwarp();
-            hbm_decode_group<U, NC, G>(bufs + (g & 1) * G * sw, sw, g * G, rows, okm, pm, v, mw,
-                                       lt, full, mout, a.status);
+            const int last = min(rows, (g + 1) * G);
+            const U *row = bufs + (g & 1) * G * sw;
+#pragma unroll 1
+            for (int r = g * G; r < last; ++r, row += sw) {
+                U *o = mout[r] + lane;
+                if (!((pm >> r) & 1)) {  // stored raw
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (32 * c + lane < v) o[32 * c] = row[32 * c + lane];
+                    continue;
+                }
+                const uint32_t *units = reinterpret_cast<const uint32_t *>(row);
+                uint32_t bits[NC], every = 0xffffffffu;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    bits[c] = units[c];
+                    every &= bits[c] | absent[c];
+                }
+                if (every == 0xffffffffu && full_fits) {
+                    U x[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        uint32_t u[H + 1];
+#pragma unroll
+                        for (int i = 0; i <= H; ++i)
+                            u[i] = *reinterpret_cast<const uint32_t *>(
+                                reinterpret_cast<const char *>(row) + t.at[c][i]);
+                        x[c] = t.word(u, t.shift[c], c, false);
+                    }
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (32 * c + lane < v) o[32 * c] = x[c];
+                    continue;
+                }
+                // some word is stored whole: offsets from a prefix sum
+                uint32_t incl[NC], tot = 0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const bool cj = (bits[c] >> lane) & 1u;
+                    incl[c] = 32 * c + lane < v ? (cj ? (uint32_t)t.nb[c] : (uint32_t)W) : 0u;
+                }
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl[c], d);
+                        if (lane >= d) incl[c] += y;
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    incl[c] += tot;
+                    tot = __shfl_sync(0xffffffffu, incl[c], 31);
+                }
+                if (mw + (int)((tot + W - 1) / W) >= v) {
+                    // a bitmap claiming a stream as long as the raw row cannot come from this
+                    // mask: report it and leave the output row alone
+                    if (lane == 0) atomicOr(a.status, kStatusCorruptRow);
+                    continue;
+                }
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (32 * c + lane < v) {
+                        const bool cj = (bits[c] >> lane) & 1u;
+                        const int32_t s = (int32_t)incl[c] - (LEFT && cj ? t.nb[c] : W);
+                        uint32_t u[H + 1];
+#pragma unroll
+                        for (int i = 0; i <= H; ++i)
+                            u[i] = *reinterpret_cast<const uint32_t *>(
+                                reinterpret_cast<const char *>(row) +
+                                T::unit_byte((s >> 5) + i, mw));
+                        o[32 * c] = t.word(u, (uint32_t)s & 31u, c, !cj);
+                    }
+                }
+            }
             __syncwarp();
         }
     }
+}
+
+template <typename U, int NC, int G>
+__global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    // the column tables, the claim pass's list, the work counter and the status words come
+    // from the kernels before this one
+    grid_dep_wait();
+    grid_dep_release();
+    // all that does not depend on one another is read first: the row count, the record of the
+    // warp's first chunk should that be one group (the list has room for every position, so
+    // reading past its length is harmless), the columns
+    const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
+    const int64_t p = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G +
+                      (threadIdx.x & 31);
+    longlong2 record0 = make_longlong2(0, -1);
+    if (a.list && (threadIdx.x & 31) < G && p < a.nrows) record0 = a.list[p];
+    ShortColumns<U, NC> cols;
+    cols.load(a.s.t, (int)a.s.v);
+    if (cols.left_fits())
+        hbm_rows<U, NC, G, true>(a, smem, cols, nrows, record0);
+    else
+        hbm_rows<U, NC, G, false>(a, smem, cols, nrows, record0);
 }
 
 // Device rows of at most 64 words, each 16-byte aligned, fetched whole by hbm_rows_kernel
