@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     GroupTables<U> gt;
     uint32_t packed_bits = 0;  // stream bits of a row whose words are all compressible
     if constexpr (ONE) {
-        gt.load(a.s.t, v, 0);
+        gt.load(a.s.t, v, mw, 0, 0);
         packed_bits = gt.total;
     } else {
         for (int64_t j = lane; j < v; j += 32) packed_bits += (uint32_t)__ldg(a.s.t.nb + j) & 0xffu;
@@ -818,11 +818,14 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         __syncwarp();
         // lengths
         int64_t end = 0;
+        unsigned fm = 0;  // rows whose words are all compressible
 #pragma unroll 1
         for (unsigned m = pm; m; m &= m - 1) {
             const int q = __ffs(m) - 1;
+            bool full;
             const uint32_t bits = row_stream_bits<U>(slots + __shfl_sync(0xffffffffu, place, q), v,
-                                                     a.s.t, packed_bits);
+                                                     a.s.t, packed_bits, full);
+            fm |= (unsigned)full << q;
             if (lane == q) end = mw + (int64_t)((bits + W - 1) / W);
         }
         // a bitmap whose stream does not fit its row cannot come from this mask: report it and
@@ -868,9 +871,9 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         if (pm) {
             if constexpr (ONE) {
                 int64_t base = 0;
-                decode_group<U, int>(gt, slots, place, out, pm, 0, mw, base);
+                decode_group<U, int>(gt, slots, place, out, pm, fm, 0, mw, base);
             } else {
-                decode_rows_long<U, int>(slots, place, out, pm, v, mw, a.s.t);
+                decode_rows_long<U, int>(slots, place, out, pm, fm, v, mw, a.s.t);
             }
         }
         __syncwarp();

@@ -225,18 +225,23 @@ __device__ __forceinline__ int64_t row_words(const U *__restrict__ buf, int64_t 
 
 // ------------------------------------------------------------------ rows decoded together
 // The tables of a group of 512 bytes of columns (64 64-bit or 128 32-bit words; column
-// g0 + 32 * c + lane) and the bits its rows hold up to each column's end when every word of
-// the group is compressible.
+// g0 + 32 * c + lane), the bits its rows hold up to each column's end when every word of
+// the group is compressible, and, for rows that are all compressible (`before` bits in earlier
+// groups), where a column's word lies: the bytes from the row to its stream units and the shift
+// that brings its bits to the end.
 template <typename U>
 struct GroupTables {
-    static constexpr int GC = 16 / sizeof(U);
+    static constexpr int GC = 16 / sizeof(U), H = sizeof(U) / 4;
     U m[GC], bv[GC], mv[GC][kMoves];
     int kept[GC];
     uint32_t incl[GC], total;
+    int at[GC][H + 1];
+    uint32_t shift[GC];
     unsigned absent[GC];  // columns past the row's end
     int left;             // columns from this lane's first to the row's end
 
-    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t g0) {
+    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t mw, int64_t g0,
+                                         int64_t before) {
         const int lane = threadIdx.x & 31;
         left = (int)min(v - g0, (int64_t)(32 * GC)) - lane;
 #pragma unroll
@@ -265,6 +270,13 @@ struct GroupTables {
         for (int c = 0; c < GC; ++c) {
             incl[c] += total;
             total = __shfl_sync(0xffffffffu, incl[c], 31);
+            const int s = (int)(before + incl[c]) - 8 * (int)sizeof(U);
+#pragma unroll
+            for (int i = 0; i <= H; ++i) {
+                const int q = (s >> 5) + i;
+                at[c][i] = (int)mw * (int)sizeof(U) + 4 * (H == 2 ? q ^ 1 : q);
+            }
+            shift[c] = (uint32_t)s & 31u;
         }
     }
 };
@@ -272,16 +284,17 @@ struct GroupTables {
 // Decode the group's words of the rows of the lanes in `lanes`: each such lane holds its row's
 // place (words from `rows`, all in shared or all in global memory: bitmap, then the stream mw
 // words on), its output row and the bits of the stream in earlier groups (base, advanced).  A
-// word's bits are read as the stream bits that end at its end, which a group whose words are
-// all compressible takes from the tables and any other from a prefix sum; the words of a
+// word's bits are read as the stream bits that end at its end: at the places in the tables for
+// the rows in `full`, which are all compressible, else at its own, from the tables for a
+// group whose words are all compressible and from a prefix sum for any other; the words of a
 // group are then read, scattered and written without a branch between them.  (Columns past the
 // end read where the row's last word ends, and what they read is not written.)  One row at a
 // time in a loop that is not unrolled: four rows' code side by side missed the instruction
 // cache (device_fetch_kernel, 100k rows of 256 32-bit words: 139 us, with the loop 83).
 template <typename U, typename Place>
 __device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *rows, Place place,
-                                             U *out, unsigned lanes, int64_t g0, int64_t mw,
-                                             int64_t &base) {
+                                             U *out, unsigned lanes, unsigned full, int64_t g0,
+                                             int64_t mw, int64_t &base) {
     constexpr int W = 8 * sizeof(U), GC = GroupTables<U>::GC;
     constexpr int LW = LogW<U>::value;
     const int lane = threadIdx.x & 31;
@@ -290,10 +303,30 @@ __device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *r
         const int q = __ffs(lanes) - 1;
         lanes &= lanes - 1;
         const U *row = rows + __shfl_sync(0xffffffffu, place, q);
-        const int64_t at = __shfl_sync(0xffffffffu, base, q);
         U *o = reinterpret_cast<U *>(
                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), q)) +
                g0 + lane;
+        if ((full >> q) & 1) {
+            constexpr int H = GroupTables<U>::H;
+            const char *r = reinterpret_cast<const char *>(row);
+            U x[GC];
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+                uint32_t u[H + 1];
+#pragma unroll
+                for (int i = 0; i <= H; ++i)
+                    u[i] = *reinterpret_cast<const uint32_t *>(r + t.at[c][i]);
+                U y = __funnelshift_l(u[1], u[0], t.shift[c]);
+                if constexpr (H == 2)
+                    y = (uint64_t)y << 32 | __funnelshift_l(u[H], u[1], t.shift[c]);
+                x[c] = scatter_word<U>(y, t.m[c], t.bv[c], t.kept[c] >> 8, t.mv[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < GC; ++c)
+                if (32 * c < t.left) o[32 * c] = x[c];
+            continue;
+        }
+        const int64_t at = __shfl_sync(0xffffffffu, base, q);
         const uint32_t *units = reinterpret_cast<const uint32_t *>(row) + (g0 >> 5);
         const U *gs = row + mw + (at >> LW);
         const int32_t off = (int32_t)(at & (W - 1));
@@ -346,13 +379,14 @@ __device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *r
 // link round trip, decode_row is shorter (2048 rows of 128 64-bit words: 48.2 against 51 us).
 template <typename U, typename Place>
 __device__ __forceinline__ void decode_rows_long(const U *rows, Place place, U *out,
-                                                 unsigned lanes, int64_t v, int64_t mw,
-                                                 const ColTables<U> &t) {
-    int64_t base = 0;
+                                                 unsigned lanes, unsigned full, int64_t v,
+                                                 int64_t mw, const ColTables<U> &t) {
+    int64_t base = 0, before = 0;
     for (int64_t g0 = 0; g0 < v; g0 += 32 * GroupTables<U>::GC) {
         GroupTables<U> gt;
-        gt.load(t, v, g0);
-        decode_group<U, Place>(gt, rows, place, out, lanes, g0, mw, base);
+        gt.load(t, v, mw, g0, before);
+        decode_group<U, Place>(gt, rows, place, out, lanes, full, g0, mw, base);
+        before += gt.total;
     }
 }
 
@@ -362,23 +396,24 @@ template <typename U>
 __device__ __noinline__ void decode_source_rows(const U *rows, int64_t place, U *out,
                                                 unsigned lanes, int64_t v, int64_t mw,
                                                 const ColTables<U> &t) {
-    decode_rows_long<U, int64_t>(rows, place, out, lanes, v, mw, t);
+    decode_rows_long<U, int64_t>(rows, place, out, lanes, 0, v, mw, t);
 }
 
-// Stream bits of the row whose bitmap is at `row`: `packed` when every word is compressible (the
-// usual row, seen from the bitmap alone), else the sum over the columns.
+// Stream bits of the row whose bitmap is at `row`: `packed` when every word is compressible
+// (`full`, the usual row, seen from the bitmap alone), else the sum over the columns.
 template <typename U>
 __device__ __forceinline__ uint32_t row_stream_bits(const U *row, int64_t v, const ColTables<U> &t,
-                                                    uint32_t packed) {
+                                                    uint32_t packed, bool &full) {
     constexpr int W = 8 * sizeof(U);
     const int lane = threadIdx.x & 31;
     const uint32_t *bitmap = reinterpret_cast<const uint32_t *>(row);
     const int64_t units = (v + 31) / 32;
     const uint32_t absent = v & 31 ? ~0u << (v & 31) : 0u;  // of the last unit
-    bool full = true;
+    full = true;
     for (int64_t i = lane; i < units; i += 32)
         full = full && (bitmap[i] | (i == units - 1 ? absent : 0u)) == ~0u;
-    if (__all_sync(0xffffffffu, full)) return packed;
+    full = __all_sync(0xffffffffu, full);
+    if (full) return packed;
     uint32_t bits = 0;
     for (int64_t j = lane; j < v; j += 32)
         bits += (bitmap[j >> 5] >> lane) & 1u ? (uint32_t)__ldg(t.nb + j) & 0xffu : (uint32_t)W;
