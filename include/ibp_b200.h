@@ -56,9 +56,10 @@ int ibp_abi_version(void);
 void ibp_set_debug(int on);
 
 /* How decompress_fetch (and its condensed and no-alloc forms) finds the repeated rows of an
- * index array, process-wide: 0 = auto (hash table for compressed rows, fixed-stride or
- * condensed, in device memory, or in host memory when the index has fewer than a quarter as
- * many entries as the set has rows; else sort), 1 = always sort (rows then fetched in row
+ * index array, process-wide: 0 = auto (rows, fixed-stride or condensed, in device memory are
+ * decoded once per index entry where that is as fast as copying repeats, else hash table; hash
+ * table for rows in host memory when the index has fewer than a quarter as many entries as the
+ * set has rows; else sort), 1 = always sort (rows then fetched in row
  * order), 2 = always hash (repeats are then copied inside the fetch for host rows).  Dense
  * host batches whose rows repeat a lot (skewed, e.g. Zipf) are faster with 2; dense batches
  * with few repeats are faster sorted.  No counterpart in the reference (it always sorts). */

@@ -94,9 +94,10 @@ _DEDUP_MODES = {"auto": 0, "sort": 1, "hash": 2}
 
 def set_fetch_dedup(mode):
     """How decompress_fetch finds the repeated rows of an index array, process-wide (no
-    counterpart in the reference, which always sorts): "auto" (hash table for compressed rows
-    in device memory and for sparse host batches, else sort), "sort", or "hash" (repeats are
-    then copied inside the fetch for host rows).  Dense batches whose rows repeat a lot are
+    counterpart in the reference, which always sorts): "auto" (rows in device memory decode
+    every position where that is as fast as copying repeats, else hash table; hash table for
+    sparse host batches, else sort), "sort", or "hash" (repeats are then copied inside the fetch
+    for host rows).  Dense batches whose rows repeat a lot are
     faster with "hash", dense batches with few repeats with "sort".  Also takes 0/1/2."""
     from . import _capi
     m = _DEDUP_MODES.get(mode, mode) if isinstance(mode, str) else mode

@@ -21,16 +21,16 @@
 //    registers, loaded once per warp; longer host rows read them through the L1 cache, four
 //    chunks at a time, and place the bits of columns that keep at most 4 directly from the
 //    mask; longer device rows load them once for up to 16 rows decoded together.
-//  * index arrays: each distinct row crosses the link once.  Dense batches of host rows (a
+//  * index arrays of host rows: each distinct row crosses the link once.  Dense batches (a
 //    quarter of the rows or more) and raw gathers are fetched in sorted index order (cub
 //    radix sort on only the bits the row count needs) so concurrent warps read neighbouring
-//    host pages.  Compressed rows (fixed-stride or condensed) in HBM, and sparse batches of
-//    them in host memory, where order gains little, claim rows in an open-addressing hash
-//    table instead: inside the fetch for host rows (hidden behind PCIe), in a claim pass
-//    that lists the distinct rows for HBM rows.  Repeats (Zipf mini-batches repeat hot
-//    rows a lot) copy their first occurrence's output row: inside the fetch for host rows,
-//    once that row is published in the table (so the copies overlap the PCIe reads), and
-//    in a copy kernel afterwards for the other modes.
+//    host pages.  Sparse batches, where order gains little, claim rows in an open-addressing
+//    hash table inside the fetch (hidden behind PCIe).  Repeats (Zipf mini-batches repeat hot
+//    rows a lot) copy their first occurrence's output row inside the fetch, once that row is
+//    published in the table (so the copies overlap the PCIe reads).
+//  * index arrays of device rows: a repeat is decoded again, its compressed row read through
+//    L1, where that is as fast as finding and copying it (kDirectRows); else a claim pass
+//    lists the distinct rows and a copy kernel fills the repeats afterwards.
 //  * no allocation, no host synchronisation: everything lives in the caller's workspace
 //    and is enqueued on the caller's stream.
 #include <cub/device/device_radix_sort.cuh>
@@ -316,9 +316,9 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
 // ------------------------------------------------------------------ HBM rows of <= 64 words
 // Rows in device memory are not bound by a link but by the instructions around the decode,
 // so this kernel keeps per-row bookkeeping to a minimum: a warp takes a chunk of listed rows
-// from a work counter (the claim pass's head records -- position with the row's
-// stored-compressed flag, and row -- or rows p, p+1, ... of an unindexed fetch; 4 to 32 rows
-// at a time by the batch's size), parks their sources and output rows in shared memory, and
+// from a work counter (positions of an index array, rows p, p+1, ... of an unindexed fetch, or
+// the claim pass's head records -- position with the row's stored-compressed flag, and row;
+// 4 to 32 rows at a time by the batch's size), parks their sources and output rows in shared memory, and
 // copies groups of G whole rows (one 16-byte cp.async per lane and row; rows must be 16-byte
 // aligned) into one of two shared buffers while it decodes the previous group from the
 // other.
@@ -328,14 +328,13 @@ __global__ void __launch_bounds__(kFetchThreads, 2) fetch_rows_kernel(FetchArgs<
 // whole kernel, funnel shifts by fixed amounts, the moves and a store (ShortTables::word);
 // any other row takes a prefix sum.  Moves: a word's halves are read either as the bits that
 // start where it starts and moved right into place (LEFT), or as the bits that end where it ends
-// and moved left; LEFT when two moves (three places) suffice for every column, as for masks
-// that drop little above what they keep, else five moves the other way.  The row's stream
+// and moved left; LEFT when one or two moves (three places) suffice for every column, as for
+// masks that drop little above what they keep, else five moves the other way.  The row's stream
 // length falls out of the offsets (no separate length pass, no tail reads), and stream offsets
 // are 32-bit.
 // Bound: issue, then HBM (whole rows are read: 512 + 512 bytes for a 64-word row).  200k rows of
 // 64 64-bit words at 264 stored bytes: 57 us with offsets and reads worked out per row, 53 with
-// 32-bit halves, 39.6 now (5.2 TB/s of the bytes it moves); the 79k distinct rows of a 400k-row
-// batch 34.1 -> 28.4 us.
+// 32-bit halves, 39.6 now (5.2 TB/s of the bytes it moves).
 template <typename U, int NC>
 struct ShortColumns {
     U mask[NC], val[NC];
@@ -353,27 +352,27 @@ struct ShortColumns {
         }
     }
 
-    // two moves suffice for every column of the row
-    __device__ __forceinline__ bool left_fits() const {
-        bool fits = true;
+    // most places any kept bit is moved when packed left
+    __device__ __forceinline__ int places() const {
+        int most = 0;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const U sel = (U)~mask[c];
-            fits = fits && moves_left((uint32_t)sel) < 4;
-            if (sizeof(U) == 8) fits = fits && moves_left((uint32_t)((uint64_t)sel >> 32)) < 4;
+            most = max(most, moves_left((uint32_t)sel));
+            if (sizeof(U) == 8) most = max(most, moves_left((uint32_t)((uint64_t)sel >> 32)));
         }
-        return __all_sync(0xffffffffu, fits);
+        return __reduce_max_sync(0xffffffffu, most);
     }
 };
 
-template <typename U, int NC, bool LEFT>
+template <typename U, int NC, int LV>
 struct ShortTables {
     static constexpr int W = 8 * sizeof(U), H = sizeof(U) / 4;  // halves, high first
-    static constexpr int MV = LEFT ? 2 : kMoves;
-    uint32_t m[NC][H], bv[NC][H], mv[NC][H][MV];
+    static constexpr bool LEFT = LV < kMoves;
+    uint32_t m[NC][H], bv[NC][H], mv[NC][H][LV];
     int nb[NC], split[NC];  // kept bits; of the high half (LEFT) or the low half
     uint32_t total;         // stream bits of a row whose words are all compressible
-    int at[NC][H + 1];      // byte offsets from the row of the units that row's word lies in
+    int at[NC][H];          // byte offsets from the row of the units that row's word lies in
     uint32_t shift[NC];
 
     // unit `q` of the stream in bytes from the row's start (mw words of bitmap before it)
@@ -401,7 +400,7 @@ struct ShortTables {
                     uint32_t all[kMoves];
                     move_masks<false>(~m[c][h], all);
 #pragma unroll
-                    for (int i = 0; i < MV; ++i) mv[c][h][i] = all[i];
+                    for (int i = 0; i < LV; ++i) mv[c][h][i] = all[i];
                 }
             }
             if constexpr (!LEFT) {
@@ -421,10 +420,22 @@ struct ShortTables {
             }
             const int32_t s = (int32_t)(total + incl) - (LEFT ? nb[c] : W);
 #pragma unroll
-            for (int i = 0; i <= H; ++i) at[c][i] = unit_byte((s >> 5) + i, mw);
+            for (int i = 0; i < H; ++i) at[c][i] = unit_byte((s >> 5) + i, mw);
             shift[c] = (uint32_t)s & 31u;
             total += __shfl_sync(0xffffffffu, incl, 31);
         }
+    }
+
+    // The word of column 32 * c + lane of an all-compressible row.
+    __device__ __forceinline__ U word_at(const U *row, int c) const {
+        const char *r = reinterpret_cast<const char *>(row);
+        uint32_t u[H + 1];
+#pragma unroll
+        for (int i = 0; i < H; ++i) u[i] = *reinterpret_cast<const uint32_t *>(r + at[c][i]);
+        // unit q + 2 lies two units after unit q, whichever way 64-bit words' halves lie (unit
+        // q + 1 after unit q for 32-bit words)
+        u[H] = *reinterpret_cast<const uint32_t *>(r + at[c][0] + 4 * H);
+        return word(u, shift[c], c, false);
     }
 
     // The word of column 32 * c + lane from the H + 1 stream units u around it (the bits start,
@@ -444,7 +455,7 @@ struct ShortTables {
 #pragma unroll
         for (int h = 0; h < H; ++h) {
             if constexpr (LEFT)
-                x[h] = scatter_top<MV>(x[h], ~m[c][h], bv[c][h], mv[c][h]);
+                x[h] = scatter_top<LV>(x[h], ~m[c][h], bv[c][h], mv[c][h]);
             else
                 x[h] = scatter_half(x[h], ~m[c][h], bv[c][h], mv[c][h]);
             x[h] = raw ? w[h] : x[h];
@@ -458,11 +469,10 @@ struct ShortTables {
 // of its (up to) 32 rows, then two buffers of G row slots.
 constexpr size_t kHbmWarpMetaBytes = 512 + 128;
 
-template <typename U, int NC, int G, bool LEFT>
+template <typename U, int NC, int G, int LV>
 __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *smem,
-                                         const ShortColumns<U, NC> &cols, int64_t nrows,
-                                         longlong2 record0) {
-    using T = ShortTables<U, NC, LEFT>;
+                                         const ShortColumns<U, NC> &cols, int64_t nrows) {
+    using T = ShortTables<U, NC, LV>;
     constexpr int per16 = 16 / sizeof(U), W = T::W, H = T::H;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char *meta = smem + warp * kHbmWarpMetaBytes;
@@ -481,11 +491,13 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
 #pragma unroll
     for (int c = 0; c < NC; ++c) absent[c] = ~__ballot_sync(0xffffffffu, 32 * c + lane < v);
     const int nq16 = v / per16;  // 16-byte blocks of a row (<= 32)
-    // chunks of 32 rows (double-buffered groups) when every warp gets several of them, of
-    // 8 (two groups) when every warp gets two, otherwise one group per chunk, so that the
-    // rows spread over all warps (each chunk costs an atomic on the one work counter)
+    // a warp's share of the rows in equal chunks of at most 32, whole groups each (a chunk costs
+    // an atomic on the one work counter and a round trip for its rows' metadata; 400k rows of
+    // 64 64-bit words in chunks of 4, 8, 16, 32: 94, 61, 56, 56 us; 100k rows in chunks of 16:
+    // 25 us, of the 24 that give every warp one: 21)
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int chunk = nrows >= 4 * 32 * nwarps ? 32 : (nrows >= 16 * nwarps ? 8 : G);
+    const int64_t share = (nrows + nwarps - 1) / nwarps, parts = max((share + 31) / 32, (int64_t)1);
+    const int chunk = (int)max((int64_t)G, ((share + parts - 1) / parts + G - 1) / G * G);
     const unsigned below = (1u << lane) - 1u;
     // a warp's first chunk is its own (warp w takes chunk w); later ones come from the work
     // counter, so the grid's warps do not all queue on the counter at the start
@@ -505,10 +517,12 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
         int64_t k = p0 + lane, key = k;
         int packed = 0;
         if (valid && a.list) {  // a head record of the claim pass: position and row
-            const longlong2 r = first && chunk == G ? record0 : a.list[p0 + lane];
+            const longlong2 r = a.list[p0 + lane];
             k = (int64_t)((uint64_t)r.x & ~kRecordPacked);
             key = r.y;
             packed = r.x < 0;
+        } else if (valid && a.keys) {
+            key = a.keys[p0 + lane];
         }
         const bool bad = valid && (key < 0 || key >= a.s.n);
         if (bad) atomicOr(a.status, kStatusBadIndex);
@@ -533,7 +547,7 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
 #pragma unroll
             for (int q = 0; q < G; ++q) {
                 const int r = g * G + q;
-                if (r < rows && lane < nq16) cp_async16(buf + q * sw, msrc[r] + lane * per16);
+                if (r < rows && lane < nq16) cp_async16<true>(buf + q * sw, msrc[r] + lane * per16);
             }
             cp_async_commit();
         };
@@ -548,6 +562,29 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
             __syncwarp();
             const int last = min(rows, (g + 1) * G);
             const U *row = bufs + (g & 1) * G * sw;
+            // lane q looks at row q's bitmap: the group is usually all compressible
+            bool full = true;
+            if (lane < last - g * G) {
+                const uint32_t *units = reinterpret_cast<const uint32_t *>(row + lane * sw);
+                uint32_t every = 0xffffffffu;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) every &= units[c] | absent[c];
+                full = every == 0xffffffffu && ((pm >> (g * G + lane)) & 1);
+            }
+            if (__all_sync(0xffffffffu, full) && full_fits) {
+#pragma unroll 2
+                for (int r = g * G; r < last; ++r, row += sw) {
+                    U *o = mout[r] + lane;
+                    U x[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) x[c] = t.word_at(row, c);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (32 * c + lane < v) o[32 * c] = x[c];
+                }
+                __syncwarp();
+                continue;
+            }
 #pragma unroll 1
             for (int r = g * G; r < last; ++r, row += sw) {
                 U *o = mout[r] + lane;
@@ -565,19 +602,9 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
                     every &= bits[c] | absent[c];
                 }
                 if (every == 0xffffffffu && full_fits) {
-                    U x[NC];
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        uint32_t u[H + 1];
-#pragma unroll
-                        for (int i = 0; i <= H; ++i)
-                            u[i] = *reinterpret_cast<const uint32_t *>(
-                                reinterpret_cast<const char *>(row) + t.at[c][i]);
-                        x[c] = t.word(u, t.shift[c], c, false);
-                    }
 #pragma unroll
                     for (int c = 0; c < NC; ++c)
-                        if (32 * c + lane < v) o[32 * c] = x[c];
+                        if (32 * c + lane < v) o[32 * c] = t.word_at(row, c);
                     continue;
                 }
                 // some word is stored whole: offsets from a prefix sum
@@ -610,7 +637,7 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
                 for (int c = 0; c < NC; ++c) {
                     if (32 * c + lane < v) {
                         const bool cj = (bits[c] >> lane) & 1u;
-                        const int32_t s = (int32_t)incl[c] - (LEFT && cj ? t.nb[c] : W);
+                        const int32_t s = (int32_t)incl[c] - (T::LEFT && cj ? t.nb[c] : W);
                         uint32_t u[H + 1];
 #pragma unroll
                         for (int i = 0; i <= H; ++i)
@@ -633,20 +660,17 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
     // from the kernels before this one
     grid_dep_wait();
     grid_dep_release();
-    // all that does not depend on one another is read first: the row count, the record of the
-    // warp's first chunk should that be one group (the list has room for every position, so
-    // reading past its length is harmless), the columns
+    // the row count and the columns do not depend on one another: read first, together
     const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
-    const int64_t p = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * G +
-                      (threadIdx.x & 31);
-    longlong2 record0 = make_longlong2(0, -1);
-    if (a.list && (threadIdx.x & 31) < G && p < a.nrows) record0 = a.list[p];
     ShortColumns<U, NC> cols;
     cols.load(a.s.t, (int)a.s.v);
-    if (cols.left_fits())
-        hbm_rows<U, NC, G, true>(a, smem, cols, nrows, record0);
+    const int places = cols.places();
+    if (places < 2)
+        hbm_rows<U, NC, G, 1>(a, smem, cols, nrows);
+    else if (places < 4)
+        hbm_rows<U, NC, G, 2>(a, smem, cols, nrows);
     else
-        hbm_rows<U, NC, G, false>(a, smem, cols, nrows, record0);
+        hbm_rows<U, NC, G, kMoves>(a, smem, cols, nrows);
 }
 
 // Device rows of at most 64 words, each 16-byte aligned, fetched whole by hbm_rows_kernel
@@ -654,7 +678,7 @@ __global__ void __launch_bounds__(256, 4) hbm_rows_kernel(FetchArgs<U> a) {
 template <typename U>
 static bool hbm_rows_fit(const FetchArgs<U> &a) {
     return a.device_rows && !a.raw_only && !a.dedup && !a.pos && !a.s.offsets &&
-           (!a.keys || a.list) && a.s.v <= 64 &&
+           a.s.v <= 64 &&
            (a.s.v * (int64_t)sizeof(U)) % 16 == 0 && (((uintptr_t)a.s.comp) & 15) == 0;
 }
 
@@ -780,7 +804,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         const int n = (int)((to + 15 - b0) >> 4);
         const char *src = reinterpret_cast<const char *>(b0) + lane * 16;
         char *dst = reinterpret_cast<char *>(slot) + (b0 - (lo & ~(uintptr_t)15)) + lane * 16;
-        for (int i = lane; i < n; i += 32, src += 512, dst += 512) cp_async16(dst, src);
+        for (int i = lane; i < n; i += 32, src += 512, dst += 512) cp_async16<true>(dst, src);
     };
 
     int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1097,6 +1121,15 @@ static ibp_status launch_prep(int32_t *status, const U *mask, const U *bitval, i
     return IBP_OK;
 }
 
+// Indexed fetches of device rows up to this many positions do not look for repeats; rows that
+// hbm_rows_kernel takes never do.  With repeats claimed and copied by two more kernels a
+// 400k-row Zipf(1.1) batch of 64 64-bit words took 74 us (three quarters of it repeats), a uniform
+// one 120; decoding every position 51 and 74, through L1 (through L2 124: one slice serves a hot
+// row's lines).  The other device rows decode 3-10 times slower: 30k positions of 65 64-bit words,
+// Zipf(1.1), 36.7 us claimed and 34.5 direct (uniform 49 and 35), 100k positions 48.9 and 68
+// (uniform 82 and 69); of 512 words 107 and 83 at 30k, 142 and 235 at 100k.
+constexpr int64_t kDirectRows = 32768;
+
 template <typename U>
 ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
                            const U *bitval, const int32_t *bitmask, const int64_t *idx,
@@ -1158,6 +1191,13 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
         return IBP_ERR_UNSUPPORTED;
     }
     const int mode = fetch_dedup_mode();
+    if (mode == 0 && (hbm_rows_fit(a) || (device_fetch_fit(a) && nidx <= kDirectRows))) {
+        // device rows that decode as fast as their repeats would be found and copied: every
+        // position decodes its row, in one kernel
+        IBP_RET(launch_prep<U>(status, mask, bitval, v, t, tables, nullptr, 0, st));
+        a.keys = idx;
+        return launch_fetch<U>(a, nblks, nthreads, st);
+    }
     if (mode == 2 || (mode == 0 && impl != 2 && (on_device || 4 * nidx < n))) {
         // compressed rows (fixed-stride or condensed) in HBM, or a sparse batch of them in
         // host memory: claim rows in a hash table instead of sorting (HBM does not care about

@@ -90,3 +90,50 @@ def test_bad_indices_are_reported_and_the_rest_is_right(wb, v):
             assert bool((out[~good] == 7).all())
     finally:
         ibp.set_fetch_dedup("auto")
+
+
+@pytest.mark.parametrize("count", [32767, 32768, 32769])
+@pytest.mark.parametrize("wb,v", [(8, 33), (8, 64), (4, 300)])
+def test_batches_around_the_direct_limit(wb, v, count):
+    """Skewed batches on both sides of the size up to which repeats are decoded again, rows of the
+    kernel that has no such limit among them; condensed rows too."""
+    import invariantbitpacking_b200 as ibp
+    rng = np.random.default_rng(count + v)
+    x, m, b = rows_of(rng, 3000, v, wb, 0.6)
+    dm, db = torch.from_numpy(m).cuda(), torch.from_numpy(b).cuda()
+    src = torch.from_numpy(x).cuda()
+    t = src.clone()
+    bm = ibp.compress_inplace(t, dm, db)
+    k = torch.from_numpy(np.minimum(rng.zipf(1.3, count) - 1, 2999)).cuda()
+    out = ibp.decompress_fetch(t, dm, db, bm, "cuda", None, k, check=True)
+    assert torch.equal(out, src[k])
+    words, offs = ibp.compress_condensed(src.clone(), dm, db)
+    out = ibp.decompress_fetch_condensed(words, offs, dm, db, v, "cuda", k, check=True)
+    assert torch.equal(out, src[k])
+
+
+@pytest.mark.parametrize("low,high", [(0, 31), (1, 30), (3, 28), (4, 27), (31, 0), (16, 16)])
+@pytest.mark.parametrize("wb,v", [(8, 64), (8, 40), (4, 64), (4, 20)])
+def test_masks_that_need_few_moves_and_many(wb, v, low, high):
+    """Kept bits in one run with `high` dropped bits above and `low` below in every 32-bit half:
+    the short-row kernel picks its moves by how many are dropped above."""
+    import invariantbitpacking_b200 as ibp
+    rng = np.random.default_rng(10 * low + v)
+    keep = ((1 << 32) - 1) >> high & ~((1 << low) - 1)
+    half = np.uint64(~keep & 0xFFFFFFFF)
+    m = np.full(v, half | (half << np.uint64(32)) if wb == 8 else half, dtype=np.uint64)
+    noise = rng.integers(0, 2**64, (700, v), dtype=np.uint64)
+    base = rng.integers(0, 2**64, v, dtype=np.uint64) & m
+    x = (noise & ~m) | base
+    x = np.where(rng.random((700, v)) < 0.02 * (rng.random((700, 1)) < 0.3), noise, x)
+    x = x.astype(UINT[wb]).view(INT[wb])
+    dm = torch.from_numpy(m.astype(UINT[wb]).view(INT[wb])).cuda()
+    db = torch.from_numpy(base.astype(UINT[wb]).view(INT[wb])).cuda()
+    src = torch.from_numpy(x).cuda()
+    t = src.clone()
+    bm = ibp.compress_inplace(t, dm, db)
+    out = ibp.decompress_fetch(t, dm, db, bm, "cuda", check=True)
+    assert torch.equal(out, src)
+    k = torch.from_numpy(rng.integers(0, 700, 5000)).cuda()
+    out = ibp.decompress_fetch(t, dm, db, bm, "cuda", None, k, check=True)
+    assert torch.equal(out, src[k])
