@@ -289,37 +289,48 @@ def decompress_fetch(comp_dataset, mask, bitval, bitmask, out_device, comp_len_=
     RuntimeError when an index was out of range or a row could not be decoded; the default
     leaves those rows unwritten without a host synchronisation (print_debug(True) prints a
     message instead)."""
-    _torch_check(comp_dataset.is_cuda or comp_dataset.is_pinned(),
-                 "Input tensor must accessible by CUDA device (GPU or pinned memory)")
-    dim = comp_dataset.dim()
-    _torch_check(dim in (1, 2),
-                 "Input tensor must be 1D [vec_size] or 2D [num_vecs x vec_size] got "
-                 f"{dim}")
-    _torch_check(comp_dataset.is_contiguous(), "Input tensor must be contiguous")
-    _torch_check(mask.is_cuda or mask.is_pinned(),
-                 "Mask tensor must accessible by CUDA device (GPU or pinned memory)")
-    _torch_check(bitval.is_cuda or bitval.is_pinned(),
-                 "Bitval tensor must accessible by CUDA device (GPU or pinned memory)")
-    wb = comp_dataset.element_size()
-    _torch_check(wb in (4, 8), "Input tensor must be 4-byte or 8-byte datatype")
-    _torch_check(mask.element_size() == wb and bitval.element_size() == wb,
-                 "Mask and bitval tensors must have the same datatype size (4-byte or 8-byte) "
-                 "as input dataset")
-    if bitmask.dtype != torch.int32:
-        raise RuntimeError(f"expected scalar type Int but found {bitmask.dtype}")
+    # written out rather than through _torch_check: a small fetch is as long as its host time,
+    # and every call and message built here showed in it
+    comp_cuda, mask_cuda = comp_dataset.is_cuda, mask.is_cuda
+    if not comp_cuda and not comp_dataset.is_pinned():
+        raise RuntimeError("Input tensor must accessible by CUDA device (GPU or pinned memory)")
     shape = comp_dataset.shape
-    n, v = (1, shape[0]) if dim == 1 else (shape[0], shape[1])
-    if not isinstance(out_device, torch.device):
+    dim = len(shape)
+    if dim != 2 and dim != 1:
+        raise RuntimeError("Input tensor must be 1D [vec_size] or 2D [num_vecs x vec_size] got "
+                           f"{dim}")
+    if not comp_dataset.is_contiguous():
+        raise RuntimeError("Input tensor must be contiguous")
+    if not mask_cuda and not mask.is_pinned():
+        raise RuntimeError("Mask tensor must accessible by CUDA device (GPU or pinned memory)")
+    if not bitval.is_cuda and not bitval.is_pinned():
+        raise RuntimeError("Bitval tensor must accessible by CUDA device (GPU or pinned memory)")
+    wb = comp_dataset.element_size()
+    if wb != 8 and wb != 4:
+        raise RuntimeError("Input tensor must be 4-byte or 8-byte datatype")
+    if mask.element_size() != wb or bitval.element_size() != wb:
+        raise RuntimeError("Mask and bitval tensors must have the same datatype size (4-byte or "
+                           "8-byte) as input dataset")
+    if bitmask.dtype is not torch.int32:
+        raise RuntimeError(f"expected scalar type Int but found {bitmask.dtype}")
+    n, v = shape if dim == 2 else (1, shape[0])
+    cur = _get_device()
+    if out_device == "cuda":
+        out_device = _cuda_devices.get(cur) or _cuda_devices.setdefault(
+            cur, torch.device("cuda", cur))
+    elif not isinstance(out_device, torch.device):
         out_device = torch.device(out_device)
-    if out_device.type == "cuda" and out_device.index is None:
-        out_device = torch.device("cuda", _get_device())
+    out_cuda = out_device.type == "cuda"
+    if out_cuda and out_device.index is None:
+        out_device = torch.device("cuda", cur)
     idx = None
     if index_array_ is not None:
-        _torch_check(index_array_.is_cuda,
-                     "Index array must accessible by CUDA device (GPU or pinned memory)")
-        _torch_check(index_array_.dim() == 1, "Index array should be 1D")
+        if not index_array_.is_cuda:
+            raise RuntimeError("Index array must accessible by CUDA device (GPU or pinned memory)")
+        if index_array_.dim() != 1:
+            raise RuntimeError("Index array should be 1D")
         idx = index_array_
-        if idx.dtype != torch.int64:
+        if idx.dtype is not torch.int64:
             idx = idx.to(torch.int64)
         if not idx.is_contiguous():
             idx = idx.contiguous()
@@ -336,13 +347,15 @@ def decompress_fetch(comp_dataset, mask, bitval, bitmask, out_device, comp_len_=
         _torch_check(output_tensor.shape[0] == nrows and output_tensor.shape[1] == v,
                      "Output tensor shape does not match expected decompressed shape")
         out = output_tensor
+    elif out_cuda:
+        out = torch.empty((nrows, v), dtype=comp_dataset.dtype, device=out_device)
     else:
         out = torch.empty((nrows, v), dtype=comp_dataset.dtype, device=out_device,
-                          pin_memory=out_device.type != "cuda")
-    if out_device.type != "cuda" and not out.is_pinned():
+                          pin_memory=True)
+    if not out_cuda and not out.is_pinned():
         out = out.pin_memory()
-    dev = _cuda_device(comp_dataset, mask, idx, out)
-    cur = _get_device()
+    dev = (comp_dataset.device if comp_cuda else mask.device if mask_cuda
+           else _cuda_device(idx, out))
     if dev.index is not None and dev.index != cur:
         with torch.cuda.device(dev):
             return _fetch_call(comp_dataset, n, v, wb, mask, bitval, bitmask, idx, nrows,
@@ -351,21 +364,25 @@ def decompress_fetch(comp_dataset, mask, bitval, bitmask, out_device, comp_len_=
                        out, nblks_, nthreads_, impl, dev, cur, check)
 
 
+_cuda_devices = {}  # device index -> torch.device
+
+
 def _fetch_call(comp_dataset, n, v, wb, mask, bitval, bitmask, idx, nrows, comp_len, out,
                 nblks_, nthreads_, impl, dev, dev_index, check):
-    need = _lib.ibp_decompress_fetch_workspace_size(nrows, v, wb, 0 if idx is None else 1)
-    ws, wsb = _workspace(need, dev)
+    wsb = _lib.ibp_decompress_fetch_workspace_size(nrows, v, wb, 0 if idx is None else 1)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
     stream = _stream_of(dev_index)
-    _check(_lib.ibp_decompress_fetch(
+    status = _lib.ibp_decompress_fetch(
         comp_dataset.data_ptr(), n, v, wb, mask.data_ptr(), bitval.data_ptr(),
         bitmask.data_ptr(), None if idx is None else idx.data_ptr(),
         -1 if idx is None else nrows, comp_len, out.data_ptr(),
         -1 if nblks_ is None else int(nblks_),
-        -1 if nthreads_ is None else int(nthreads_), impl,
-        None if ws is None else ws.data_ptr(), wsb, stream))
+        -1 if nthreads_ is None else int(nthreads_), impl, ws.data_ptr(), wsb, stream)
+    if status:
+        _check(status)
     if check:
         _raise_on_status(ws, "decompress_fetch")
-    elif _debug and ws is not None:
+    elif _debug:
         st = torch.zeros(1, dtype=torch.int32)
         import ctypes
         _check(_lib.ibp_read_status(_ptr(ws), ctypes.c_void_p(st.data_ptr()), stream))
