@@ -205,17 +205,16 @@ __device__ __forceinline__ int unit_slot(int64_t q) {
     return sizeof(U) == 8 ? (int)(q ^ 1) : (int)q;
 }
 
-// OR a word's bits (left-aligned in hi:lo, the rest zero; hi alone for 32-bit words) into a
-// shared-memory image at bit s.  The image's units are in stream order.
+// OR up to 64 bits (left-aligned in hi:lo, the rest zero) into a shared-memory image at bit s.
+// The image's units are in stream order; units of no bits are ORed too (a test costs more).
 __device__ __forceinline__ void or_shared(uint32_t addr, uint32_t x) {
     asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
 }
-template <typename U>
 __device__ __forceinline__ void put_bits(uint32_t image, uint32_t s, uint32_t hi, uint32_t lo) {
     const uint32_t at = image + ((s >> 3) & ~3u), off = s & 31;
     or_shared(at, hi >> off);
     or_shared(at + 4, __funnelshift_r(lo, hi, off));
-    if constexpr (sizeof(U) == 8) or_shared(at + 8, __funnelshift_r(0, lo, off));
+    or_shared(at + 8, __funnelshift_r(0, lo, off));
 }
 
 // Read L (0..W) bits at stream offset s from W-bit words (MSB-first); needs word s/W + 1.

@@ -174,50 +174,72 @@ struct PackArgs {
     int64_t buf_words;  // shared-memory words per output row
 };
 
-// A lane's tables for NC columns (32 * c + lane of a group of 32 * NC), and where each column's
-// bits start, and the group's end, when all of it is compressible.
+// A lane packs 64 bits of a row at a time, as two halves, high first: one 64-bit word, or two
+// neighbouring 32-bit words, each compressible or not on its own.  A chunk is 32 lanes of that
+// (32 or 64 columns), a group NC chunks.  The tables of a lane's halves in a group, where each
+// lane's bits start and where the group's end when all of it is compressible.
 template <typename U, int NC>
 struct PackTables {
-    static constexpr int H = sizeof(U) / 4;  // 32-bit halves, high first
-    uint32_t m[NC][H], bv[NC][H], mv[NC][H][kMoves];
-    uint32_t nb[NC], nbh[NC];  // kept bits of the word, of its high half
-    uint32_t before[NC], all, valid[NC];
-    int levels;  // moves the group's columns need (gather_left)
+    static constexpr bool PAIR = sizeof(U) == 4;
+    static constexpr int COLS = PAIR ? 64 : 32;      // columns of a chunk
+    static constexpr int UNITS = NC * (COLS / 32);   // bitmap units of a group
+    uint32_t m[NC][2], bv[NC][2], mv[NC][2][kMoves];
+    uint32_t nb[NC], nbh[NC];  // kept bits of both halves, of the first
+    uint32_t before[NC], all;
+    uint32_t valid;  // lane u < UNITS: the columns of bitmap unit u that exist
+    int left;        // columns from this lane's first in the group to the row's end
+    int levels;      // moves the group's columns need (gather_left)
 
-    __device__ __forceinline__ static void split(U x, uint32_t (&h)[H]) {
-        if constexpr (H == 2) {
-            h[0] = (uint32_t)(x >> 32);
-            h[1] = (uint32_t)x;
-        } else {
-            h[0] = x;
-        }
+    __device__ __forceinline__ static void split(U x, uint32_t (&h)[2]) {
+        h[0] = (uint32_t)((uint64_t)x >> 32);
+        h[1] = (uint32_t)x;
     }
 
-    __device__ __forceinline__ void load(const ColTables<U> &t, int64_t v, int64_t j0,
+    __device__ __forceinline__ void load(const ColTables<U> &t, int v, int j0,
                                          bool count_levels = false) {
         const int lane = threadIdx.x & 31;
         uint32_t moves[kMoves] = {};
+        const int of_unit = v - j0 - 32 * lane;
+        valid = lane >= UNITS || of_unit <= 0 ? 0u : (of_unit >= 32 ? ~0u : (1u << of_unit) - 1u);
+        left = v - j0 - (PAIR ? 2 : 1) * lane;
         all = 0;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const int64_t j = j0 + 32 * c + lane;
-            const bool in = j < v;  // a column past the end: no bits, always compressible
-            valid[c] = __ballot_sync(0xffffffffu, in);
-            split(in ? __ldg(&t.mask[j]) : (U)0, m[c]);
-            split(in ? __ldg(&t.bitval[j]) : (U)0, bv[c]);
-            const uint32_t k = in ? (uint32_t)__ldg(&t.nb[j]) : 0u;
-            nb[c] = k & 0xffu;
-            nbh[c] = nb[c] - (k >> 8);
+            // a column past the end: no bits, always compressible
+            if constexpr (PAIR) {
+                uint32_t k[2];
 #pragma unroll
-            for (int i = 0; i < kMoves; ++i) {
-                uint32_t h[H];
-                split(in ? __ldg(&t.mv[i * v + j]) : (U)0, h);
+                for (int h = 0; h < 2; ++h) {
+                    const int64_t j = j0 + COLS * c + 2 * lane + h;
+                    const bool in = j < v;
+                    m[c][h] = in ? __ldg(&t.mask[j]) : 0u;
+                    bv[c][h] = in ? __ldg(&t.bitval[j]) : 0u;
+                    k[h] = in ? (uint32_t)__ldg(&t.nb[j]) : 0u;
 #pragma unroll
-                for (int x = 0; x < H; ++x) {
-                    mv[c][x][i] = h[x];
-                    moves[i] |= h[x];
+                    for (int i = 0; i < kMoves; ++i)
+                        mv[c][h][i] = in ? __ldg(&t.mv[i * (int64_t)v + j]) : 0u;
+                    if (!in) m[c][h] = bv[c][h] = 0;
+                }
+                nbh[c] = k[0];
+                nb[c] = k[0] + k[1];
+            } else {
+                const int64_t j = j0 + COLS * c + lane;
+                const bool in = j < v;
+                split(in ? __ldg(&t.mask[j]) : (U)0, m[c]);
+                split(in ? __ldg(&t.bitval[j]) : (U)0, bv[c]);
+                const uint32_t k = in ? (uint32_t)__ldg(&t.nb[j]) : 0u;
+                nb[c] = k & 0xffu;
+                nbh[c] = nb[c] - (k >> 8);
+#pragma unroll
+                for (int i = 0; i < kMoves; ++i) {
+                    uint32_t h[2];
+                    split(in ? __ldg(&t.mv[i * (int64_t)v + j]) : (U)0, h);
+                    mv[c][0][i] = h[0];
+                    mv[c][1][i] = h[1];
                 }
             }
+#pragma unroll
+            for (int i = 0; i < kMoves; ++i) moves[i] |= mv[c][0][i] | mv[c][1][i];
             uint32_t incl = nb[c];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -233,6 +255,27 @@ struct PackTables {
 #pragma unroll
             for (int i = 0; i < kMoves; ++i)
                 if (__any_sync(0xffffffffu, moves[i] != 0)) levels = i + 1;
+        }
+    }
+
+    // this lane's halves of chunk c of a row (p: the row's word at the lane's first column of the
+    // group; wide: pairs of words are 8-byte aligned)
+    __device__ __forceinline__ void read(const U *p, int c, int left_, bool wide,
+                                         uint32_t (&x)[2]) const {
+        x[0] = x[1] = 0;
+        if constexpr (PAIR) {
+            if (wide) {
+                if (COLS * c < left_) {
+                    const uint2 y = *reinterpret_cast<const uint2 *>(p + COLS * c);
+                    x[0] = y.x;
+                    x[1] = y.y;
+                }
+            } else {
+                if (COLS * c < left_) x[0] = p[COLS * c];
+                if (COLS * c + 1 < left_) x[1] = p[COLS * c + 1];
+            }
+        } else {
+            if (COLS * c < left_) split(p[COLS * c], x);
         }
     }
 };
@@ -269,12 +312,14 @@ __device__ __forceinline__ void write_image(U *__restrict__ dst, uint32_t *image
 // shared-memory image at the word's bit offset, the row's length falls out of the last offset,
 // and only then is it known whether the row is stored compressed; the image is written (or, for
 // a row that stays raw, dropped) and zeroed for the next.  Offsets come from the tables where
-// a group is all compressible, else from a prefix sum.  Rows of up to 32 * NC words keep their
+// a group is all compressible, else from a prefix sum.  Rows of up to one group keep their
 // tables in registers (ONE); longer ones load them per group of columns, for Q rows at once.
 // The words of the next step are loaded while this one is packed.  LEVELS: moves per gather.
 template <typename U, int NC, int Q, bool ONE, bool INDEX, int LEVELS>
 __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC> &t) {
+    using T = PackTables<U, NC>;
     constexpr int W = 8 * sizeof(U), H = sizeof(U) / 4;
+    constexpr int GCOLS = T::COLS * NC, STEP = T::PAIR ? 2 : 1;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     uint32_t *images = reinterpret_cast<uint32_t *>(smem) +
@@ -286,7 +331,8 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t batches = (a.nrows + Q - 1) / Q;
-    const int groups = ONE ? 1 : (v + 32 * NC - 1) / (32 * NC);
+    const int groups = ONE ? 1 : (v + GCOLS - 1) / GCOLS;
+    const bool wide = T::PAIR && v % 2 == 0 && (((uintptr_t)a.src) & 7) == 0;
     for (int k = lane; k < Q * image_units; k += 32) images[k] = 0;
     __syncwarp();
     // source row of position batch * Q + q (-1: none)
@@ -297,14 +343,14 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
         const int64_t r = a.idx[i];
         return r >= 0 && r < a.n ? r : -1;
     };
-    auto load = [&](int64_t batch, int g, U (&x)[Q][NC]) {
-        const int j = g * 32 * NC + lane;
+    auto load = [&](int64_t batch, int g, uint32_t (&x)[Q][NC][2]) {
+        const int j = g * GCOLS + STEP * lane;
         if (!INDEX && (batch + 1) * Q <= a.nrows) {  // Q rows one after the other
             const U *p = a.src + batch * Q * v + j;
 #pragma unroll
             for (int q = 0; q < Q; ++q, p += v)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) x[q][c] = j + 32 * c < v ? p[32 * c] : (U)0;
+                for (int c = 0; c < NC; ++c) t.read(p, c, v - j, wide, x[q][c]);
             return;
         }
 #pragma unroll
@@ -312,60 +358,74 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
             const int64_t r = source(batch, q);
             const U *p = a.src + (r < 0 ? 0 : r) * v + j;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) x[q][c] = r >= 0 && j + 32 * c < v ? p[32 * c] : (U)0;
+            for (int c = 0; c < NC; ++c) t.read(p, c, r < 0 ? 0 : v - j, wide, x[q][c]);
         }
     };
     // fixed-stride rows of whole 16-byte blocks, at most one per lane
     const int n16 = v * (int)sizeof(U) / 16;
     const bool blocks = ONE && a.out && n16 <= 32 && v * (int)sizeof(U) % 16 == 0 &&
                         (((uintptr_t)a.out) & 15) == 0;
-    U x[Q][NC];
+    uint32_t x[Q][NC][2];
     if (warp < batches) load(warp, 0, x);
     for (int64_t batch = warp; batch < batches; batch += nwarps) {
         uint32_t at[Q];  // stream bits so far
 #pragma unroll
         for (int q = 0; q < Q; ++q) at[q] = stream0;
         for (int g = 0; g < groups; ++g) {
-            U y[Q][NC];
+            uint32_t y[Q][NC][2];
             const bool more = g + 1 < groups;
             if (more || batch + nwarps < batches)
                 load(more ? batch : batch + nwarps, more ? g + 1 : 0, y);
-            if (!ONE) t.load(a.t, v, (int64_t)g * 32 * NC);
+            if (!ONE) t.load(a.t, v, g * GCOLS);
+            const int chunks = ONE ? NC : min(NC, (v - g * GCOLS + T::COLS - 1) / T::COLS);
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                uint32_t hi[NC], lo[NC], off[NC], bal[NC];
-                bool cj[NC];
-                uint32_t every = 0xffffffffu;
+                uint32_t p0[NC], p1[NC], off[NC];  // the halves' bits, gathered left
+                bool c0[NC], c1[NC];               // the halves compress (64-bit words: together)
+                bool every = true;
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    if (!ONE && t.valid[c] == 0) {  // a chunk past the row's end
-                        cj[c] = true;
-                        hi[c] = lo[c] = off[c] = bal[c] = 0;
+                    if (!ONE && c >= chunks) {  // past the row's end
+                        c0[c] = c1[c] = true;
+                        p0[c] = p1[c] = 0;
+                        off[c] = at[q];
                         continue;
                     }
-                    uint32_t h[H];
-                    PackTables<U, NC>::split(x[q][c], h);
-                    uint32_t e = (h[0] & t.m[c][0]) ^ t.bv[c][0];
-                    if (H == 2) e |= (h[H - 1] & t.m[c][H - 1]) ^ t.bv[c][H - 1];
-                    cj[c] = e == 0;
-                    bal[c] = __ballot_sync(0xffffffffu, cj[c]);
-                    every &= bal[c];
-                    hi[c] = gather_left<LEVELS>(h[0], t.m[c][0], t.mv[c][0]);
-                    lo[c] = 0;
-                    if (H == 2) {
-                        const uint32_t l =
-                            gather_left<LEVELS>(h[H - 1], t.m[c][H - 1], t.mv[c][H - 1]);
-                        hi[c] |= __funnelshift_rc(l, 0, t.nbh[c]);
-                        lo[c] = __funnelshift_rc(0, l, t.nbh[c]);
-                    }
+                    const uint32_t e0 = (x[q][c][0] & t.m[c][0]) ^ t.bv[c][0];
+                    const uint32_t e1 = (x[q][c][1] & t.m[c][1]) ^ t.bv[c][1];
+                    c0[c] = T::PAIR ? e0 == 0 : (e0 | e1) == 0;
+                    c1[c] = T::PAIR ? e1 == 0 : c0[c];
+                    every = every && (e0 | e1) == 0;
+                    p0[c] = gather_left<LEVELS>(x[q][c][0], t.m[c][0], t.mv[c][0]);
+                    p1[c] = gather_left<LEVELS>(x[q][c][1], t.m[c][1], t.mv[c][1]);
                     off[c] = at[q] + t.before[c];
                 }
-                if (every == 0xffffffffu) {
+                uint32_t bits = t.valid;  // lane u < UNITS: bitmap unit u of the group
+                uint32_t split[NC];       // bits of the first half
+#pragma unroll
+                for (int c = 0; c < NC; ++c) split[c] = t.nbh[c];
+                if (__all_sync(0xffffffffu, every)) {
                     at[q] += t.all;
                 } else {
+                    bits = 0;
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
-                        const uint32_t len = cj[c] ? t.nb[c] : (uint32_t)W;
+                        // bitmap units, LSB-first
+                        if constexpr (T::PAIR) {
+                            const uint32_t f = (uint32_t)c0[c] | (uint32_t)c1[c] << 1;
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const uint32_t z =
+                                    __shfl_sync(0xffffffffu, f, 16 * h + (lane >> 1));
+                                const uint32_t b = __ballot_sync(0xffffffffu, (z >> (lane & 1)) & 1);
+                                if (lane == 2 * c + h) bits = b;
+                            }
+                        } else {
+                            const uint32_t b = __ballot_sync(0xffffffffu, c0[c]);
+                            if (lane == c) bits = b;
+                        }
+                        split[c] = c0[c] ? t.nbh[c] : 32u;
+                        const uint32_t len = split[c] + (c1[c] ? t.nb[c] - t.nbh[c] : 32u);
                         uint32_t incl = len;
 #pragma unroll
                         for (int o = 1; o < 32; o <<= 1) {
@@ -374,28 +434,28 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                         }
                         off[c] = at[q] + incl - len;
                         at[q] += __shfl_sync(0xffffffffu, incl, 31);
-                        uint32_t h[H];
-                        PackTables<U, NC>::split(x[q][c], h);
-                        hi[c] = cj[c] ? hi[c] : h[0];
-                        if (H == 2) lo[c] = cj[c] ? lo[c] : h[H - 1];
+                        p0[c] = c0[c] ? p0[c] : x[q][c][0];
+                        p1[c] = c1[c] ? p1[c] : x[q][c][1];
                     }
+                    bits &= t.valid;
                 }
-                // the group's bitmap units, LSB-first, in memory order (units past the row's
-                // last are zero and belong to the stream, where an OR of nothing does no harm)
-                uint32_t mine = 0;
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (lane == c) mine = bal[c] & t.valid[c];
+                // bitmap units in memory order (units past the row's last are zero and belong to
+                // the stream, where an OR of nothing does no harm)
                 const uint32_t image = images_at + q * image_units * 4;
-                or_shared(image + (uint32_t)((g * NC + (lane & (NC - 1))) ^ (H - 1)) * 4, mine);
+                or_shared(image + (uint32_t)((g * T::UNITS + (lane & (T::UNITS - 1))) ^ (H - 1)) * 4,
+                          bits);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
-                    if (ONE || t.valid[c]) put_bits<U>(image, off[c], hi[c], lo[c]);
+                    if (ONE || c < chunks)
+                        put_bits(image, off[c], p0[c] | __funnelshift_rc(p1[c], 0, split[c]),
+                                 __funnelshift_rc(0, p1[c], split[c]));
             }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) x[q][c] = y[q][c];
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) x[q][c][h] = y[q][c][h];
         }
         __syncwarp();
         unsigned packed = 0;
@@ -448,14 +508,16 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
 // then HBM.  600k rows of 64 64-bit words: 459 us with tables read through L1 and the row staged
 // and packed in two passes; 317 with tables in registers; 207 with 32-bit indices and images in
 // stream order; 188 with the moves chosen once; 163 without a test per atomic (its branches cost
-// more than the atomics of zeros); 140 now with the 16-byte epilogue, 4.0 TB/s.  Rows whose
+// more than the atomics of zeros); 137 now with the 16-byte epilogue, 4.1 TB/s.  32-bit words
+// two to a lane rather than one (half the prefix sums, three atomics for two words instead of
+// four): 200k rows of 99 words 254 us at first, 110, 92 now; of 400 words 308, 164, 150.  Rows whose
 // tables stay in registers choose their moves once (LEVELS 2 covers masks that drop at most
 // three bits above any kept one, as quantised floats do).
 template <typename U, int NC, int Q, bool ONE, bool INDEX>
 __global__ void __launch_bounds__(256, 2) pack_rows_kernel(PackArgs<U> a) {
     PackTables<U, NC> t;
     if (ONE) {
-        t.load(a.t, a.v, 0, true);
+        t.load(a.t, (int)a.v, 0, true);
         if (t.levels <= 2) {
             pack_rows<U, NC, Q, ONE, INDEX, 2>(a, t);
             return;
@@ -493,15 +555,14 @@ static ibp_status launch_pack(PackArgs<U> a, cudaStream_t st) {
         (size_t)(a.v + meta_bytes(a.v, sizeof(U)) / (int64_t)sizeof(U)) + 16 / sizeof(U),
         16 / sizeof(U));
     const size_t row = (size_t)a.buf_words * sizeof(U);
-    constexpr int NC = 16 / sizeof(U);  // 64 64-bit words or 128 32-bit words: 512 bytes
-    if (a.v <= 32) return launch_pack_q<U, 1, 4, true>(a, 8, 4 * 8 * row, st);
-    if (a.v <= 64) return launch_pack_q<U, 2, 4, true>(a, 8, 4 * 8 * row, st);
-    if (a.v <= 32 * NC) return launch_pack_q<U, NC, 4, true>(a, 8, 4 * 8 * row, st);
+    constexpr int cols = PackTables<U, 1>::COLS;
+    if (a.v <= cols) return launch_pack_q<U, 1, 4, true>(a, 8, 4 * 8 * row, st);
+    if (a.v <= 2 * cols) return launch_pack_q<U, 2, 4, true>(a, 8, 4 * 8 * row, st);
     // longer rows: 4 rows share a load of the tables while two blocks of 8 warps fit an SM,
     // else 1 row and as many warps as fit
-    if (4 * 8 * row <= 100 * 1024) return launch_pack_q<U, NC, 4, false>(a, 8, 4 * 8 * row, st);
+    if (4 * 8 * row <= 100 * 1024) return launch_pack_q<U, 2, 4, false>(a, 8, 4 * 8 * row, st);
     const int warps = (int)std::min<size_t>(8, (size_t)maxs / row);
-    return launch_pack_q<U, NC, 1, false>(a, warps, (size_t)warps * row, st);
+    return launch_pack_q<U, 2, 1, false>(a, warps, (size_t)warps * row, st);
 }
 
 template <typename U>
