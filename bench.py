@@ -663,10 +663,10 @@ def run_device_graph(args):
     bdev = [torch.from_numpy(bt).cuda() for bt in batches]
     uniq = [np.unique(bt) for bt in batches]
     # per batch, outside the timed region: compressed bytes of its distinct rows, and the
-    # algorithmic bytes of the whole call / of the fetch kernel alone
+    # algorithmic bytes of the call (the fetch kernel reads and writes all of them: repeats are
+    # decoded again, not copied by another kernel)
     comp_b = [int(sizes_np[u].sum()) for u in uniq]
     call_b = [comp_b[j] + len(batches[j]) * V * 8 for j in range(len(batches))]
-    kern_b = [comp_b[j] + len(uniq[j]) * V * 8 for j in range(len(batches))]
     nmax = max(len(bt) for bt in batches)
     out = torch.empty((nmax, V), dtype=torch.int64, device="cuda")
     wsb = lib.ibp_decompress_fetch_workspace_size(nmax, V, 8, 1)
@@ -704,7 +704,7 @@ def run_device_graph(args):
             j = step(k)
             rows += len(batches[j])
             call_bytes += call_b[j]
-            kern_bytes += kern_b[j]
+            kern_bytes += call_b[j]
         e1.record()
         e1.synchronize()
     launches = lib.ibp_kernel_launch_count() - n0
@@ -747,8 +747,8 @@ def run_device_graph(args):
         "fetch_kernel": {"achieved": round(kern_gbs, 1), "frac": round(kern_gbs / hbm_peak, 4),
                          "unit": "GB/s",
                          "ms_per_launch": round(kms / max(got, 1), 4),
-                         "what": "row-fetch kernel alone: compressed bytes read + decoded "
-                                 "bytes written of the distinct rows / its CUDA-event time"},
+                         "what": "row-fetch kernel alone: compressed bytes of the distinct rows "
+                                 "read + every output row written / its CUDA-event time"},
         "reference_gpu": ref,
         "clocks": clk.summary(),
         "gpu_launches": int(launches),
@@ -1722,7 +1722,7 @@ def main():
     for r in range(4):
         engine_step(k400, xd)
     dms = kernel_ms(4)
-    # the whole call (claim pass, fetch, repeat copies) on the same batch
+    # the whole call (prep and fetch) on the same batch
     torch.cuda.synchronize()
     w0, w1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     w0.record()
@@ -1732,21 +1732,21 @@ def main():
     w1.synchronize()
     call_ms = w0.elapsed_time(w1) / 10
     nuniq = len(np.unique(batches[k400]))
-    hbm_bytes = uniq_bytes[k400] + nuniq * V * 8
-    hbm_gbs = hbm_bytes / (sum(dms) / len(dms)) / 1e6
     call_bytes = uniq_bytes[k400] + len(batches[k400]) * V * 8
+    hbm_gbs = call_bytes / (sum(dms) / len(dms)) / 1e6
     hbm = {"bound": "hbm", "achieved": round(hbm_gbs, 1), "peak": hbm_peak, "unit": "GB/s",
            "frac": round(hbm_gbs / hbm_peak, 4), "traffic": None,
            "what": f"row-fetch kernel, device-resident copy of the set, 400k-row batch: "
-                   f"compressed bytes read + decoded bytes written of {nuniq} distinct rows",
+                   f"compressed bytes of {nuniq} distinct rows read + all 400k output rows "
+                   "written",
            "kernel_ms_per_launch": round(sum(dms) / len(dms), 4),
            "peak_source": hbm_src,
            "whole_call": {"ms": round(call_ms, 4),
                           "achieved": round(call_bytes / call_ms / 1e6, 1),
                           "frac": round(call_bytes / call_ms / 1e6 / hbm_peak, 4),
-                          "what": "the whole device-resident call (claim pass, fetch, repeat "
-                                  "copies): compressed bytes of the distinct rows read + all "
-                                  "400k output rows written, per call"}}
+                          "what": "the whole device-resident call (prep, fetch): compressed "
+                                  "bytes of the distinct rows read + all 400k output rows "
+                                  "written, per call"}}
     del xd
 
     line = None
