@@ -168,7 +168,8 @@ masks_from_counts_kernel(const uint32_t *__restrict__ counts, int64_t n, int64_t
 // PACK: S_t of a row fits 16 bits, two thresholds to a register in the sums over lanes.
 // Bound: the integer pipe, 3 operations per word and threshold there and one on the
 // multiply-add pipe (600k rows of 64 64-bit words, 7 thresholds: 550 us with 14 table loads per
-// word, 119 with the adds on the integer pipe as well, 100 now, 3.1 TB/s).
+// word, 119 with the adds on the integer pipe as well, 100 now; rows of up to 512 bytes take
+// check_sweep_kernel).
 template <typename U, int A, int G, int T, bool PACK>
 __global__ void __launch_bounds__(256, 2)
 check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
@@ -293,6 +294,162 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
     }
     __syncthreads();
     if (threadIdx.x < nthr && blk[threadIdx.x]) atomicAdd(&saved[threadIdx.x], blk[threadIdx.x]);
+}
+
+// The sweep over rows of at most 512 bytes in whole 16-byte pieces (32- and 64-bit words): the
+// masks being nested, a bit has a level, the number of masks it is in, and a word matches the
+// thresholds from the highest level among its mismatching bits on.  Levels are three bit planes,
+// so that highest level is found by three tests from the top (the mismatches with the plane's
+// bit, if there are any, are the ones that go on), and the word's set bits for each threshold
+// from there on, packed into 16 bytes, come out of a shared table: about 18 integer operations
+// a 64-bit word where seven compares take 31, and a third of the table registers.
+// 600k rows of 64 64-bit words: check_saved_kernel 100 us, this 82 (88 with
+// generic addresses for the table).
+template <typename U, int G>
+__global__ void __launch_bounds__(256, 2)
+check_sweep_kernel(const U *__restrict__ data, int64_t n, int v, int nthr,
+                   const U *__restrict__ masks, const U *__restrict__ bitvals,
+                   unsigned long long *__restrict__ saved, uint32_t one) {
+    using C = Chunk<U, 16, G>;
+    constexpr int WPP = 16 / sizeof(U), H = sizeof(U) / 4;  // words of a piece, registers of a word
+    constexpr int RPW = 32 / G, Q = 4, S = 4, L = Q * S > G ? Q * S / G : 1;
+    extern __shared__ __align__(16) uint4 bits_from[];  // [level][word of piece][piece]
+    __shared__ unsigned long long blk[kMaxThresholds];
+    if (threadIdx.x < kMaxThresholds) blk[threadIdx.x] = 0;
+    grid_dep_wait();
+    grid_dep_release();
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), gin = lane / G;
+    const int pieces = v / WPP;
+    const int stride = (v + 7) & ~7;  // whole rows of banks, so that levels do not meet
+    for (int e = threadIdx.x; e < 8 * v; e += blockDim.x) {
+        const int from = e / v, w = e % v;
+        uint32_t pc[8] = {};
+        for (int t = from; t < nthr; ++t) pc[t] = popc_w(masks[(int64_t)t * v + w]);
+        bits_from[from * stride + (w % WPP) * pieces + w / WPP] =
+            make_uint4(pc[0] | pc[1] << 16, pc[2] | pc[3] << 16, pc[4] | pc[5] << 16, pc[6]);
+    }
+    uint32_t b[4] = {}, p0[4] = {}, p1[4] = {}, p2[4] = {};
+    if (sub < pieces) {
+        C::load_words(bitvals, sub, pieces, b);
+        uint32_t m[7][4];
+#pragma unroll
+        for (int t = 0; t < 7; ++t) {
+            if (t < nthr) {
+                C::load_words(masks + (int64_t)t * v, sub, pieces, m[t]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) m[t][i] = 0;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // masks a bit is in, as a three-bit number
+            uint32_t s0, s1, c0, c1, c2;
+            carry_save(c0, s0, m[0][i], m[1][i], m[2][i]);
+            carry_save(c1, s1, m[3][i], m[4][i], m[5][i]);
+            carry_save(c2, p0[i], s0, s1, m[6][i]);
+            carry_save(p2[i], p1[i], c0, c1, c2);
+        }
+    }
+    __syncthreads();
+    const int64_t row_bytes = (int64_t)v * (int)sizeof(U);
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t batches = (n + RPW * Q - 1) / (RPW * Q);
+    auto load = [&](int64_t batch, uint32_t (&x)[Q][4]) {
+        const int64_t r0 = batch * (RPW * Q) + gin;
+        const char *p = reinterpret_cast<const char *>(data) + r0 * row_bytes;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            C::load(p + q * RPW * row_bytes, sub, r0 + q * RPW < n ? pieces : 0, x[q]);
+    };
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(bits_from) + sub * 16, step = stride * 16;
+    unsigned long long acc[L][2] = {};
+    uint32_t x[Q][4];
+    // from the last rows to the first, as in check_saved_kernel
+    int64_t batch = batches - 1 - warp;
+    if (batch >= 0) load(batch, x);
+    for (; batch >= 0; batch -= nwarps) {
+        uint32_t y[Q][4], f[Q * S] = {};
+        if (batch >= nwarps) load(batch - nwarps, y);
+        const int64_t left = n - (batch * (RPW * Q) + gin);
+        if (sub < pieces) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                if (q * RPW >= left) continue;
+#pragma unroll
+                for (int w = 0; w < WPP; ++w) {
+                    uint32_t e[H];
+                    uint32_t top = 0, mid = 0, low = 0;
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        e[h] = x[q][w * H + h] ^ b[w * H + h];
+                        top |= e[h] & p2[w * H + h];
+                    }
+                    if (top) {
+#pragma unroll
+                        for (int h = 0; h < H; ++h) e[h] &= p2[w * H + h];
+                    }
+#pragma unroll
+                    for (int h = 0; h < H; ++h) mid |= e[h] & p1[w * H + h];
+                    if (mid) {
+#pragma unroll
+                        for (int h = 0; h < H; ++h) e[h] &= p1[w * H + h];
+                    }
+#pragma unroll
+                    for (int h = 0; h < H; ++h) low |= e[h] & p0[w * H + h];
+                    uint32_t from = at + w * pieces * 16, z[4];
+                    if (top) from += 4 * step;
+                    if (mid) from += 2 * step;
+                    if (low) from += step;
+                    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                        : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3])
+                        : "r"(from));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) f[q * S + i] = z[i] * one + f[q * S + i];
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[q][i] = y[q][i];
+        group_sums<Q * S, G>(f, one);
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const uint32_t lo = f[l] & 0xffffu, hi = f[l] >> 16;
+            if (lo > (uint32_t)v) acc[l][0] += lo - (uint32_t)v;
+            if (hi > (uint32_t)v) acc[l][1] += hi - (uint32_t)v;
+        }
+    }
+    if ((sub & (group_sums_copies<Q * S, G>() - 1)) == 0) {
+        const int first = group_sums_value<Q * S, G>(sub);
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const int t = 2 * ((first + l) % S);
+            if (acc[l][0]) atomicAdd(&blk[t], acc[l][0]);
+            if (acc[l][1]) atomicAdd(&blk[t + 1], acc[l][1]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < nthr && blk[threadIdx.x]) atomicAdd(&saved[threadIdx.x], blk[threadIdx.x]);
+}
+
+template <typename U>
+static ibp_status launch_check_sweep(const U *data, int64_t n, int64_t v, int nthr, const U *masks,
+                                     const U *bitvals, unsigned long long *saved,
+                                     cudaStream_t st) {
+    const bool narrow = v * (int64_t)sizeof(U) <= 128;
+    auto kern = narrow ? check_sweep_kernel<U, 8> : check_sweep_kernel<U, 32>;
+    const size_t smem = sizeof(uint4) * 8 * (size_t)((v + 7) & ~(int64_t)7);
+    const int64_t per_block = 8 * 4 * (narrow ? 4 : 1);
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, 256, smem, &per_sm));
+    const int64_t blocks =
+        std::min<int64_t>((n + per_block - 1) / per_block, (int64_t)device_sm_count() * per_sm);
+    IBP_CUDA(launch_dependent(kern, (unsigned)blocks, 256, smem, st, data, n, (int)v, nthr, masks,
+                              bitvals, saved, 1u));
+    IBP_LAUNCHED("check_sweep_kernel");
+    return IBP_OK;
 }
 
 template <typename U, int A>
@@ -434,7 +591,15 @@ ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold,
         if (n > 0) {
             const U *rows = stage ? stage : data;
             const int a = row_piece_bytes(rows, v, wb);
-            if (a == 16)
+            // a sweep over rows that one warp covers with a 16-byte piece a lane
+            const bool sweep = wb >= 4 && a == 16 && thr.count > 1 && v * wb <= 512;
+            if constexpr (wb >= 4)
+                if (sweep)
+                    IBP_RET((launch_check_sweep<U>(rows, n, v, thr.count, masks, bitvals, saved,
+                                                   st)));
+            if (sweep) {
+                // done
+            } else if (a == 16)
                 IBP_RET((launch_check<U, 16>(rows, n, v, thr.count, masks, bitvals, saved, st)));
             else if (a == 4 && wb < 4)
                 IBP_RET((launch_check<U, wb < 4 ? 4 : 16>(rows, n, v, thr.count, masks, bitvals,
