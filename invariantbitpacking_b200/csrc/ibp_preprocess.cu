@@ -303,8 +303,8 @@ check_saved_kernel(const U *__restrict__ data, int64_t n, int64_t v, int nthr,
 // bit, if there are any, are the ones that go on), and the word's set bits for each threshold
 // from there on, packed into 16 bytes, come out of a shared table: about 18 integer operations
 // a 64-bit word where seven compares take 31, and a third of the table registers.
-// 600k rows of 64 64-bit words: check_saved_kernel 100 us, this 82 (88 with
-// generic addresses for the table).
+// 600k rows of 64 64-bit words: check_saved_kernel 100 us, this 82 (88 with generic addresses
+// for the table).
 template <typename U, int G>
 __global__ void __launch_bounds__(256, 2)
 check_sweep_kernel(const U *__restrict__ data, int64_t n, int v, int nthr,
@@ -455,11 +455,17 @@ static ibp_status launch_check_sweep(const U *data, int64_t n, int64_t v, int nt
 template <typename U, int A>
 static ibp_status launch_check(const U *data, int64_t n, int64_t v, int nthr, const U *masks,
                                const U *bitvals, unsigned long long *saved, cudaStream_t st) {
+    // a sweep over rows that one warp covers with a 16-byte piece a lane: 100 us there, 82 here
+    constexpr bool has_sweep = A == 16 && sizeof(U) >= 4;
+    static_assert(!has_sweep || 8 * A * Chunk<U, A, 8>::NS <= 512);
+    if constexpr (has_sweep)
+        if (nthr > 1 && v * (int64_t)sizeof(U) <= 512)
+            return launch_check_sweep<U>(data, n, v, nthr, masks, bitvals, saved, st);
     const bool narrow = v * (int64_t)sizeof(U) <= 8 * A * Chunk<U, A, 8>::NS;
     const bool pack = v * 8 * (int64_t)sizeof(U) < 65536;
     auto kern = nthr == 1 ? (narrow ? check_saved_kernel<U, A, 8, 1, false>
                                     : check_saved_kernel<U, A, 32, 1, false>)
-                          : (narrow ? check_saved_kernel<U, A, 8, 7, true>
+                          : (narrow ? check_saved_kernel<U, A, has_sweep ? 32 : 8, 7, true>
                                     : (pack ? check_saved_kernel<U, A, 32, 7, true>
                                             : check_saved_kernel<U, A, 32, 7, false>));
     const int64_t per_block = 8 * (nthr == 1 ? 8 : 4) * (narrow ? 4 : 1);
@@ -591,15 +597,7 @@ ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold,
         if (n > 0) {
             const U *rows = stage ? stage : data;
             const int a = row_piece_bytes(rows, v, wb);
-            // a sweep over rows that one warp covers with a 16-byte piece a lane
-            const bool sweep = wb >= 4 && a == 16 && thr.count > 1 && v * wb <= 512;
-            if constexpr (wb >= 4)
-                if (sweep)
-                    IBP_RET((launch_check_sweep<U>(rows, n, v, thr.count, masks, bitvals, saved,
-                                                   st)));
-            if (sweep) {
-                // done
-            } else if (a == 16)
+            if (a == 16)
                 IBP_RET((launch_check<U, 16>(rows, n, v, thr.count, masks, bitvals, saved, st)));
             else if (a == 4 && wb < 4)
                 IBP_RET((launch_check<U, wb < 4 ? 4 : 16>(rows, n, v, thr.count, masks, bitvals,

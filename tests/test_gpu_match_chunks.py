@@ -40,7 +40,8 @@ SHAPES = [(1, 1, 70), (1, 5, 1000), (1, 16, 333), (1, 33, 517), (1, 130, 200), (
           (2, 1, 40), (2, 3, 999), (2, 8, 64), (2, 64, 700), (2, 129, 333), (2, 130, 100),
           (4, 1, 35), (4, 4, 600), (4, 33, 1001), (4, 64, 2000), (4, 140, 65), (4, 2100, 40),
           (8, 1, 100), (8, 2, 500), (8, 16, 300), (8, 17, 301), (8, 64, 5000), (8, 65, 257),
-          (8, 1030, 50)]
+          (8, 1030, 50),
+          (4, 32, 900), (4, 36, 331), (4, 128, 700), (4, 132, 300), (8, 62, 401), (8, 66, 150)]
 
 
 @pytest.mark.parametrize("offset", [0, 1])
