@@ -88,8 +88,9 @@ assign_kernel(const U *__restrict__ data, int64_t n, int64_t v, const U *__restr
 // with byte values 2^(7 - s), so every common bit adds 128 to a 32-bit accumulator of
 // mma.m16n8k32 (u8 x u8, exact).  The order of K is free, so a lane takes 16 consecutive
 // bytes of a row and no operand is shuffled.  mma.sync rather than tcgen05: A exists only in
-// registers (expanding it into shared memory or TMEM would cost more than the product), and N
-// is the number of centroids.  Bound: issue (8 ANDs, 4 products and one 16-byte shared read
+// registers and N is the number of centroids: with the rows expanded into tensor memory and
+// kind::i8 products of 128 rows x 16 centroids the ten rounds of the table below took 504 us
+// a call, with these 451.  Bound: issue (8 ANDs, 4 products and one 16-byte shared read
 // per 32 rows x 8 bits of a lane's unit).
 __device__ __forceinline__ void mma_u8(int32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                        uint32_t b1) {
@@ -298,8 +299,8 @@ __device__ __forceinline__ void count_task(const uint32_t *__restrict__ data, in
 // only rows that changed cluster are listed, once to add and once to take away (a fifth of
 // the rows in the second round of a 16-cluster mixture, a fiftieth in the last).  The
 // reference issues an atomic per set bit, and this kernel's predecessors formed a ballot per
-// bit of every word (200k rows of 32 64-bit words, 16 clusters: 777 us a round; this kernel 38 us, 12 of them the
-// products at the rate mma.sync reaches, 8 cycles each per scheduler).
+// bit of every word (200k rows of 32 64-bit words, 16 clusters: 777 us a round; this kernel
+// 38 us, 12 of them the products at the rate mma.sync reaches, 8 cycles each per scheduler).
 // Block: 16 warps, one block per SM, tiles of n / SMs rows, so that a cluster's rows of a
 // tile make a task long enough to pay for its flush.
 template <bool V16, int VEC>
