@@ -1125,9 +1125,11 @@ static ibp_status launch_prep(int32_t *status, const U *mask, const U *bitval, i
 // hbm_rows_kernel takes never do.  With repeats claimed and copied by two more kernels a
 // 400k-row Zipf(1.1) batch of 64 64-bit words took 74 us (three quarters of it repeats), a uniform
 // one 120; decoding every position 51 and 74, through L1 (through L2 124: one slice serves a hot
-// row's lines).  The other device rows decode 3-10 times slower: 30k positions of 65 64-bit words,
-// Zipf(1.1), 36.7 us claimed and 34.5 direct (uniform 49 and 35), 100k positions 48.9 and 68
-// (uniform 82 and 69); of 512 words 107 and 83 at 30k, 142 and 235 at 100k.
+// row's lines).  The other device rows decode 3-10 times slower.  Rows of at most 512 bytes (33
+// 64-bit words, claimed / direct): 65k positions Zipf(1.1) 34.8 / 35.5 us, uniform 55.2 / 37.3;
+// 100k 39.8 / 50.6 and 72.5 / 51.7; 33, 99 and 128 32-bit words alike.  Longer rows (512 words):
+// 30k positions 107 / 83 us, 100k 142 / 235.
+constexpr int64_t kDirectShortRows = 65536;
 constexpr int64_t kDirectRows = 32768;
 
 template <typename U>
@@ -1191,7 +1193,8 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
         return IBP_ERR_UNSUPPORTED;
     }
     const int mode = fetch_dedup_mode();
-    if (mode == 0 && (hbm_rows_fit(a) || (device_fetch_fit(a) && nidx <= kDirectRows))) {
+    const int64_t direct = v * wb <= 512 ? kDirectShortRows : kDirectRows;
+    if (mode == 0 && (hbm_rows_fit(a) || (device_fetch_fit(a) && nidx <= direct))) {
         // device rows that decode as fast as their repeats would be found and copied: every
         // position decodes its row, in one kernel
         IBP_RET(launch_prep<U>(status, mask, bitval, v, t, tables, nullptr, 0, st));
