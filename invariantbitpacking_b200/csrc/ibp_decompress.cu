@@ -705,6 +705,10 @@ static ibp_status launch_hbm_nc(FetchArgs<U> a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ other HBM rows
+// Words of a row whose bitmap one lane looks through: 100k rows of 256 32-bit words 80 -> 74 us
+// (sets with few full rows 113 -> 111), no difference left at 512.
+constexpr int kLaneBitmap = 256;
+
 // Rows in device memory of any length and alignment, fixed-stride or condensed (EXACT): a warp
 // takes up to `slots` rows (the claim pass's head records, sorted positions, or rows p, p + 1,
 // ... of an unindexed fetch) at a time, lane q holding row q's metadata.  Their 16-byte
@@ -717,7 +721,9 @@ static ibp_status launch_hbm_nc(FetchArgs<U> a, cudaStream_t st) {
 // Bound: issue and the integer pipe (a 32-bit half takes five masked moves).  Whole sets: 100k
 // rows of 256 32-bit words at half the bits 174 -> 83 us, 40k rows of 512 64-bit words at a
 // quarter 254 -> 91 us; 50k condensed rows of 99 32-bit words 87 -> 45 us (a row at a time
-// before, with eight table loads a word).
+// before, with eight table loads a word).  What a short row costs beside its decode is shared
+// too: lane q looks through row q's bitmap (a warp's sum per row before: 200k rows of 33 64-bit
+// words 93 us, so 72), and rows of few blocks are copied two or four at a time (61).
 template <typename U, bool ONE, bool EXACT>
 __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -797,14 +803,16 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         }
         return b;
     };
-    // the 16-byte blocks of [from, to) into the slot whose first block is that of `lo`
+    // the 16-byte blocks of [from, to) into the slot whose first block is that of `lo`, by `of`
+    // lanes of which this is the one numbered `sub`
     const uintptr_t comp = (uintptr_t)a.s.comp;
-    auto copy_blocks = [&](U *slot, uintptr_t lo, uintptr_t from, uintptr_t to) {
+    auto copy_blocks = [&](U *slot, uintptr_t lo, uintptr_t from, uintptr_t to, int sub, int of) {
         const uintptr_t b0 = from & ~(uintptr_t)15;
         const int n = (int)((to + 15 - b0) >> 4);
-        const char *src = reinterpret_cast<const char *>(b0) + lane * 16;
-        char *dst = reinterpret_cast<char *>(slot) + (b0 - (lo & ~(uintptr_t)15)) + lane * 16;
-        for (int i = lane; i < n; i += 32, src += 512, dst += 512) cp_async16<true>(dst, src);
+        const char *src = reinterpret_cast<const char *>(b0) + sub * 16;
+        char *dst = reinterpret_cast<char *>(slot) + (b0 - (lo & ~(uintptr_t)15)) + sub * 16;
+        for (int i = sub; i < n; i += of, src += of * 16, dst += of * 16)
+            cp_async16<true>(dst, src);
     };
 
     int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -820,12 +828,19 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         unsigned pm = __ballot_sync(0xffffffffu, cur.ok && cur.packed);
         const unsigned rm = __ballot_sync(0xffffffffu, cur.ok && !cur.packed && fits);
         unsigned wide = __ballot_sync(0xffffffffu, cur.ok && !cur.packed && !fits);
+        // rows of up to 8 or 16 blocks four or two at a time
+        const bool mine = ((pm | rm) >> lane) & 1u;
+        const int most = (int)__reduce_max_sync(
+            0xffffffffu,
+            mine ? (unsigned)((lo & 15) + len * (int64_t)sizeof(U) + 15) >> 4 : 0u);
+        const int of = most <= 8 ? 8 : (most <= 16 ? 16 : 32), sub = lane & (of - 1);
 #pragma unroll 1
-        for (unsigned m = pm | rm; m; m &= m - 1) {
-            const int q = __ffs(m) - 1;
+        for (int q0 = 0; q0 < per; q0 += 32 / of) {
+            const int q = q0 + lane / of;
             const uintptr_t l = __shfl_sync(0xffffffffu, (unsigned long long)lo, q);
-            const int64_t n = __shfl_sync(0xffffffffu, len, q);
-            copy_blocks(slots + q * sw, l, l, l + n * (int64_t)sizeof(U));
+            const int n = __shfl_sync(0xffffffffu, (int)len, q);
+            if (((pm | rm) >> q) & 1u)
+                copy_blocks(slots + q * sw, l, l, l + n * (int64_t)sizeof(U), sub, of);
         }
         cp_async_commit();
         cur = next;
@@ -841,10 +856,22 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         cp_async_wait_all();
         __syncwarp();
         // lengths
-        int64_t end = 0;
+        int64_t end = mw + (int64_t)((packed_bits + W - 1) / W);
         unsigned fm = 0;  // rows whose words are all compressible
+        if (v <= kLaneBitmap) {
+            // each lane looks at its row's bitmap; only rows that are not full take the warp's sum
+            bool full = (pm >> lane) & 1u;
+            if (full) {
+                const uint32_t *bitmap = reinterpret_cast<const uint32_t *>(slots + place);
+                for (int j = 0; full && j < (int)v; j += 32) {
+                    const uint32_t absent = v - j < 32 ? ~0u << (v - j) : 0u;
+                    full = (bitmap[j >> 5] | absent) == ~0u;
+                }
+            }
+            fm = __ballot_sync(0xffffffffu, full);
+        }
 #pragma unroll 1
-        for (unsigned m = pm; m; m &= m - 1) {
+        for (unsigned m = pm & ~fm; m; m &= m - 1) {
             const int q = __ffs(m) - 1;
             bool full;
             const uint32_t bits = row_stream_bits<U>(slots + __shfl_sync(0xffffffffu, place, q), v,
@@ -870,7 +897,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
                     const int64_t n = __shfl_sync(0xffffffffu, len, q);
                     const int64_t e = __shfl_sync(0xffffffffu, end, q);
                     copy_blocks(slots + q * sw, l, l + n * (int64_t)sizeof(U),
-                                l + e * (int64_t)sizeof(U));
+                                l + e * (int64_t)sizeof(U), lane, 32);
                 }
                 cp_async_commit();
                 cp_async_wait_all();
