@@ -746,8 +746,10 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     }
     const int64_t nrows = a.list ? (int64_t)*a.list_len : a.nrows;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    // rows at a time: fewer when the fetch does not fill every warp's slots
-    const int per = (int)max((int64_t)1, min((int64_t)a.slots, nrows / nwarps));
+    // rows at a time: as many as make the fewest rounds, equal ones (80k positions of 33 64-bit
+    // words: 35.2 us as two rounds of 16 rows and a short third, 31.1 as three of 12)
+    const int64_t rounds = max((int64_t)1, (nrows + nwarps * a.slots - 1) / (nwarps * a.slots));
+    const int per = (int)max((int64_t)1, (nrows + nwarps * rounds - 1) / (nwarps * rounds));
     const int64_t units = (nrows + per - 1) / per;
 
     // this lane's row of unit u: position and row ...
@@ -1152,11 +1154,12 @@ static ibp_status launch_prep(int32_t *status, const U *mask, const U *bitval, i
 // hbm_rows_kernel takes never do.  With repeats claimed and copied by two more kernels a
 // 400k-row Zipf(1.1) batch of 64 64-bit words took 74 us (three quarters of it repeats), a uniform
 // one 120; decoding every position 51 and 74, through L1 (through L2 124: one slice serves a hot
-// row's lines).  The other device rows decode 3-10 times slower.  Rows of at most 512 bytes (33
-// 64-bit words, claimed / direct): 65k positions Zipf(1.1) 34.8 / 35.5 us, uniform 55.2 / 37.3;
-// 100k 39.8 / 50.6 and 72.5 / 51.7; 33, 99 and 128 32-bit words alike.  Longer rows (512 words):
-// 30k positions 107 / 83 us, 100k 142 / 235.
-constexpr int64_t kDirectShortRows = 65536;
+// row's lines).  The other device rows decode 2-10 times slower.  Rows of at most 512 bytes (33
+// 64-bit words, claimed / direct): 65k positions Zipf(1.1) 29.4 / 23.0 us, uniform 43.7 / 25.3;
+// 100k 32.2 / 33.2 and 56.5 / 35.2, 130k 33.9 / 39.4 and 61.7 / 45.2; 99 32-bit words alike.
+// Longer rows (512 words): 30k positions 107 / 82 and 101 / 88 us, 45k 111 / 113 and 134 / 120,
+// 65k 126 / 157 and 241 / 169.
+constexpr int64_t kDirectShortRows = 98304;
 constexpr int64_t kDirectRows = 32768;
 
 template <typename U>

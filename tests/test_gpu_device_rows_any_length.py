@@ -92,7 +92,7 @@ def test_bad_indices_are_reported_and_the_rest_is_right(wb, v):
         ibp.set_fetch_dedup("auto")
 
 
-@pytest.mark.parametrize("count", [32767, 32768, 32769, 65535, 65536, 65537])
+@pytest.mark.parametrize("count", [32767, 32768, 32769, 98303, 98304, 98305])
 @pytest.mark.parametrize("wb,v", [(8, 33), (8, 64), (4, 128), (4, 129), (4, 300)])
 def test_batches_around_the_direct_limit(wb, v, count):
     """Skewed batches on both sides of the size up to which repeats are decoded again, rows of the
