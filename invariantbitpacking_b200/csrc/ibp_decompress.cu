@@ -231,8 +231,15 @@ static ibp_status launch_fill_hashed(const int64_t *idx, int64_t nidx, int64_t n
     IBP_RET(kernel_blocks_per_sm((const void *)kern, kFillThreads, 0, &per_sm));
     const int64_t fb = std::min<int64_t>((nidx + kFillThreads - 1) / kFillThreads,
                                          (int64_t)device_sm_count() * per_sm);
-    IBP_CUDA(launch_dependent(kern, (unsigned)fb, kFillThreads, 0, st, idx, nidx, n, hkeys, hpos,
-                              slots, out, v));
+    // Launched while the fetch runs, the copies of rows longer than 512 bytes keep the fetch's
+    // division of each SM's storage and with it a small L1 for the hot rows: 30k Zipf(1.1)
+    // positions of 512 64-bit words 107 us a call, after the fetch 72 (uniform ones 102 and
+    // 107; shorter rows 31 and 33 us).
+    if (v * (int64_t)sizeof(U) <= 512)
+        IBP_CUDA(launch_dependent(kern, (unsigned)fb, kFillThreads, 0, st, idx, nidx, n, hkeys,
+                                  hpos, slots, out, v));
+    else
+        kern<<<(unsigned)fb, kFillThreads, 0, st>>>(idx, nidx, n, hkeys, hpos, slots, out, v);
     IBP_LAUNCHED("fill_hashed_kernel");
     return IBP_OK;
 }
@@ -1157,10 +1164,10 @@ static ibp_status launch_prep(int32_t *status, const U *mask, const U *bitval, i
 // row's lines).  The other device rows decode 2-10 times slower.  Rows of at most 512 bytes (33
 // 64-bit words, claimed / direct): 65k positions Zipf(1.1) 29.4 / 23.0 us, uniform 43.7 / 25.3;
 // 100k 32.2 / 33.2 and 56.5 / 35.2, 130k 33.9 / 39.4 and 61.7 / 45.2; 99 32-bit words alike.
-// Longer rows (512 words): 30k positions 107 / 82 and 101 / 88 us, 45k 111 / 113 and 134 / 120,
-// 65k 126 / 157 and 241 / 169.
+// Longer rows (129 64-bit words): 30k positions 39.4 / 33.2 and 51.2 / 31.2 us, 65k 46.1 / 57.8
+// and 76.9 / 56.8; of 512 words 30k 72 / 82 and 107 / 88, hence also a line in bytes.
 constexpr int64_t kDirectShortRows = 98304;
-constexpr int64_t kDirectRows = 32768;
+constexpr int64_t kDirectRows = 32768, kDirectBytes = 64 << 20;
 
 template <typename U>
 ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
@@ -1223,7 +1230,8 @@ ibp_status decompress_impl(const U *comp, int64_t n, int64_t v, const U *mask,
         return IBP_ERR_UNSUPPORTED;
     }
     const int mode = fetch_dedup_mode();
-    const int64_t direct = v * wb <= 512 ? kDirectShortRows : kDirectRows;
+    const int64_t direct =
+        v * wb <= 512 ? kDirectShortRows : std::min(kDirectRows, kDirectBytes / (v * wb));
     if (mode == 0 && (hbm_rows_fit(a) || (device_fetch_fit(a) && nidx <= direct))) {
         // device rows that decode as fast as their repeats would be found and copied: every
         // position decodes its row, in one kernel

@@ -112,6 +112,11 @@ def test_batches_around_the_direct_limit(wb, v, count):
     assert torch.equal(out, src[k])
 
 
+@pytest.mark.parametrize("count", [16384, 16385])
+def test_long_rows_around_the_direct_limit_in_bytes(count):
+    test_batches_around_the_direct_limit(8, 512, count)
+
+
 @pytest.mark.parametrize("low,high", [(0, 31), (1, 30), (3, 28), (4, 27), (31, 0), (16, 16)])
 @pytest.mark.parametrize("wb,v", [(8, 64), (8, 40), (4, 64), (4, 20)])
 def test_masks_that_need_few_moves_and_many(wb, v, low, high):
