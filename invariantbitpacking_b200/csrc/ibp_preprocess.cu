@@ -401,9 +401,12 @@ check_sweep_kernel(const U *__restrict__ data, int64_t n, int v, int nthr,
                     if (top) from += 4 * step;
                     if (mid) from += 2 * step;
                     if (low) from += step;
-                    asm("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                        : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3])
-                        : "r"(from));
+                    // volatile, and a memory clobber: the barrier after the table's stores is
+                    // all that orders them before this read
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(z[0]), "=r"(z[1]), "=r"(z[2]), "=r"(z[3])
+                                 : "r"(from)
+                                 : "memory");
 #pragma unroll
                     for (int i = 0; i < 4; ++i) f[q * S + i] = z[i] * one + f[q * S + i];
                 }
