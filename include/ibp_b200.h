@@ -178,9 +178,12 @@ ibp_status ibp_compress_condensed(const void *dataset, int64_t num_vecs, int64_t
  * length, a tuning hint only.  nblks / nthreads / impl follow the reference knobs:
  * impl -1 auto, 0/1/5 decompress (the engine picks its own kernel shape), 2 = plain
  * uncompressed gather of the stored rows (the reference's baseline); other values are
- * IBP_ERR_UNSUPPORTED.  nblks/nthreads <= 0 pick defaults.  word_bytes in {4,8}.
- * With an index, rows are fetched in sorted order and each distinct row is read once;
- * repeats are copied on the device. */
+ * IBP_ERR_UNSUPPORTED.  nblks/nthreads <= 0 pick defaults; values above what the kernel takes
+ * are cut to it, and the kernel for 16-byte aligned device rows of at most 64 words picks its own.
+ * word_bytes in {4,8}.
+ * With an index, each distinct row of a host set is read once and its repeats are copied on
+ * the device; repeats of device rows are decoded again or copied, whichever is faster
+ * (ibp_set_fetch_dedup). */
 size_t ibp_decompress_fetch_workspace_size(int64_t num_index, int64_t vec_size, int word_bytes,
                                            int has_index);
 ibp_status ibp_decompress_fetch(const void *comp, int64_t num_vecs, int64_t vec_size,

@@ -952,6 +952,12 @@ static int64_t device_slot_words(const RowSet<U> &s) {
     return (int64_t)align_up((size_t)words + 2 * per16 + 2, per16);
 }
 
+// Threads of a block for the caller's nthreads (whole warps, at most kFetchThreads).
+static int block_threads(int nthreads) {
+    if (nthreads <= 0) return kFetchThreads;
+    return std::min(std::max(nthreads / 32 * 32, 32), kFetchThreads);
+}
+
 // Every fetch of device rows but raw gathers and rows too long for one slot per block.
 template <typename U>
 static bool device_fetch_fit(const FetchArgs<U> &a) {
@@ -960,13 +966,14 @@ static bool device_fetch_fit(const FetchArgs<U> &a) {
 }
 
 template <typename U>
-static ibp_status launch_device_fetch(FetchArgs<U> a, cudaStream_t st) {
+static ibp_status launch_device_fetch(FetchArgs<U> a, int nblks, int nthreads, cudaStream_t st) {
     a.slot_words = device_slot_words<U>(a.s);
     const size_t slot = (size_t)a.slot_words * sizeof(U);
     // up to 16 rows share a load of the tables as long as two blocks of 8 warps fit an SM
     a.slots = 16;
     while (a.slots > 1 && 8 * a.slots * slot > 110 * 1024) a.slots /= 2;
-    const int warps = (int)std::min<size_t>(8, (size_t)device_max_smem_optin() / (a.slots * slot));
+    const int warps = (int)std::min<size_t>(block_threads(nthreads) / 32,
+                                            (size_t)device_max_smem_optin() / (a.slots * slot));
     const bool one = a.s.v * (int64_t)sizeof(U) <= 512;
     auto kern = a.s.offsets
                     ? (one ? device_fetch_kernel<U, true, true> : device_fetch_kernel<U, false, true>)
@@ -975,8 +982,8 @@ static ibp_status launch_device_fetch(FetchArgs<U> a, cudaStream_t st) {
     const size_t smem = slot * a.slots * warps;
     int per_sm = 0;
     IBP_RET(kernel_blocks_per_sm((const void *)kern, warps * 32, smem, &per_sm));
-    const int64_t blocks = std::min<int64_t>((a.nrows + warps - 1) / warps,
-                                             (int64_t)device_sm_count() * per_sm);
+    const int64_t blocks = std::min<int64_t>(
+        (a.nrows + warps - 1) / warps, nblks > 0 ? nblks : (int64_t)device_sm_count() * per_sm);
     const int pslot = profile_begin(st);
     IBP_CUDA(launch_dependent(kern, (unsigned)blocks, warps * 32, smem, st, a));
     IBP_LAUNCHED("device_fetch_kernel");
@@ -1052,8 +1059,7 @@ size_t decompress_workspace(int64_t nidx, int64_t v, int wb, bool has_index) {
 template <typename U, int NC, bool EXACT>
 static ibp_status launch_fetch_nc(FetchArgs<U> a, int nblks, int nthreads, cudaStream_t st) {
     const size_t slot_bytes = (size_t)a.slot_words * sizeof(U);
-    int threads = nthreads > 0 ? nthreads : kFetchThreads;
-    threads = threads < 32 ? 32 : (threads > kFetchThreads ? kFetchThreads : threads / 32 * 32);
+    int threads = block_threads(nthreads);
     const int maxs = device_max_smem_optin();
     // row slots per warp: up to kRowsInFlight within ~96 KB per block; long rows get fewer
     // slots and then fewer warps
@@ -1106,7 +1112,7 @@ static ibp_status launch_fetch(FetchArgs<U> a, int nblks, int nthreads, cudaStre
     constexpr int per16 = 16 / sizeof(U);
     if (hbm_rows_fit(a))
         return a.s.v > 32 ? launch_hbm_nc<U, 2>(a, st) : launch_hbm_nc<U, 1>(a, st);
-    if (device_fetch_fit(a)) return launch_device_fetch<U>(a, st);
+    if (device_fetch_fit(a)) return launch_device_fetch<U>(a, nblks, nthreads, st);
     if (a.s.offsets) {
         // a condensed row starts at any word: room for the blocks around it and the padding
         a.slot_words = (int64_t)align_up((size_t)a.s.v + 2 * per16 + 2, per16);
