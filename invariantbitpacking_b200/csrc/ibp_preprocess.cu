@@ -3,8 +3,9 @@
 // include/preproc/ibp_preproc_kernels.cuh:7-77).
 //
 // B200 design
-//  * census: rows are taken in 16-byte pieces whatever the word size (a group of up to 16 rows
-//    is a whole number of them), each thread counting the set bits of one piece's positions in
+//  * census: the dataset is taken in 16-byte pieces whatever the word size and wherever it starts
+//    (as many bytes as up to 16 rows have are a whole number of pieces, from the first 16-byte
+//    boundary on), each thread counting the set bits of one piece's positions in
 //    bit planes (ibp_bitcount.cuh), 8 pieces in flight; shared counters per block, one global
 //    atomic per (position, block) at the end.  A host-resident dataset is optionally staged
 //    into HBM during this pass so the second pass reads HBM instead of PCIe.
@@ -23,15 +24,16 @@ namespace ibp200 {
 constexpr int kCensusThreads = 256;
 constexpr int kCensusCols = 64;   // most 16-byte pieces a block covers side by side
 
-// counts[p] += rows whose bit p (word p / W, bit p % W) is set, over groups of k rows that
-// make up `pieces` 16-byte pieces each (bit p of a group is bit p % row_bits of a row).
+// counts[p] += rows whose bit p (word p / W, bit p % W) is set, over groups of as many bytes as k
+// rows have, `pieces` 16-byte pieces each.  `data` is the dataset's first 16-byte boundary, `turn`
+// bits from its start: bit p of a group is bit (turn + p) % row_bits of a row.
 // Block bx * tiles + tile covers pieces [tile * cpb, tile * cpb + cpb) of every group; the R =
 // kCensusThreads / cpb row slots of a tile's blocks take the groups in turn.
 // Bound: HBM (600k rows of 512 bytes: 126 -> 54 us, 5.7 TB/s; a thread per word, a
 // ripple-carry add into 8 planes and 64 KiB of counters per block before).
 __global__ void __launch_bounds__(kCensusThreads, 2)
 census_kernel(const uint4 *__restrict__ data, int64_t groups, int64_t pieces, int cpb, int tiles,
-              int64_t row_bits, bool folded, uint32_t *__restrict__ counts,
+              int64_t row_bits, int turn, bool folded, uint32_t *__restrict__ counts,
               uint4 *__restrict__ stage) {
     extern __shared__ uint32_t sc[];  // [128][cpb | 1]
     const int stride = cpb | 1;
@@ -86,38 +88,40 @@ census_kernel(const uint4 *__restrict__ data, int64_t groups, int64_t pieces, in
         const int64_t piece = col0 + cc;
         const uint32_t x = sc[b * stride + cc];
         if (piece < pieces && x) {
-            const int64_t p = piece * 128 + b;
+            const int64_t p = piece * 128 + b + turn;
             atomicAdd(&counts[folded ? p % row_bits : p], x);
         }
     }
 }
 
-// The rows the 16-byte pieces leave over (fewer than a group), or all of them when the dataset
-// does not start on a 16-byte boundary: a thread per word and 32 rows, an atomic per set bit.
+// The words the 16-byte pieces leave over, those before `head` and from `tail` to the dataset's
+// last: a thread per column, which sees at most 32 of them, an atomic per set bit.
 template <typename U>
 __global__ void __launch_bounds__(kCensusThreads)
-census_rest_kernel(const U *__restrict__ data, int64_t n, int64_t v, uint32_t *__restrict__ counts,
-                   U *__restrict__ stage) {
-    constexpr int W = WordBits<U>::value;
-    const int64_t total = (n + 31) / 32 * v;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t col = e % v, r0 = e / v * 32;
-        const int rows = (int)min((int64_t)32, n - r0);
-        BitPlanes<sizeof(U) == 8 ? 2 : 1> bp;
+census_rest_kernel(const U *__restrict__ data, int64_t words, int64_t v, int64_t head,
+                   int64_t tail, uint32_t *__restrict__ counts, U *__restrict__ stage) {
+    constexpr int W = WordBits<U>::value, R = sizeof(U) == 8 ? 2 : 1;
+    for (int64_t col = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; col < v;
+         col += (int64_t)gridDim.x * blockDim.x) {
+        BitPlanes<R> bp;
         bp.clear();
-        for (int r = 0; r < rows; r += 8) {
-            uint32_t x[8][sizeof(U) == 8 ? 2 : 1];
+        // words col, col + v, ... of each of the two ranges, eight at a time
+        auto count = [&](int64_t from, int64_t to) {
+            for (int64_t w = from; w < to; w += 8 * v) {
+                uint32_t x[8][R];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const bool in = r + q < rows;
-                const U y = in ? data[(r0 + r + q) * v + col] : (U)0;
-                if (in && stage) stage[(r0 + r + q) * v + col] = y;
-                x[q][0] = (uint32_t)y;
-                if constexpr (sizeof(U) == 8) x[q][1] = (uint32_t)(y >> 32);
+                for (int q = 0; q < 8; ++q) {
+                    const bool in = w + q * v < to;
+                    const U y = in ? data[w + q * v] : (U)0;
+                    if (in && stage) stage[w + q * v] = y;
+                    x[q][0] = (uint32_t)y;
+                    if constexpr (R == 2) x[q][1] = (uint32_t)((uint64_t)y >> 32);
+                }
+                bp.add8(x);
             }
-            bp.add8(x);
-        }
+        };
+        count(col, head);
+        count(tail + (col - tail % v + v) % v, words);
 #pragma unroll
         for (int b = 0; b < W; ++b) {
             const uint32_t x = (bp.bytes(b / 32, b % 8) >> (8 * (b % 32 / 8))) & 0xffu;
@@ -518,15 +522,21 @@ ThrList sweep_thresholds(float threshold) {
     return l;
 }
 
-// Counts of the whole dataset: groups of k rows as 16-byte pieces, then the rows left over.
+// Counts of the whole dataset: 16-byte pieces in groups of k rows' bytes, then the words left over
+// at its ends.  `stage` (or null) starts on a 16-byte boundary, and with it `data`.
 template <typename U>
 static ibp_status launch_census(const U *data, int64_t n, int64_t v, uint32_t *counts, U *stage,
                                 cudaStream_t st) {
     const int64_t row_bytes = v * (int64_t)sizeof(U);
     int64_t k = 1;
     while (k * row_bytes % 16) k *= 2;
-    const bool aligned = ((((uintptr_t)data) | ((uintptr_t)stage)) & 15) == 0;
-    const int64_t groups = aligned ? n / k : 0;
+    // Pieces from the first 16-byte boundary on, wherever the dataset starts: the bits of a group
+    // are then those of k rows turned by the words before it.  192 MiB of 64-bit words 8 bytes off
+    // a boundary take as long as on one (rows of 64 words 35 us, of one word 61); a thread per
+    // word and 32 rows with an atomic per set bit, for such data before, took 1098 and 30561 us.
+    const int64_t head = (int64_t)(-(uintptr_t)data & 15) / (int64_t)sizeof(U);
+    const int64_t groups = std::max<int64_t>(0, (n * v - head) / (k * v));
+    const int64_t tail = groups > 0 ? head + groups * k * v : 0;
     const int sms = device_sm_count();
     if (groups > 0) {
         const int64_t pieces = k * row_bytes / 16;
@@ -540,16 +550,17 @@ static ibp_status launch_census(const U *data, int64_t n, int64_t v, uint32_t *c
         const int64_t gx = std::max<int64_t>(
             1, std::min<int64_t>((groups + R * 32 - 1) / (R * 32), (int64_t)sms * per_sm / tiles));
         census_kernel<<<(unsigned)(gx * tiles), kCensusThreads, smem, st>>>(
-            reinterpret_cast<const uint4 *>(data), groups, pieces, cpb, (int)tiles, row_bytes * 8, k > 1, counts, reinterpret_cast<uint4 *>(stage));
+            reinterpret_cast<const uint4 *>(data + head), groups, pieces, cpb, (int)tiles,
+            row_bytes * 8, (int)(head * 8 * (int64_t)sizeof(U)), k > 1 || head > 0, counts,
+            reinterpret_cast<uint4 *>(stage));
         IBP_LAUNCHED("census_kernel");
     }
-    const int64_t done = groups * k;
-    if (done < n) {
-        const int64_t threads = (n - done + 31) / 32 * v;
-        const int64_t blocks = std::min<int64_t>((threads + kCensusThreads - 1) / kCensusThreads,
-                                                 (int64_t)sms * 8);
-        census_rest_kernel<U><<<(unsigned)blocks, kCensusThreads, 0, st>>>(
-            data + done * v, n - done, v, counts, stage ? stage + done * v : nullptr);
+    const int64_t first = groups > 0 ? head : 0;
+    if (first > 0 || tail < n * v) {
+        const int64_t blocks =
+            std::min<int64_t>((v + kCensusThreads - 1) / kCensusThreads, (int64_t)sms * 8);
+        census_rest_kernel<U><<<(unsigned)blocks, kCensusThreads, 0, st>>>(data, n * v, v, first,
+                                                                           tail, counts, stage);
         IBP_LAUNCHED("census_rest_kernel");
     }
     return IBP_OK;
@@ -588,6 +599,12 @@ ibp_status preprocess_impl(const U *data, int64_t n, int64_t v, float threshold,
     }
     U *stage = nullptr;
     if (data_on_host && thr.count > 0) stage = c.take<U>((size_t)(n * v));  // null if it does not fit
+    if (stage && (((uintptr_t)data | (uintptr_t)stage) & 15) && n > 0 && v > 0) {
+        // host rows off a 16-byte boundary: the copy engine stages them, the census reads the copy
+        IBP_CUDA(cudaMemcpyAsync(stage, data, (size_t)(n * v) * wb, cudaMemcpyDefault, st));
+        data = stage;
+        stage = nullptr;
+    }
     // the saved bits and the counts follow one another
     IBP_CUDA(cudaMemsetAsync(saved, 0, (size_t)((char *)(counts + v * 8 * wb) - (char *)saved), st));
     if (n > 0 && v > 0) IBP_RET(launch_census<U>(data, n, v, counts, stage, st));
