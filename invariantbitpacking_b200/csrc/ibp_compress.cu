@@ -278,6 +278,21 @@ struct PackTables {
             if (COLS * c < left_) split(p[COLS * c], x);
         }
     }
+
+    // and back to a row at o, for a group that starts it
+    __device__ __forceinline__ void write(U *__restrict__ o, int c, const uint32_t (&x)[2]) const {
+        o += COLS * c + (PAIR ? 2 : 1) * (threadIdx.x & 31);
+        if constexpr (PAIR) {
+            if ((((uintptr_t)o) & 7) == 0 && COLS * c + 1 < left) {
+                *reinterpret_cast<uint2 *>(o) = make_uint2(x[0], x[1]);
+            } else {
+                if (COLS * c < left) o[0] = x[0];
+                if (COLS * c + 1 < left) o[1] = x[1];
+            }
+        } else {
+            if (COLS * c < left) *o = (U)((uint64_t)x[0] << 32 | x[1]);
+        }
+    }
 };
 
 // Moves `words` words of a row image (units in stream order: a 64-bit word's high half first)
@@ -307,13 +322,196 @@ __device__ __forceinline__ void write_image(U *__restrict__ dst, uint32_t *image
     }
 }
 
+// Packs a group of a row (x: this lane's halves): its bitmap units and its words' kept bits are
+// ORed into the row's zeroed image (a shared address) from stream bit `at` on, which moves past
+// the group.  Offsets come from the tables where the group is all compressible, else from a
+// prefix sum.  A group that would end past stream bit `limit` leaves the image alone.
+template <typename U, int NC, bool ONE, int LEVELS>
+__device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uint32_t (&x)[NC][2],
+                                           int g, int chunks, uint32_t image, uint32_t &at,
+                                           uint32_t limit) {
+    using T = PackTables<U, NC>;
+    constexpr int H = sizeof(U) / 4;
+    const int lane = threadIdx.x & 31;
+    uint32_t p0[NC], p1[NC], off[NC];  // the halves' bits, gathered left
+    bool c0[NC], c1[NC];               // the halves compress (64-bit words: together)
+    bool every = true;
+    auto gather = [&](int c) {
+        p0[c] = gather_left<LEVELS>(x[c][0], t.m[c][0], t.mv[c][0]);
+        p1[c] = gather_left<LEVELS>(x[c][1], t.m[c][1], t.mv[c][1]);
+    };
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        if (!ONE && c >= chunks) {  // past the row's end
+            c0[c] = c1[c] = true;
+            p0[c] = p1[c] = 0;
+            off[c] = at;
+            continue;
+        }
+        const uint32_t e0 = (x[c][0] & t.m[c][0]) ^ t.bv[c][0];
+        const uint32_t e1 = (x[c][1] & t.m[c][1]) ^ t.bv[c][1];
+        c0[c] = T::PAIR ? e0 == 0 : (e0 | e1) == 0;
+        c1[c] = T::PAIR ? e1 == 0 : c0[c];
+        every = every && (e0 | e1) == 0;
+        if (!ONE) gather(c);
+        off[c] = at + t.before[c];
+    }
+    uint32_t bits = t.valid;  // lane u < UNITS: bitmap unit u of the group
+    uint32_t split[NC];       // bits of the first half
+#pragma unroll
+    for (int c = 0; c < NC; ++c) split[c] = t.nbh[c];
+    if (__all_sync(0xffffffffu, every)) {
+        at += t.all;
+        if (ONE && at > limit) return;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+            if (ONE) gather(c);
+    } else {
+        bits = 0;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            // bitmap units, LSB-first
+            if constexpr (T::PAIR) {
+                const uint32_t f = (uint32_t)c0[c] | (uint32_t)c1[c] << 1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t z = __shfl_sync(0xffffffffu, f, 16 * h + (lane >> 1));
+                    const uint32_t b = __ballot_sync(0xffffffffu, (z >> (lane & 1)) & 1);
+                    if (lane == 2 * c + h) bits = b;
+                }
+            } else {
+                const uint32_t b = __ballot_sync(0xffffffffu, c0[c]);
+                if (lane == c) bits = b;
+            }
+            split[c] = c0[c] ? t.nbh[c] : 32u;
+            const uint32_t len = split[c] + (c1[c] ? t.nb[c] - t.nbh[c] : 32u);
+            uint32_t incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t z = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += z;
+            }
+            off[c] = at + incl - len;
+            at += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        bits &= t.valid;
+        if (ONE && at > limit) return;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (ONE) gather(c);
+            p0[c] = c0[c] ? p0[c] : x[c][0];
+            p1[c] = c1[c] ? p1[c] : x[c][1];
+        }
+    }
+    // bitmap units in memory order (units past the row's last are zero and belong to
+    // the stream, where an OR of nothing does no harm)
+    or_shared(image + (uint32_t)((g * T::UNITS + (lane & (T::UNITS - 1))) ^ (H - 1)) * 4, bits);
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+        if (ONE || c < chunks)
+            put_bits(image, off[c], p0[c] | __funnelshift_rc(p1[c], 0, split[c]),
+                     __funnelshift_rc(0, p1[c], split[c]));
+}
+
+// Whether the rows at src(0), ..., src(Q - 1) save so few bits that all of them stay raw: the bits
+// set in the masks of their matching words are added up, as in the size pass.
+template <typename U, int Q, typename Src>
+__device__ __forceinline__ bool all_raw(const ColTables<U> &t, int v, Src src) {
+    constexpr int N = 8 / Q, P = 16 / sizeof(U);  // blocks of a lane and row in flight, their words
+    const int lane = threadIdx.x & 31;
+    const U *row[Q];
+    uint32_t s[Q];
+    bool aligned = v % P == 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        row[q] = src(q);
+        s[q] = 0;
+        aligned = aligned && (((uintptr_t)row[q]) & 15) == 0;
+    }
+    if (aligned) {
+        const uint4 *mask = reinterpret_cast<const uint4 *>(t.mask);
+        const uint4 *value = reinterpret_cast<const uint4 *>(t.bitval);
+        for (int i0 = lane; i0 < v / P; i0 += 32 * N) {
+            uint4 x[Q][N];
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    if (i0 + 32 * k < v / P)
+                        x[q][k] = reinterpret_cast<const uint4 *>(row[q])[i0 + 32 * k];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                if (i0 + 32 * k >= v / P) break;
+                const uint4 m = __ldg(mask + i0 + 32 * k), b = __ldg(value + i0 + 32 * k);
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const uint32_t e[4] = {(x[q][k].x & m.x) ^ b.x, (x[q][k].y & m.y) ^ b.y,
+                                           (x[q][k].z & m.z) ^ b.z, (x[q][k].w & m.w) ^ b.w};
+                    const uint32_t c[4] = {(uint32_t)__popc(m.x), (uint32_t)__popc(m.y),
+                                           (uint32_t)__popc(m.z), (uint32_t)__popc(m.w)};
+                    if constexpr (sizeof(U) == 8) {
+                        if ((e[0] | e[1]) == 0) s[q] += c[0] + c[1];
+                        if ((e[2] | e[3]) == 0) s[q] += c[2] + c[3];
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (e[i] == 0) s[q] += c[i];
+                    }
+                }
+            }
+        }
+    } else {
+        for (int j = lane; j < v; j += 32) {
+            const U m = __ldg(t.mask + j), b = __ldg(t.bitval + j);
+            const uint32_t saved = popc_w(m);
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if ((U)(row[q][j] & m) == b) s[q] += saved;
+        }
+    }
+    // none saves more than the one that saves most
+    uint32_t most = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) most = max(most, __reduce_add_sync(0xffffffffu, s[q]));
+    return compressed_bytes(v, (int)sizeof(U), most) == v * (int64_t)sizeof(U);
+}
+
+// Whether the words x of a row's first group save less than a sixteenth of their bits.
+template <typename U, int NC>
+__device__ __forceinline__ bool saves_little(const ColTables<U> &t, int v, const uint32_t (&x)[NC][2]) {
+    using T = PackTables<U, NC>;
+    const int lane = threadIdx.x & 31;
+    uint32_t s = 0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        if constexpr (T::PAIR) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = T::COLS * c + 2 * lane + h;
+                const U m = j < v ? __ldg(t.mask + j) : (U)0;
+                if ((x[c][h] & m) == (j < v ? __ldg(t.bitval + j) : (U)0)) s += popc_w(m);
+            }
+        } else {
+            const int j = T::COLS * c + lane;
+            const U m = j < v ? __ldg(t.mask + j) : (U)0, y = (U)((uint64_t)x[c][0] << 32 | x[c][1]);
+            if ((U)(y & m) == (j < v ? __ldg(t.bitval + j) : (U)0)) s += popc_w(m);
+        }
+    }
+    return __reduce_add_sync(0xffffffffu, s) * 16 <
+           (uint32_t)min(v, NC * T::COLS) * 8 * (uint32_t)sizeof(U);
+}
+
 // A warp takes Q consecutive positions at a time.  Each row goes through registers once: a
 // lane gathers its words' kept bits (left-aligned) and ORs them into the row's zeroed
-// shared-memory image at the word's bit offset, the row's length falls out of the last offset,
-// and only then is it known whether the row is stored compressed; the image is written (or, for
-// a row that stays raw, dropped) and zeroed for the next.  Offsets come from the tables where
-// a group is all compressible, else from a prefix sum.  Rows of up to one group keep their
-// tables in registers (ONE); longer ones load them per group of columns, for Q rows at once.
+// shared-memory image at the word's bit offset, and the row's length falls out of the last
+// offset; the image is then written and zeroed for the next row.  Rows of up to one group keep
+// their tables in registers (ONE), and one that stays raw is known before it is packed and
+// written from the registers.  Longer ones load the tables per group of columns, for Q rows at
+// once, and a warp passes over the batches it starts with for as long as all their rows stay raw,
+// looking closer where the first group of the first row saves next to nothing.  Calls whose rows
+// all stay raw: 200k rows of 128 and 20k of 1000 32-bit words 111 and 77 us with a size pass
+// before every row, 140 and 148 packed and dropped, 101 and 66 now; 200k and 30k of 64 and 300
+// 64-bit words 85 and 56, 115 and 95, 75 and 51.
 // The words of the next step are loaded while this one is packed.  LEVELS: moves per gather.
 template <typename U, int NC, int Q, bool ONE, bool INDEX, int LEVELS>
 __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC> &t) {
@@ -328,6 +526,7 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
     const uint32_t images_at = (uint32_t)__cvta_generic_to_shared(images);
     const int v = (int)a.v;
     const uint32_t stream0 = (uint32_t)meta_bytes(v, (int)sizeof(U)) * 8;
+    const uint32_t limit = (uint32_t)(v - 1) * W;  // last stream bit of a row below the raw one
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t batches = (a.nrows + Q - 1) / Q;
@@ -361,13 +560,38 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
             for (int c = 0; c < NC; ++c) t.read(p, c, r < 0 ? 0 : v - j, wide, x[q][c]);
         }
     };
+    // where row i of the output starts
+    auto target = [&](int64_t i) -> U * {
+        return a.out ? a.out + i * v
+                     : reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
+                                             (i ? a.offsets[i - 1] : 0));
+    };
     // fixed-stride rows of whole 16-byte blocks, at most one per lane
     const int n16 = v * (int)sizeof(U) / 16;
     const bool blocks = ONE && a.out && n16 <= 32 && v * (int)sizeof(U) % 16 == 0 &&
                         (((uintptr_t)a.out) & 15) == 0;
     uint32_t x[Q][NC][2];
-    if (warp < batches) load(warp, 0, x);
-    for (int64_t batch = warp; batch < batches; batch += nwarps) {
+    int64_t batch = warp;
+    if (batch < batches) load(batch, 0, x);
+    if constexpr (!ONE) {
+        // batches of rows that all stay raw, up to the first other one
+        while (batch < batches && saves_little<U, NC>(a.t, v, x[0])) {
+            const bool raw = all_raw<U, Q>(a.t, v, [&](int q) {
+                const int64_t r = source(batch, q);
+                return a.src + (r < 0 ? 0 : r) * v;
+            });
+            if (!raw) break;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int64_t i = batch * Q + q, r = source(batch, q);
+                if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
+                if (r < 0 && i < a.nrows && lane == 0) atomicOr(a.status, kStatusBadIndex);
+            }
+            batch += nwarps;
+            if (batch < batches) load(batch, 0, x);
+        }
+    }
+    for (; batch < batches; batch += nwarps) {
         uint32_t at[Q];  // stream bits so far
 #pragma unroll
         for (int q = 0; q < Q; ++q) at[q] = stream0;
@@ -378,77 +602,22 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                 load(more ? batch : batch + nwarps, more ? g + 1 : 0, y);
             if (!ONE) t.load(a.t, v, g * GCOLS);
             const int chunks = ONE ? NC : min(NC, (v - g * GCOLS + T::COLS - 1) / T::COLS);
+if constexpr (ONE) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                uint32_t p0[NC], p1[NC], off[NC];  // the halves' bits, gathered left
-                bool c0[NC], c1[NC];               // the halves compress (64-bit words: together)
-                bool every = true;
+                for (int q = 0; q < Q; ++q) {
+                    pack_group<U, NC, ONE, LEVELS>(t, x[q], g, chunks,
+                                                   images_at + q * image_units * 4, at[q], limit);
+                    if (at[q] > limit && !a.in_place && source(batch, q) >= 0) {
+                        U *o = target(batch * Q + q);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if (!ONE && c >= chunks) {  // past the row's end
-                        c0[c] = c1[c] = true;
-                        p0[c] = p1[c] = 0;
-                        off[c] = at[q];
-                        continue;
+                        for (int c = 0; c < NC; ++c) t.write(o, c, x[q][c]);
                     }
-                    const uint32_t e0 = (x[q][c][0] & t.m[c][0]) ^ t.bv[c][0];
-                    const uint32_t e1 = (x[q][c][1] & t.m[c][1]) ^ t.bv[c][1];
-                    c0[c] = T::PAIR ? e0 == 0 : (e0 | e1) == 0;
-                    c1[c] = T::PAIR ? e1 == 0 : c0[c];
-                    every = every && (e0 | e1) == 0;
-                    p0[c] = gather_left<LEVELS>(x[q][c][0], t.m[c][0], t.mv[c][0]);
-                    p1[c] = gather_left<LEVELS>(x[q][c][1], t.m[c][1], t.mv[c][1]);
-                    off[c] = at[q] + t.before[c];
                 }
-                uint32_t bits = t.valid;  // lane u < UNITS: bitmap unit u of the group
-                uint32_t split[NC];       // bits of the first half
+            } else {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) split[c] = t.nbh[c];
-                if (__all_sync(0xffffffffu, every)) {
-                    at[q] += t.all;
-                } else {
-                    bits = 0;
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        // bitmap units, LSB-first
-                        if constexpr (T::PAIR) {
-                            const uint32_t f = (uint32_t)c0[c] | (uint32_t)c1[c] << 1;
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const uint32_t z =
-                                    __shfl_sync(0xffffffffu, f, 16 * h + (lane >> 1));
-                                const uint32_t b = __ballot_sync(0xffffffffu, (z >> (lane & 1)) & 1);
-                                if (lane == 2 * c + h) bits = b;
-                            }
-                        } else {
-                            const uint32_t b = __ballot_sync(0xffffffffu, c0[c]);
-                            if (lane == c) bits = b;
-                        }
-                        split[c] = c0[c] ? t.nbh[c] : 32u;
-                        const uint32_t len = split[c] + (c1[c] ? t.nb[c] - t.nbh[c] : 32u);
-                        uint32_t incl = len;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const uint32_t z = __shfl_up_sync(0xffffffffu, incl, o);
-                            if (lane >= o) incl += z;
-                        }
-                        off[c] = at[q] + incl - len;
-                        at[q] += __shfl_sync(0xffffffffu, incl, 31);
-                        p0[c] = c0[c] ? p0[c] : x[q][c][0];
-                        p1[c] = c1[c] ? p1[c] : x[q][c][1];
-                    }
-                    bits &= t.valid;
-                }
-                // bitmap units in memory order (units past the row's last are zero and belong to
-                // the stream, where an OR of nothing does no harm)
-                const uint32_t image = images_at + q * image_units * 4;
-                or_shared(image + (uint32_t)((g * T::UNITS + (lane & (T::UNITS - 1))) ^ (H - 1)) * 4,
-                          bits);
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (ONE || c < chunks)
-                        put_bits(image, off[c], p0[c] | __funnelshift_rc(p1[c], 0, split[c]),
-                                 __funnelshift_rc(0, p1[c], split[c]));
+                for (int q = 0; q < Q; ++q)
+                    pack_group<U, NC, ONE, LEVELS>(t, x[q], g, chunks,
+                                                   images_at + q * image_units * 4, at[q], ~0u);
             }
 #pragma unroll
             for (int q = 0; q < Q; ++q)
@@ -477,24 +646,14 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                         reinterpret_cast<uint4 *>(a.out + i * v)[lane] =
                             H == 2 ? make_uint4(x.y, x.x, x.w, x.z) : x;
                     }
-                } else if (a.out)
-                    write_image<U>(a.out + i * v, image, v);
-                else
-                    write_image<U>(reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
-                                                         (i ? a.offsets[i - 1] : 0)),
-                                   image, words);
+                } else {
+                    write_image<U>(target(i), image, a.out ? v : words);
+                }
                 continue;
             }
-            if (r >= 0) {
-                if (!a.out)
-                    warp_copy<U>(reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
-                                                       (i ? a.offsets[i - 1] : 0)),
-                                 a.src + r * v, v);
-                else if (!a.in_place)
-                    warp_copy<U>(a.out + i * v, a.src + r * v, v);
-            } else if (lane == 0) {
-                atomicOr(a.status, kStatusBadIndex);
-            }
+            if (r < 0 && lane == 0) atomicOr(a.status, kStatusBadIndex);
+            if (ONE && words >= v) continue;  // nothing was packed, and the row is written
+            if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
             for (int k = lane; k < words * H; k += 32) image[k] = 0;
         }
         // Q divides 32 and the batch starts at a multiple of Q: one bitmask word
@@ -559,8 +718,9 @@ static ibp_status launch_pack(PackArgs<U> a, cudaStream_t st) {
     if (a.v <= cols) return launch_pack_q<U, 1, 4, true>(a, 8, 4 * 8 * row, st);
     if (a.v <= 2 * cols) return launch_pack_q<U, 2, 4, true>(a, 8, 4 * 8 * row, st);
     // longer rows: 4 rows share a load of the tables while two blocks of 8 warps fit an SM,
-    // else 1 row and as many warps as fit
-    if (4 * 8 * row <= 100 * 1024) return launch_pack_q<U, 2, 4, false>(a, 8, 4 * 8 * row, st);
+    // else 1 row and as many warps as fit; and 1 row where every row has a warp of its own
+    if (4 * 8 * row <= 100 * 1024 && a.nrows > (int64_t)device_sm_count() * 16)
+        return launch_pack_q<U, 2, 4, false>(a, 8, 4 * 8 * row, st);
     const int warps = (int)std::min<size_t>(8, (size_t)maxs / row);
     return launch_pack_q<U, 2, 1, false>(a, warps, (size_t)warps * row, st);
 }

@@ -1,0 +1,96 @@
+"""Rows that stay raw among rows that are packed, against the CPU oracle: all raw, raw up to some
+position, rows whose first columns save nothing though the row does, and the other way round; short
+rows, rows of several groups of columns, few rows and more than the grid has warps, bad indices.
+And packing rows that all stay raw takes less time than packing rows that do not."""
+import numpy as np
+import pytest
+import torch
+from torch.profiler import ProfilerActivity, profile
+
+pytestmark = pytest.mark.gpu
+
+INT = {4: np.int32, 8: np.int64}
+UINT = {4: np.uint32, 8: np.uint64}
+
+
+def rows_of(rng, n, v, wb, kind):
+    """Half of every word's bits invariant; `kind` says which words are off the pattern."""
+    m = rng.integers(0, 2**64, v, dtype=np.uint64)
+    base = rng.integers(0, 2**64, v, dtype=np.uint64) & m
+    noise = rng.integers(0, 2**64, (n, v), dtype=np.uint64)
+    x = (noise & ~m) | base
+    first = np.arange(v) < min(v, 512 // wb)     # the first group of columns
+    row = np.arange(n)[:, None]
+    off = {"all": np.ones((n, v), bool),
+           "leading": np.broadcast_to(row < 2 * n // 3, (n, v)),
+           "some": np.broadcast_to(rng.random((n, 1)) < 0.3, (n, v)),
+           "first": np.broadcast_to(first & (row % 5 != 0), (n, v)),
+           "but_first": np.broadcast_to(~first, (n, v))}[kind]
+    x = np.where(off, noise, x)
+    return tuple(a.astype(UINT[wb]).view(INT[wb]) for a in (x, m, base))
+
+
+@pytest.mark.parametrize("kind", ["all", "leading", "some", "first", "but_first"])
+@pytest.mark.parametrize("wb,v,n", [(4, 1, 50), (4, 64, 300), (4, 127, 333), (4, 128, 90),
+                                    (4, 129, 7), (4, 140, 2401), (4, 260, 9700), (4, 1100, 2450),
+                                    (8, 2, 70), (8, 33, 101), (8, 64, 130), (8, 65, 2500),
+                                    (8, 130, 9600), (8, 700, 5), (8, 4100, 40)])
+def test_raw_rows_among_packed_ones(oracle, wb, v, n, kind):
+    import invariantbitpacking_b200 as ibp
+    rng = np.random.default_rng(100 * v + wb + n)
+    x, m, b = rows_of(rng, n, v, wb, kind)
+    dm, db = torch.from_numpy(m).cuda(), torch.from_numpy(b).cuda()
+    src = torch.from_numpy(x).cuda()
+    want, want_bits = oracle.compress(x, m, b)
+    t = src.clone()
+    bits = ibp.compress_inplace(t, dm, db)
+    torch.cuda.synchronize()
+    assert np.array_equal(bits.cpu().numpy(), want_bits)
+    assert np.array_equal(t.cpu().numpy(), want.view(INT[wb]))
+    words, offs = oracle.compress_condensed(x, m, b)
+    cw, co = ibp.compress_condensed(src, dm, db)
+    torch.cuda.synchronize()
+    assert np.array_equal(co.cpu().numpy(), offs)
+    assert np.array_equal(cw.cpu().numpy(), words.view(INT[wb]))
+    # bad positions among them take no bytes; an index in place reads every row first
+    idx = rng.integers(0, n, n)
+    bad = rng.random(n) < 0.2
+    words, offs = oracle.compress_condensed(x, m, b, idx[~bad])
+    cw, co = ibp.compress_condensed(src, dm, db, torch.from_numpy(np.where(bad, n, idx)).cuda())
+    torch.cuda.synchronize()
+    assert np.array_equal(co.cpu().numpy()[~bad], offs)
+    assert np.array_equal(cw.cpu().numpy(), words.view(INT[wb]))
+    want, want_bits = oracle.compress(x, m, b, idx)
+    t = src.clone()
+    bits = ibp.compress_inplace(t, dm, db, torch.from_numpy(idx).cuda())
+    torch.cuda.synchronize()
+    assert np.array_equal(bits.cpu().numpy(), want_bits)
+    assert np.array_equal(t.cpu().numpy(), want.view(INT[wb]))
+
+
+@pytest.mark.parametrize("wb,v", [(4, 64), (4, 256), (4, 1000), (8, 64), (8, 128), (8, 300)])
+def test_raw_rows_take_less_time_than_packed_ones(wb, v):
+    import invariantbitpacking_b200 as ibp
+    n = (96 << 20) // (v * wb)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(v)
+    dtype = torch.from_numpy(np.zeros(1, INT[wb])).dtype
+    noise = torch.randint(-2**63, 2**63 - 1, (n, v), generator=g, device="cuda").to(dtype)
+    mask = torch.randint(-2**63, 2**63 - 1, (v,), generator=g, device="cuda").to(dtype)
+
+    def pack_us(x):
+        rows = x.clone()
+        ibp.compress_inplace(rows, mask, mask)
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            for _ in range(4):
+                rows.copy_(x)
+                ibp.compress_inplace(rows, mask, mask)
+            torch.cuda.synchronize()
+        took = [e.self_device_time_total for e in prof.key_averages() if "pack" in e.key]
+        assert took
+        return sum(took) / 4
+
+    packed = pack_us(noise | mask)
+    raw = pack_us(noise)
+    assert raw < packed, (raw, packed)
