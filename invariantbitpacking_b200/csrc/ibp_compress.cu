@@ -172,6 +172,7 @@ struct PackArgs {
     int32_t *bitmask;
     int32_t *status;
     int64_t buf_words;  // shared-memory words per output row
+    int64_t stage_words;  // and per input row, for rows in host memory
 };
 
 // A lane packs 64 bits of a row at a time, as two halves, high first: one 64-bit word, or two
@@ -278,21 +279,6 @@ struct PackTables {
             if (COLS * c < left_) split(p[COLS * c], x);
         }
     }
-
-    // and back to a row at o, for a group that starts it
-    __device__ __forceinline__ void write(U *__restrict__ o, int c, const uint32_t (&x)[2]) const {
-        o += COLS * c + (PAIR ? 2 : 1) * (threadIdx.x & 31);
-        if constexpr (PAIR) {
-            if ((((uintptr_t)o) & 7) == 0 && COLS * c + 1 < left) {
-                *reinterpret_cast<uint2 *>(o) = make_uint2(x[0], x[1]);
-            } else {
-                if (COLS * c < left) o[0] = x[0];
-                if (COLS * c + 1 < left) o[1] = x[1];
-            }
-        } else {
-            if (COLS * c < left) *o = (U)((uint64_t)x[0] << 32 | x[1]);
-        }
-    }
 };
 
 // Moves `words` words of a row image (units in stream order: a 64-bit word's high half first)
@@ -325,7 +311,7 @@ __device__ __forceinline__ void write_image(U *__restrict__ dst, uint32_t *image
 // Packs a group of a row (x: this lane's halves): its bitmap units and its words' kept bits are
 // ORed into the row's zeroed image (a shared address) from stream bit `at` on, which moves past
 // the group.  Offsets come from the tables where the group is all compressible, else from a
-// prefix sum.  A group that would end past stream bit `limit` leaves the image alone.
+// prefix sum.  A row of one group that would end past stream bit `limit` leaves the image alone.
 template <typename U, int NC, bool ONE, int LEVELS>
 __device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uint32_t (&x)[NC][2],
                                            int g, int chunks, uint32_t image, uint32_t &at,
@@ -336,10 +322,6 @@ __device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uin
     uint32_t p0[NC], p1[NC], off[NC];  // the halves' bits, gathered left
     bool c0[NC], c1[NC];               // the halves compress (64-bit words: together)
     bool every = true;
-    auto gather = [&](int c) {
-        p0[c] = gather_left<LEVELS>(x[c][0], t.m[c][0], t.mv[c][0]);
-        p1[c] = gather_left<LEVELS>(x[c][1], t.m[c][1], t.mv[c][1]);
-    };
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         if (!ONE && c >= chunks) {  // past the row's end
@@ -353,7 +335,8 @@ __device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uin
         c0[c] = T::PAIR ? e0 == 0 : (e0 | e1) == 0;
         c1[c] = T::PAIR ? e1 == 0 : c0[c];
         every = every && (e0 | e1) == 0;
-        if (!ONE) gather(c);
+        p0[c] = gather_left<LEVELS>(x[c][0], t.m[c][0], t.mv[c][0]);
+        p1[c] = gather_left<LEVELS>(x[c][1], t.m[c][1], t.mv[c][1]);
         off[c] = at + t.before[c];
     }
     uint32_t bits = t.valid;  // lane u < UNITS: bitmap unit u of the group
@@ -362,10 +345,6 @@ __device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uin
     for (int c = 0; c < NC; ++c) split[c] = t.nbh[c];
     if (__all_sync(0xffffffffu, every)) {
         at += t.all;
-        if (ONE && at > limit) return;
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-            if (ONE) gather(c);
     } else {
         bits = 0;
 #pragma unroll
@@ -393,16 +372,12 @@ __device__ __forceinline__ void pack_group(const PackTables<U, NC> &t, const uin
             }
             off[c] = at + incl - len;
             at += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        bits &= t.valid;
-        if (ONE && at > limit) return;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            if (ONE) gather(c);
             p0[c] = c0[c] ? p0[c] : x[c][0];
             p1[c] = c1[c] ? p1[c] : x[c][1];
         }
+        bits &= t.valid;
     }
+    if (ONE && at > limit) return;
     // bitmap units in memory order (units past the row's last are zero and belong to
     // the stream, where an OR of nothing does no harm)
     or_shared(image + (uint32_t)((g * T::UNITS + (lane & (T::UNITS - 1))) ^ (H - 1)) * 4, bits);
@@ -505,13 +480,13 @@ __device__ __forceinline__ bool saves_little(const ColTables<U> &t, int v, const
 // lane gathers its words' kept bits (left-aligned) and ORs them into the row's zeroed
 // shared-memory image at the word's bit offset, and the row's length falls out of the last
 // offset; the image is then written and zeroed for the next row.  Rows of up to one group keep
-// their tables in registers (ONE), and one that stays raw is known before it is packed and
-// written from the registers.  Longer ones load the tables per group of columns, for Q rows at
-// once, and a warp passes over the batches it starts with for as long as all their rows stay raw,
-// looking closer where the first group of the first row saves next to nothing.  Calls whose rows
-// all stay raw: 200k rows of 128 and 20k of 1000 32-bit words 111 and 77 us with a size pass
-// before every row, 140 and 148 packed and dropped, 101 and 66 now; 200k and 30k of 64 and 300
-// 64-bit words 85 and 56, 115 and 95, 75 and 51.
+// their tables in registers (ONE), and one that stays raw is known before it reaches its image.
+// Longer ones load the tables per group of columns, for Q rows at once.  A warp passes over the
+// batches it starts with for as long as all their rows stay raw, looking through them where the
+// first group of the first row saves next to nothing.  Calls whose rows all stay raw: 200k rows
+// of 128 and 20k of 1000 32-bit words 111 and 77 us with a size pass before every row, 140 and 148
+// packed and dropped, 76 and 58 now; 200k and 30k of 64 and 300 64-bit words 85 and 56, 115 and
+// 95, 77 and 54.
 // The words of the next step are loaded while this one is packed.  LEVELS: moves per gather.
 template <typename U, int NC, int Q, bool ONE, bool INDEX, int LEVELS>
 __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC> &t) {
@@ -573,23 +548,26 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
     uint32_t x[Q][NC][2];
     int64_t batch = warp;
     if (batch < batches) load(batch, 0, x);
-    if constexpr (!ONE) {
-        // batches of rows that all stay raw, up to the first other one
-        while (batch < batches && saves_little<U, NC>(a.t, v, x[0])) {
-            const bool raw = all_raw<U, Q>(a.t, v, [&](int q) {
-                const int64_t r = source(batch, q);
-                return a.src + (r < 0 ? 0 : r) * v;
-            });
-            if (!raw) break;
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int64_t i = batch * Q + q, r = source(batch, q);
-                if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
-                if (r < 0 && i < a.nrows && lane == 0) atomicOr(a.status, kStatusBadIndex);
-            }
-            batch += nwarps;
-            if (batch < batches) load(batch, 0, x);
+    // batches of rows that all stay raw, up to the first other one
+    while (batch < batches && saves_little<U, NC>(a.t, v, x[0])) {
+        if (!INDEX && batch + nwarps < batches) {  // the next batch's rows, a line a lane
+            const char *next = reinterpret_cast<const char *>(a.src + (batch + nwarps) * Q * v);
+            const int64_t bytes = min((int64_t)Q, a.nrows - (batch + nwarps) * Q) * v * (int)sizeof(U);
+            if (lane * 128 < bytes) asm volatile("prefetch.global.L1 [%0];" ::"l"(next + lane * 128));
         }
+        const bool raw = all_raw<U, Q>(a.t, v, [&](int q) {
+            const int64_t r = source(batch, q);
+            return a.src + (r < 0 ? 0 : r) * v;
+        });
+        if (!raw) break;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int64_t i = batch * Q + q, r = source(batch, q);
+            if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
+            if (r < 0 && i < a.nrows && lane == 0) atomicOr(a.status, kStatusBadIndex);
+        }
+        batch += nwarps;
+        if (batch < batches) load(batch, 0, x);
     }
     for (; batch < batches; batch += nwarps) {
         uint32_t at[Q];  // stream bits so far
@@ -602,23 +580,10 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                 load(more ? batch : batch + nwarps, more ? g + 1 : 0, y);
             if (!ONE) t.load(a.t, v, g * GCOLS);
             const int chunks = ONE ? NC : min(NC, (v - g * GCOLS + T::COLS - 1) / T::COLS);
-if constexpr (ONE) {
 #pragma unroll
-                for (int q = 0; q < Q; ++q) {
-                    pack_group<U, NC, ONE, LEVELS>(t, x[q], g, chunks,
-                                                   images_at + q * image_units * 4, at[q], limit);
-                    if (at[q] > limit && !a.in_place && source(batch, q) >= 0) {
-                        U *o = target(batch * Q + q);
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) t.write(o, c, x[q][c]);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < Q; ++q)
-                    pack_group<U, NC, ONE, LEVELS>(t, x[q], g, chunks,
-                                                   images_at + q * image_units * 4, at[q], ~0u);
-            }
+            for (int q = 0; q < Q; ++q)
+                pack_group<U, NC, ONE, LEVELS>(t, x[q], g, chunks,
+                                               images_at + q * image_units * 4, at[q], limit);
 #pragma unroll
             for (int q = 0; q < Q; ++q)
 #pragma unroll
@@ -652,8 +617,8 @@ if constexpr (ONE) {
                 continue;
             }
             if (r < 0 && lane == 0) atomicOr(a.status, kStatusBadIndex);
-            if (ONE && words >= v) continue;  // nothing was packed, and the row is written
             if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
+            if (ONE && words >= v) continue;  // nothing was packed
             for (int k = lane; k < words * H; k += 32) image[k] = 0;
         }
         // Q divides 32 and the batch starts at a multiple of Q: one bitmask word
@@ -683,6 +648,80 @@ __global__ void __launch_bounds__(256, 2) pack_rows_kernel(PackArgs<U> a) {
         }
     }
     pack_rows<U, NC, Q, ONE, INDEX, kMoves>(a, t);
+}
+
+// Rows in host memory: a warp brings a row over the link once, whole, into shared memory, where
+// its size is taken, and writes it from there or packs it.  Bound: the link.  Through
+// pack_rows_kernel, whose lanes fetch their own words of four rows and which reads a row that
+// stays raw twice: 30k rows of 300 64-bit words in place 2372 us, here 2007; 10k raw ones of 1000
+// back to back 6421 and 4605.
+template <typename U, int NC, bool ONE, bool INDEX>
+__global__ void __launch_bounds__(256, 2) pack_host_rows_kernel(PackArgs<U> a) {
+    using T = PackTables<U, NC>;
+    constexpr int W = 8 * sizeof(U), H = sizeof(U) / 4, GCOLS = T::COLS * NC;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    U *row = reinterpret_cast<U *>(smem) +
+             (int64_t)(threadIdx.x >> 5) * (a.stage_words + a.buf_words);
+    uint32_t *image = reinterpret_cast<uint32_t *>(row + a.stage_words);
+    const uint32_t image_at = (uint32_t)__cvta_generic_to_shared(image);
+    const int v = (int)a.v;
+    const uint32_t stream0 = (uint32_t)meta_bytes(v, (int)sizeof(U)) * 8;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int k = lane; k < (int)a.buf_words * H; k += 32) image[k] = 0;
+    T t;
+    if (ONE) t.load(a.t, v, 0);
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < a.nrows;
+         i += nwarps) {
+        const int64_t r = INDEX ? a.idx[i] : i;
+        if (INDEX && (r < 0 || r >= a.n)) {
+            if (lane == 0) atomicOr(a.status, kStatusBadIndex);
+            continue;
+        }
+        warp_copy<U>(row, a.src + r * v, v);
+        __syncwarp();
+        uint32_t s = 0;
+        for (int j = lane; j < v; j += 32) {
+            const U m = __ldg(a.t.mask + j);
+            if ((U)(row[j] & m) == __ldg(a.t.bitval + j)) s += popc_w(m);
+        }
+        s = __reduce_add_sync(0xffffffffu, s);
+        U *o = a.out ? a.out + i * v
+                     : reinterpret_cast<U *>(reinterpret_cast<char *>(a.cond) +
+                                             (i ? a.offsets[i - 1] : 0));
+        if (compressed_bytes(v, (int)sizeof(U), s) == v * (int64_t)sizeof(U)) {
+            if (!a.in_place) warp_copy<U>(o, row, v);
+            __syncwarp();
+            continue;
+        }
+        uint32_t at = stream0;
+        for (int j0 = 0, g = 0; j0 < v; j0 += GCOLS, ++g) {
+            if (!ONE) t.load(a.t, v, j0);
+            const int j = j0 + (T::PAIR ? 2 : 1) * lane;
+            uint32_t x[NC][2];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) t.read(row + j, c, v - j, v % 2 == 0, x[c]);
+            pack_group<U, NC, ONE, kMoves>(t, x, g, min(NC, (v - j0 + T::COLS - 1) / T::COLS),
+                                           image_at, at, ~0u);
+        }
+        __syncwarp();
+        write_image<U>(o, image, a.out ? v : (int)((at + W - 1) / W));
+        if (a.out && lane == 0) atomicOr(&a.bitmask[i >> 5], (int32_t)(1u << (i & 31)));
+        __syncwarp();
+    }
+}
+
+template <typename U, int NC, bool ONE>
+static ibp_status launch_pack_host(const PackArgs<U> &a, size_t row, cudaStream_t st) {
+    auto kern = a.idx ? pack_host_rows_kernel<U, NC, ONE, true> : pack_host_rows_kernel<U, NC, ONE, false>;
+    const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, 96 * 1024 / row));
+    int per_sm = 0;
+    IBP_RET(kernel_blocks_per_sm((const void *)kern, warps * 32, warps * row, &per_sm));
+    const int64_t blocks =
+        std::min<int64_t>((a.nrows + warps - 1) / warps, (int64_t)device_sm_count() * per_sm);
+    kern<<<(unsigned)blocks, warps * 32, warps * row, st>>>(a);
+    IBP_LAUNCHED("pack_host_rows_kernel");
+    return IBP_OK;
 }
 
 template <typename U, int NC, int Q, bool ONE>
@@ -715,6 +754,24 @@ static ibp_status launch_pack(PackArgs<U> a, cudaStream_t st) {
         16 / sizeof(U));
     const size_t row = (size_t)a.buf_words * sizeof(U);
     constexpr int cols = PackTables<U, 1>::COLS;
+    // Host rows of whole 16-byte blocks and at least 512 bytes; and tiny ones packed back to back
+    // (500k rows of two 64-bit words 1655 us, here 1242).  Other rows, above all those off 16-byte
+    // boundaries, are brought faster four at a time (200k of 99 32-bit words in place 2478 us,
+    // here 4567; of 16 words 1192 and 1320; of 64 words 2083 and 2073).
+    const int64_t row_bytes = a.v * (int64_t)sizeof(U);
+    const bool whole = row_bytes >= 512 && row_bytes % 16 == 0 && (((uintptr_t)a.src) & 15) == 0;
+    if ((a.in_place || !a.out) && (whole || (!a.out && row_bytes <= 32))) {
+        cudaPointerAttributes pa{};
+        if (cudaPointerGetAttributes(&pa, a.src) != cudaSuccess) cudaGetLastError();
+        a.stage_words = (int64_t)align_up((size_t)a.v, 16 / sizeof(U));
+        const size_t both = row + (size_t)a.stage_words * sizeof(U);
+        // (the longest rows' words and image do not both fit)
+        if (pa.type == cudaMemoryTypeHost && both <= (size_t)maxs) {
+            if (a.v <= cols) return launch_pack_host<U, 1, true>(a, both, st);
+            if (a.v <= 2 * cols) return launch_pack_host<U, 2, true>(a, both, st);
+            return launch_pack_host<U, 2, false>(a, both, st);
+        }
+    }
     if (a.v <= cols) return launch_pack_q<U, 1, 4, true>(a, 8, 4 * 8 * row, st);
     if (a.v <= 2 * cols) return launch_pack_q<U, 2, 4, true>(a, 8, 4 * 8 * row, st);
     // longer rows: 4 rows share a load of the tables while two blocks of 8 warps fit an SM,

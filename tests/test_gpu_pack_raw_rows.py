@@ -94,3 +94,55 @@ def test_raw_rows_take_less_time_than_packed_ones(wb, v):
     packed = pack_us(noise | mask)
     raw = pack_us(noise)
     assert raw < packed, (raw, packed)
+
+
+@pytest.mark.parametrize("kind", ["all", "some", "but_first"])
+@pytest.mark.parametrize("wb,v,n", [(4, 1, 70), (4, 33, 300), (4, 128, 200), (4, 200, 90),
+                                    (8, 2, 90), (8, 3, 40), (8, 64, 130), (8, 65, 300),
+                                    (8, 128, 70), (8, 1000, 20), (8, 14000, 3), (8, 14500, 2)])
+def test_host_rows(oracle, wb, v, n, kind):
+    """Rows in pinned memory: whole 16-byte blocks and not, tiny rows, rows longer than a warp's
+    words and image together; in place, back to back, and by an index with bad positions."""
+    import invariantbitpacking_b200 as ibp
+    rng = np.random.default_rng(100 * v + wb + n)
+    x, m, b = rows_of(rng, n, v, wb, kind)
+    dm, db = torch.from_numpy(m).cuda(), torch.from_numpy(b).cuda()
+    src = torch.from_numpy(x).pin_memory()
+    words, offs = oracle.compress_condensed(x, m, b)
+    cw, co = ibp.compress_condensed(src, dm, db)
+    assert np.array_equal(co.numpy(), offs) and np.array_equal(cw.numpy(), words.view(INT[wb]))
+    idx = rng.integers(0, n, n)
+    bad = rng.random(n) < 0.2
+    words, offs = oracle.compress_condensed(x, m, b, idx[~bad])
+    cw, co = ibp.compress_condensed(src, dm, db, torch.from_numpy(np.where(bad, -1, idx)).cuda())
+    assert np.array_equal(co.numpy()[~bad], offs) and np.array_equal(cw.numpy(), words.view(INT[wb]))
+    want, want_bits = oracle.compress(x, m, b)
+    bits = ibp.compress_inplace(src, dm, db)
+    assert np.array_equal(bits.cpu().numpy(), want_bits)
+    assert np.array_equal(src.numpy(), want.view(INT[wb]))
+
+
+def test_raw_host_rows_cross_the_link_once():
+    """Raw host rows of 8 KiB packed back to back: read once and written once, in little more than
+    the packed ones' time (they write twice as much)."""
+    import invariantbitpacking_b200 as ibp
+    n, v = 8000, 1000
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    noise = torch.randint(-2**63, 2**63 - 1, (n, v), generator=g, device="cuda")
+    mask = torch.randint(-2**63, 2**63 - 1, (v,), generator=g, device="cuda")
+
+    def pack_us(x):
+        rows = x.cpu().pin_memory()
+        ibp.compress_condensed(rows, mask, mask)
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            for _ in range(4):
+                ibp.compress_condensed(rows, mask, mask)
+            torch.cuda.synchronize()
+        took = [e.self_device_time_total for e in prof.key_averages() if "pack" in e.key]
+        assert took
+        return sum(took) / 4
+
+    read = n * v * 8 / 55e3  # us at the link's rate, either way
+    assert pack_us(noise) < 1.7 * read
