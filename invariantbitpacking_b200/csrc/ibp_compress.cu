@@ -114,12 +114,93 @@ compress_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
     }
 }
 
+// Few rows of more than one step: a row to a warp or, with ROWS == 1, to a block of 8 warps, 4 steps
+// of a warp in flight.
+template <typename U, int A, int ROWS, bool INDEX>
+__global__ void __launch_bounds__(256, 4)
+few_rows_size_kernel(const U *__restrict__ data, int64_t n, int64_t v,
+                     const U *__restrict__ mask, const U *__restrict__ bitval,
+                     const int64_t *__restrict__ idx, int64_t nrows,
+                     int64_t *__restrict__ sizes, unsigned long long *__restrict__ total,
+                     int32_t *__restrict__ status, uint32_t one) {
+    using C = Chunk<U, A, 32>;
+    constexpr int P = 4, SP = 32 * C::NS, WARPS = 8 / ROWS;  // warps of a row
+    __shared__ uint32_t sums[2][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t row_bytes = v * (int64_t)sizeof(U);
+    const int64_t chunks = row_bytes / A;
+    const int part = warp % WARPS;
+    unsigned long long acc = 0;
+    int now = 0;
+    for (int64_t i = (int64_t)blockIdx.x * ROWS + warp / WARPS; i < nrows;
+         i += (int64_t)gridDim.x * ROWS) {
+        const int64_t r = INDEX ? idx[i] : i;
+        if (INDEX && (r < 0 || r >= n)) {
+            if (part == 0 && lane == 0) {
+                sizes[i] = 0;
+                if (status) atomicOr(status, kStatusBadIndex);
+            }
+            continue;
+        }
+        const char *row = reinterpret_cast<const char *>(data) + r * row_bytes;
+        uint32_t s = 0;
+        for (int64_t c = (int64_t)part * P * SP + lane; c < chunks; c += WARPS * P * SP) {
+            uint32_t x[P][C::NR];
+#pragma unroll
+            for (int p = 0; p < P; ++p) C::load(row, c + p * SP, chunks, x[p]);
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                uint32_t m[C::NR], b[C::NR], pc[C::NW];
+                C::load_words(mask, c + p * SP, chunks, m);
+                C::load_words(bitval, c + p * SP, chunks, b);
+                C::set_bits(m, pc);
+                C::matched(s, [&](int k) { return (x[p][k] & m[k]) ^ b[k]; }, pc, one);
+            }
+        }
+        s = __reduce_add_sync(0xffffffffu, s);
+        if constexpr (WARPS > 1) {
+            // (two sets of sums: the one read here is next written after the next row's barrier)
+            if (lane == 0) sums[now][warp] = s;
+            __syncthreads();
+            s = __reduce_add_sync(0xffffffffu, lane < WARPS ? sums[now][lane] : 0u);
+            now ^= 1;
+        }
+        if (part == 0 && lane == 0) {
+            const int64_t sz = compressed_bytes(v, (int)sizeof(U), s);
+            sizes[i] = sz;
+            acc += (unsigned long long)sz;
+        }
+    }
+    if (total && acc) atomicAdd(total, acc);
+}
+
 template <typename U, int A>
 static ibp_status launch_sizes(const U *data, int64_t n, int64_t v, const U *mask,
                                const U *bitval, const int64_t *idx, int64_t nrows,
                                int64_t *sizes, int64_t *total, int32_t *status,
                                cudaStream_t st) {
     const int64_t chunks = v * (int64_t)sizeof(U) / A;
+    int per_sm = 0;
+    // Rows of several steps, too few for every warp to have 8: a block each up to 8 rows per SM (and
+    // of long ones up to 32), a warp each up to 48.  600 rows of 60,000 32-bit words: a warp each
+    // and a word a lane 425 us, eight to a warp 545, a block each 50; 3333 of 4096, indexed: 18.7, 31.5,
+    // 19.4 (a block each 22); 10,000 of 2000 64-bit words 48, 46 (a block each 50), and off 16-byte
+    // boundaries, where eight rows to a warp are slower, 48, 57, 38.
+    const int64_t sms = device_sm_count();
+    const bool block_each = nrows <= 8 * sms || (nrows <= 32 * sms && v * sizeof(U) >= 32768);
+    if (chunks > 32 * Chunk<U, A, 32>::NS && (block_each || nrows <= (A == 16 ? 48 : 128) * sms)) {
+        auto few = block_each ? (idx ? few_rows_size_kernel<U, A, 1, true>
+                                     : few_rows_size_kernel<U, A, 1, false>)
+                              : (idx ? few_rows_size_kernel<U, A, 8, true>
+                                     : few_rows_size_kernel<U, A, 8, false>);
+        IBP_RET(kernel_blocks_per_sm((const void *)few, 256, 0, &per_sm));
+        const int64_t blocks =
+            std::min<int64_t>(block_each ? nrows : (nrows + 7) / 8, sms * per_sm);
+        few<<<(unsigned)blocks, 256, 0, st>>>(data, n, v, mask, bitval, idx, nrows, sizes,
+                                              (unsigned long long *)total, status, 1u);
+        IBP_LAUNCHED("few_rows_size_kernel");
+        return IBP_OK;
+    }
     auto kern = idx ? compress_size_kernel<U, A, 32, true> : compress_size_kernel<U, A, 32, false>;
     int lanes = 32;
     if (chunks <= 8 * Chunk<U, A, 8>::NS) {
@@ -130,7 +211,6 @@ static ibp_status launch_sizes(const U *data, int64_t n, int64_t v, const U *mas
         lanes = 16;
     }
     const int64_t per_block = 8 * kSizeRows * (32 / lanes);
-    int per_sm = 0;
     IBP_RET(kernel_blocks_per_sm((const void *)kern, 256, 0, &per_sm));
     const int64_t blocks = std::min<int64_t>((nrows + per_block - 1) / per_block,
                                              (int64_t)device_sm_count() * per_sm);
