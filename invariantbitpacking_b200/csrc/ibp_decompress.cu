@@ -723,17 +723,22 @@ constexpr int kLaneBitmap = 256;
 // fixed-stride row, all of a condensed one -- while the next rows' metadata is loaded; a
 // fixed-stride row that needs more gets its tail the same way, and the rows are decoded
 // together (decode_group).  One set of slots per warp: a decode takes several times a read's
-// latency and the SM's other warps hide that.  Rows of up to 512 bytes of columns (ONE) keep the
-// tables in registers for the whole kernel.
+// latency and the SM's other warps hide that.  Rows of up to 512 bytes of columns, NC chunks of 32
+// (NC > 0), keep the tables in registers for the whole kernel; condensed ones, read whole,
+// also find their lengths in the decode.
 // Bound: issue and the integer pipe (a 32-bit half takes five masked moves).  Whole sets: 100k
 // rows of 256 32-bit words at half the bits 174 -> 83 us, 40k rows of 512 64-bit words at a
 // quarter 254 -> 91 us; 50k condensed rows of 99 32-bit words 87 -> 45 us (a row at a time
 // before, with eight table loads a word).  What a short row costs beside its decode is shared
 // too: lane q looks through row q's bitmap (a warp's sum per row before: 200k rows of 33 64-bit
-// words 93 us, so 72), and rows of few blocks are copied two or four at a time (61).
-template <typename U, bool ONE, bool EXACT>
+// words 93 us, so 72), and rows of few blocks are copied two or four at a time (61).  Rows that have
+// words stored whole pay for chunks their columns do not fill and for a length of their own: 200k
+// condensed rows of 16 32-bit words, all such, 71 us a row at a time, 122 in four chunks with a sum
+// per row, 40 in one without.
+template <typename U, int NC, bool EXACT>
 __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr bool ONE = NC > 0, CHECK = ONE && EXACT;
     constexpr int W = 8 * sizeof(U), per16 = 16 / sizeof(U);
     const int lane = threadIdx.x & 31;
     const int64_t v = a.s.v, mw = a.s.mw;
@@ -742,7 +747,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     // tables, counters, head records and sorted keys come from the kernels before this one
     grid_dep_wait();
     grid_dep_release();
-    GroupTables<U> gt;
+    GroupTables<U, ONE ? NC : 1> gt;
     uint32_t packed_bits = 0;  // stream bits of a row whose words are all compressible
     if constexpr (ONE) {
         gt.load(a.s.t, v, mw, 0, 0);
@@ -880,7 +885,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
             fm = __ballot_sync(0xffffffffu, full);
         }
 #pragma unroll 1
-        for (unsigned m = pm & ~fm; m; m &= m - 1) {
+        for (unsigned m = CHECK ? 0u : pm & ~fm; m; m &= m - 1) {
             const int q = __ffs(m) - 1;
             bool full;
             const uint32_t bits = row_stream_bits<U>(slots + __shfl_sync(0xffffffffu, place, q), v,
@@ -891,7 +896,8 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         // a bitmap whose stream does not fit its row cannot come from this mask: report it and
         // leave the output row alone
         const bool packed = (pm >> lane) & 1u;
-        const bool corrupt = packed && (EXACT ? end > len : end >= v);
+        const bool corrupt = packed && (!CHECK || ((fm >> lane) & 1u)) &&
+                             (EXACT ? end > len : end >= v);
         if (corrupt) atomicOr(a.status, kStatusCorruptRow);
         pm &= ~__ballot_sync(0xffffffffu, corrupt);
         if constexpr (!EXACT) {
@@ -931,7 +937,8 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         if (pm) {
             if constexpr (ONE) {
                 int64_t base = 0;
-                decode_group<U, int>(gt, slots, place, out, pm, fm, 0, mw, base);
+                decode_group<U, NC, CHECK, int>(gt, slots, place, out, pm, fm, 0, mw, base,
+                                                (int)len, a.status);
             } else {
                 decode_rows_long<U, int>(slots, place, out, pm, fm, v, mw, a.s.t);
             }
@@ -974,11 +981,15 @@ static ibp_status launch_device_fetch(FetchArgs<U> a, int nblks, int nthreads, c
     while (a.slots > 1 && 8 * a.slots * slot > 110 * 1024) a.slots /= 2;
     const int warps = (int)std::min<size_t>(block_threads(nthreads) / 32,
                                             (size_t)device_max_smem_optin() / (a.slots * slot));
-    const bool one = a.s.v * (int64_t)sizeof(U) <= 512;
-    auto kern = a.s.offsets
-                    ? (one ? device_fetch_kernel<U, true, true> : device_fetch_kernel<U, false, true>)
-                    : (one ? device_fetch_kernel<U, true, false>
-                           : device_fetch_kernel<U, false, false>);
+    // chunks of 32 columns of rows of up to 512 bytes (of 64-bit words at most 2)
+    auto kern = a.s.offsets ? device_fetch_kernel<U, 0, true> : device_fetch_kernel<U, 0, false>;
+    if (a.s.v <= 32)
+        kern = a.s.offsets ? device_fetch_kernel<U, 1, true> : device_fetch_kernel<U, 1, false>;
+    else if (a.s.v <= 64)
+        kern = a.s.offsets ? device_fetch_kernel<U, 2, true> : device_fetch_kernel<U, 2, false>;
+    else if (a.s.v * (int64_t)sizeof(U) <= 512)
+        kern = a.s.offsets ? device_fetch_kernel<U, 16 / sizeof(U), true>
+                           : device_fetch_kernel<U, 16 / sizeof(U), false>;
     const size_t smem = slot * a.slots * warps;
     int per_sm = 0;
     IBP_RET(kernel_blocks_per_sm((const void *)kern, warps * 32, smem, &per_sm));

@@ -224,14 +224,14 @@ __device__ __forceinline__ int64_t row_words(const U *__restrict__ buf, int64_t 
 
 
 // ------------------------------------------------------------------ rows decoded together
-// The tables of a group of 512 bytes of columns (64 64-bit or 128 32-bit words; column
-// g0 + 32 * c + lane), the bits its rows hold up to each column's end when every word of
+// The tables of a group of columns (column g0 + 32 * c + lane, c < GC: 512 bytes, 64 64-bit or 128
+// 32-bit words, or fewer where the rows are shorter), the bits its rows hold up to each column's end when every word of
 // the group is compressible, and, for rows that are all compressible (`before` bits in earlier
 // groups), where a column's word lies: the bytes from the row to its stream units and the shift
 // that brings its bits to the end.
-template <typename U>
+template <typename U, int GC>
 struct GroupTables {
-    static constexpr int GC = 16 / sizeof(U), H = sizeof(U) / 4;
+    static constexpr int H = sizeof(U) / 4;
     U m[GC], bv[GC], mv[GC][kMoves];
     int kept[GC];
     uint32_t incl[GC], total;
@@ -288,14 +288,17 @@ struct GroupTables {
 // the rows in `full`, which are all compressible, else at its own, from the tables for a
 // group whose words are all compressible and from a prefix sum for any other; the words of a
 // group are then read, scattered and written without a branch between them.  (Columns past the
-// end read where the row's last word ends, and what they read is not written.)  One row at a
+// end read where the row's last word ends, and what they read is not written.)  CHECK: the rows
+// are one group long and their lengths not yet known; a row whose words do not fit the `most` its
+// lane allows, which this mask cannot have made, is reported and left alone.  One row at a
 // time in a loop that is not unrolled: four rows' code side by side missed the instruction
 // cache (device_fetch_kernel, 100k rows of 256 32-bit words: 139 us, with the loop 83).
-template <typename U, typename Place>
-__device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *rows, Place place,
-                                             U *out, unsigned lanes, unsigned full, int64_t g0,
-                                             int64_t mw, int64_t &base) {
-    constexpr int W = 8 * sizeof(U), GC = GroupTables<U>::GC;
+template <typename U, int GC, bool CHECK, typename Place>
+__device__ __forceinline__ void decode_group(const GroupTables<U, GC> &t, const U *rows,
+                                             Place place, U *out, unsigned lanes, unsigned full,
+                                             int64_t g0, int64_t mw, int64_t &base,
+                                             int most = 0, int32_t *status = nullptr) {
+    constexpr int W = 8 * sizeof(U);
     constexpr int LW = LogW<U>::value;
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -307,7 +310,7 @@ __device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *r
                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), q)) +
                g0 + lane;
         if ((full >> q) & 1) {
-            constexpr int H = GroupTables<U>::H;
+            constexpr int H = GroupTables<U, GC>::H;
             const char *r = reinterpret_cast<const char *>(row);
             U x[GC];
 #pragma unroll
@@ -358,6 +361,10 @@ __device__ __forceinline__ void decode_group(const GroupTables<U> &t, const U *r
                 end[c] += all;
                 all = __shfl_sync(0xffffffffu, end[c], 31);
             }
+            if (CHECK && (int)mw + (int)((all + W - 1) / W) > __shfl_sync(0xffffffffu, most, q)) {
+                if (lane == 0) atomicOr(status, kStatusCorruptRow);
+                continue;
+            }
         }
         U x[GC];
 #pragma unroll
@@ -381,11 +388,12 @@ template <typename U, typename Place>
 __device__ __forceinline__ void decode_rows_long(const U *rows, Place place, U *out,
                                                  unsigned lanes, unsigned full, int64_t v,
                                                  int64_t mw, const ColTables<U> &t) {
+    constexpr int GC = 16 / sizeof(U);
     int64_t base = 0, before = 0;
-    for (int64_t g0 = 0; g0 < v; g0 += 32 * GroupTables<U>::GC) {
-        GroupTables<U> gt;
+    for (int64_t g0 = 0; g0 < v; g0 += 32 * GC) {
+        GroupTables<U, GC> gt;
         gt.load(t, v, mw, g0, before);
-        decode_group<U, Place>(gt, rows, place, out, lanes, full, g0, mw, base);
+        decode_group<U, GC, false, Place>(gt, rows, place, out, lanes, full, g0, mw, base);
         before += gt.total;
     }
 }
