@@ -725,7 +725,7 @@ constexpr int kLaneBitmap = 256;
 // together (decode_group).  One set of slots per warp: a decode takes several times a read's
 // latency and the SM's other warps hide that.  Rows of up to 512 bytes of columns, NC chunks of 32
 // (NC > 0), keep the tables in registers for the whole kernel; condensed ones, read whole,
-// also find their lengths in the decode.
+// also find their lengths in the decode.  LONE: warps are likely to hold one row.
 // Bound: issue and the integer pipe (a 32-bit half takes five masked moves).  Whole sets: 100k
 // rows of 256 32-bit words at half the bits 174 -> 83 us, 40k rows of 512 64-bit words at a
 // quarter 254 -> 91 us; 50k condensed rows of 99 32-bit words 87 -> 45 us (a row at a time
@@ -735,7 +735,7 @@ constexpr int kLaneBitmap = 256;
 // words stored whole pay for chunks their columns do not fill and for a length of their own: 200k
 // condensed rows of 16 32-bit words, all such, 71 us a row at a time, 122 in four chunks with a sum
 // per row, 40 in one without.
-template <typename U, int NC, bool EXACT>
+template <typename U, int NC, bool EXACT, bool LONE = false>
 __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr bool ONE = NC > 0, CHECK = ONE && EXACT;
@@ -940,7 +940,15 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
                 decode_group<U, NC, CHECK, int>(gt, slots, place, out, pm, fm, 0, mw, base,
                                                 (int)len, a.status);
             } else {
-                decode_rows_long<U, int>(slots, place, out, pm, fm, v, mw, a.s.t);
+                if (LONE && packed_bits <= 4 * v && (pm & (pm - 1)) == 0) {
+                    const int q = __ffs(pm) - 1;
+                    decode_lone_row<U>(
+                        slots + __shfl_sync(0xffffffffu, place, q), v, mw, a.s.t,
+                        reinterpret_cast<U *>(__shfl_sync(
+                            0xffffffffu, reinterpret_cast<unsigned long long>(out), q)));
+                } else {
+                    decode_rows_long<U, int>(slots, place, out, pm, fm, v, mw, a.s.t);
+                }
             }
         }
         __syncwarp();
@@ -983,6 +991,10 @@ static ibp_status launch_device_fetch(FetchArgs<U> a, int nblks, int nthreads, c
                                             (size_t)device_max_smem_optin() / (a.slots * slot));
     // chunks of 32 columns of rows of up to 512 bytes (of 64-bit words at most 2)
     auto kern = a.s.offsets ? device_fetch_kernel<U, 0, true> : device_fetch_kernel<U, 0, false>;
+    // condensed rows too long for a second slot, or no more than two blocks' warps per SM: the kernel
+    // that may decode a row by itself (with many rows to a warp it is 4% slower)
+    if (a.s.offsets && (a.slots == 1 || a.nrows <= (int64_t)device_sm_count() * 2 * warps))
+        kern = device_fetch_kernel<U, 0, true, true>;
     if (a.s.v <= 32)
         kern = a.s.offsets ? device_fetch_kernel<U, 1, true> : device_fetch_kernel<U, 1, false>;
     else if (a.s.v <= 64)
