@@ -1,9 +1,9 @@
 // ibp_bitcount.cuh -- set-bit counts per bit position over many words, in bit planes: plane d
 // of a word holds bit d of the 32 positions' counts.  Eight words go in at a time through a
-// tree of carry-save adders (7 of them, two logic operations each; the positional population
-// count of R. Zhang, "Faster population counts using AVX2 instructions", W. Mula, N. Kurz,
-// D. Lemire, The Computer Journal 61(1), 2018, applied per position), so a 32-bit word costs
-// ~3 logic operations where a ripple-carry add into eight planes costs 16.
+// tree of carry-save adders (7 of them, two logic operations each; the tree of W. Mula, N. Kurz and
+// D. Lemire, "Faster population counts using AVX2 instructions", The Computer Journal 61(1),
+// 2018, kept per bit position), so a 32-bit word costs ~3 logic operations where a ripple-carry
+// add into eight planes costs 16.
 #pragma once
 
 #include "ibp_common.cuh"

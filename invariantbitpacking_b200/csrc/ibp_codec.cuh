@@ -68,11 +68,7 @@ ColTables<U> carve_tables(Carver &c, int64_t v) {
     return t;
 }
 
-// Shifts that are well defined for every amount in [0, W].
-template <typename U>
-__device__ __forceinline__ U shl_w(U x, int s) {
-    return s >= (int)(8 * sizeof(U)) ? (U)0 : (U)(x << s);
-}
+// A shift that is well defined for every amount in [0, W].
 template <typename U>
 __device__ __forceinline__ U shr_w(U x, int s) {
     return s >= (int)(8 * sizeof(U)) ? (U)0 : (U)(x >> s);
@@ -200,10 +196,6 @@ inline ibp_status build_tables(const U *mask, const U *bitval, int64_t v, ColTab
 // ---- MSB-first stream access on 32-bit units.  Stream bit s of a W-bit word stream
 // lives in 32-bit unit s/32 of the stream when W == 32, and in unit (s/32) ^ 1 when
 // W == 64 (the high half of a little-endian 64-bit word comes second in memory).
-template <typename U>
-__device__ __forceinline__ int unit_slot(int64_t q) {
-    return sizeof(U) == 8 ? (int)(q ^ 1) : (int)q;
-}
 
 // OR up to 64 bits (left-aligned in hi:lo, the rest zero) into a shared-memory image at bit s.
 // The image's units are in stream order; units of no bits are ORed too (a test costs more).

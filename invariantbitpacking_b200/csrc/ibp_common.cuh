@@ -159,16 +159,6 @@ __device__ __forceinline__ int popc_w(U x) {
         return __popc((unsigned)x);
 }
 
-template <typename U>
-__device__ __forceinline__ int clz_w(U x) {
-    if constexpr (sizeof(U) == 8)
-        return __clzll((long long)x);
-    else if constexpr (sizeof(U) == 4)
-        return __clz((int)x);
-    else
-        return __clz((int)(unsigned)x) - (32 - 8 * (int)sizeof(U));
-}
-
 // Bytes of the per-row compressed-word bitmap (one bit per word, padded to whole words):
 // include/compress/ibp_compress_dev.cuh:12-15.
 __host__ __device__ inline int64_t meta_bytes(int64_t v, int wb) {
@@ -184,8 +174,6 @@ __host__ __device__ inline int64_t compressed_bytes(int64_t v, int wb, uint64_t 
     int64_t sz = meta_bytes(v, wb) + data;
     return sz < vb ? sz : vb;
 }
-
-__device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 // Sum over the lanes of aligned groups of G lanes (G a power of two <= 32).
 template <int G, typename T>

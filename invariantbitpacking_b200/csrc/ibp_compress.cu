@@ -4,13 +4,14 @@
 //
 // B200 design
 //  * sizes: 8, 16 or 32 lanes per row, 16 bytes a lane where rows allow it, 8 rows in flight, the
-//    columns' tables in registers; no shared-memory atomics (the reference uses one
-//    256-thread block per row with smem atomics).
-//  * packing: a warp per row and 4 rows in flight; words go from memory to registers once,
-//    each lane gathers its words' non-invariant bits with the Hacker's Delight move masks (in
-//    registers for rows of up to 64 words) and ORs them into a shared-memory image of the
-//    output row (32-bit shared atomics, at most 3 per word).  The finished row goes back with
-//    one coalesced pass; an incompressible row compressed in place is not written at all.
+//    columns' tables in registers (few long rows: a warp or a block each); no shared-memory
+//    atomics (the reference uses one 256-thread block per row with smem atomics).
+//  * packing: a warp per row and 4 rows in flight; words go from memory to registers once
+//    (host rows of whole 16-byte blocks: to shared memory), each lane gathers its words'
+//    non-invariant bits with the Hacker's Delight move masks (in registers for rows of up to 512
+//    bytes) and ORs them into a shared-memory image of the output row (three 32-bit shared
+//    atomics per 64 bits of the row).  The finished row goes back with one coalesced pass; an
+//    incompressible row compressed in place is not written at all.
 //    No global workspace is cudaMalloc'd or freed per call (the reference does both and
 //    thereby blocks the host).
 #include <cub/device/device_scan.cuh>

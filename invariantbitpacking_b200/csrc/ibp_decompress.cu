@@ -2,10 +2,11 @@
 // (replaces src/decompress.cu:10-156 and include/decompress/).
 //
 // B200 design
-//  * rows come from pinned host memory (zero-copy over PCIe) or HBM.  A warp takes a chunk
-//    of consecutive positions from a global work counter (up to its row slots for host
-//    rows, so the rows the grid has in flight stay close together; 32 for HBM rows; fewer
-//    towards the end of the work so the last chunks finish together), loads their keys,
+//  * rows come from pinned host memory (zero-copy over PCIe) or HBM; each has its kernels
+//    (fetch_rows_kernel; hbm_rows_kernel and device_fetch_kernel below).  For host rows a warp
+//    takes a chunk of consecutive positions from a global work counter (up to its row slots,
+//    so the rows the grid has in flight stay close together; 32 for raw gathers of HBM
+//    rows; fewer towards the end of the work so the last chunks finish together), loads their keys,
 //    output positions and bitmask bits lane-parallel, and then loads the first read of up
 //    to kRowsInFlight distinct rows into registers (16-byte loads, all rows before any
 //    store) and parks them in shared-memory slots, so several PCIe round trips overlap per
@@ -554,7 +555,7 @@ __device__ __forceinline__ void hbm_rows(const FetchArgs<U> &a, unsigned char *s
 #pragma unroll
             for (int q = 0; q < G; ++q) {
                 const int r = g * G + q;
-                if (r < rows && lane < nq16) cp_async16<true>(buf + q * sw, msrc[r] + lane * per16);
+                if (r < rows && lane < nq16) cp_async16(buf + q * sw, msrc[r] + lane * per16);
             }
             cp_async_commit();
         };
@@ -727,8 +728,8 @@ constexpr int kLaneBitmap = 256;
 // (NC > 0), keep the tables in registers for the whole kernel; condensed ones, read whole,
 // also find their lengths in the decode.  LONE: warps are likely to hold one row.
 // Bound: issue and the integer pipe (a 32-bit half takes five masked moves).  Whole sets: 100k
-// rows of 256 32-bit words at half the bits 174 -> 83 us, 40k rows of 512 64-bit words at a
-// quarter 254 -> 91 us; 50k condensed rows of 99 32-bit words 87 -> 45 us (a row at a time
+// rows of 256 32-bit words at half the bits 174 -> 70 us, 40k rows of 512 64-bit words at a
+// quarter 254 -> 91 us; 200k condensed rows of 99 32-bit words 203 -> 57 us (a row at a time
 // before, with eight table loads a word).  What a short row costs beside its decode is shared
 // too: lane q looks through row q's bitmap (a warp's sum per row before: 200k rows of 33 64-bit
 // words 93 us, so 72), and rows of few blocks are copied two or four at a time (61).  Rows that have
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(256, 2) device_fetch_kernel(FetchArgs<U> a) {
         const char *src = reinterpret_cast<const char *>(b0) + sub * 16;
         char *dst = reinterpret_cast<char *>(slot) + (b0 - (lo & ~(uintptr_t)15)) + sub * 16;
         for (int i = sub; i < n; i += of, src += of * 16, dst += of * 16)
-            cp_async16<true>(dst, src);
+            cp_async16(dst, src);
     };
 
     int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -614,15 +614,13 @@ __device__ __forceinline__ void fetch_heads(const RowSet<U> &s, const LaneTables
     }
 }
 
-// 16 bytes to shared memory; kL1: through the SM's L1, so that rows read by many warps (the hot
-// rows of a skewed batch, every read of which one L2 slice would serve) leave L2 once per SM.
-template <bool kL1>
+// 16 bytes to shared memory through the SM's L1, so that rows read by many warps (the hot rows of a
+// skewed batch, every read of which one L2 slice would serve) leave L2 once per SM.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const uint32_t to = (uint32_t)__cvta_generic_to_shared(smem);
-    if constexpr (kL1)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(to), "l"(gmem) : "memory");
-    else
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(gmem) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(smem)),
+                 "l"(gmem)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
