@@ -563,11 +563,10 @@ __device__ __forceinline__ bool saves_little(const ColTables<U> &t, int v, const
 // offset; the image is then written and zeroed for the next row.  Rows of up to one group keep
 // their tables in registers (ONE), and one that stays raw is known before it reaches its image.
 // Longer ones load the tables per group of columns, for Q rows at once.  A warp passes over the
-// batches it starts with for as long as all their rows stay raw, looking through them where the
-// first group of the first row saves next to nothing.  Calls whose rows all stay raw: 200k rows
-// of 128 and 20k of 1000 32-bit words 111 and 77 us with a size pass before every row, 140 and 148
-// packed and dropped, 76 and 58 now; 200k and 30k of 64 and 300 64-bit words 85 and 56, 115 and
-// 95, 77 and 54.
+// batches it starts with for as long as all their rows stay raw (long ones are looked through only
+// where the first group of the first row saves next to nothing).  96 MiB of rows that all stay raw,
+// kernel time, packed and dropped before and now: of 64 32-bit words 129 and 58 us, of 256 100 and
+// 31, of 1000 140 and 36; of 64 64-bit words 82 and 37, of 300 93 and 30.
 // The words of the next step are loaded while this one is packed.  LEVELS: moves per gather.
 template <typename U, int NC, int Q, bool ONE, bool INDEX, int LEVELS>
 __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC> &t) {
@@ -628,13 +627,11 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
                         (((uintptr_t)a.out) & 15) == 0;
     uint32_t x[Q][NC][2];
     int64_t batch = warp;
-    if (batch < batches) load(batch, 0, x);
     // batches of rows that all stay raw, up to the first other one
-    while (batch < batches && saves_little<U, NC>(a.t, v, x[0])) {
-        if (!INDEX && batch + nwarps < batches) {  // the next batch's rows, a line a lane
-            const char *next = reinterpret_cast<const char *>(a.src + (batch + nwarps) * Q * v);
-            const int64_t bytes = min((int64_t)Q, a.nrows - (batch + nwarps) * Q) * v * (int)sizeof(U);
-            if (lane * 128 < bytes) asm volatile("prefetch.global.L1 [%0];" ::"l"(next + lane * 128));
+    for (; batch < batches; batch += nwarps) {
+        if constexpr (!ONE) {
+            load(batch, 0, x);
+            if (!saves_little<U, NC>(a.t, v, x[0])) break;
         }
         const bool raw = all_raw<U, Q>(a.t, v, [&](int q) {
             const int64_t r = source(batch, q);
@@ -647,9 +644,8 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
             if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
             if (r < 0 && i < a.nrows && lane == 0) atomicOr(a.status, kStatusBadIndex);
         }
-        batch += nwarps;
-        if (batch < batches) load(batch, 0, x);
     }
+    if (ONE && batch < batches) load(batch, 0, x);
     for (; batch < batches; batch += nwarps) {
         uint32_t at[Q];  // stream bits so far
 #pragma unroll
@@ -710,12 +706,14 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
 }
 
 // Bound: the integer pipe (three operations per move and 32-bit half) and the shared atomics,
-// then HBM.  600k rows of 64 64-bit words: 459 us with tables read through L1 and the row staged
+// then HBM. 600k rows of 64 64-bit words: 459 us with tables read through L1 and the row staged
 // and packed in two passes; 317 with tables in registers; 207 with 32-bit indices and images in
 // stream order; 188 with the moves chosen once; 163 without a test per atomic (its branches cost
-// more than the atomics of zeros); 137 now with the 16-byte epilogue, 4.1 TB/s.  32-bit words
-// two to a lane rather than one (half the prefix sums, three atomics for two words instead of
-// four): 200k rows of 99 words 254 us at first, 110, 92 now; of 400 words 308, 164, 150.  Rows whose
+// more than the atomics of zeros); 137 with the 16-byte epilogue; 120 now, 4.6 TB/s, with raw
+// rows out of the loop's way (what else stands in the function decides how the loop is compiled:
+// the same loop took 120 to 143 under different ways to pass over raw batches). 32-bit words two
+// to a lane rather than one (half the prefix sums, three atomics for two words instead of four):
+// 200k rows of 99 words 254 us at first, 110, 92 now; of 400 words 308, 164, 150. Rows whose
 // tables stay in registers choose their moves once (LEVELS 2 covers masks that drop at most
 // three bits above any kept one, as quantised floats do).
 template <typename U, int NC, int Q, bool ONE, bool INDEX>
