@@ -4,6 +4,7 @@ and with the running total; and in about the time the same bytes take as many sh
 import numpy as np
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from test_gpu_match_chunks import INT, put, rows_of
 
@@ -46,17 +47,17 @@ def test_few_long_rows_take_about_as_long_as_many(wb, v, rows):
     x = x.view(torch.from_numpy(np.zeros(1, INT[wb])).dtype)
     m = torch.randint(-128, 128, (v * wb,), dtype=torch.int8, device="cuda").view(x.dtype)
 
-    def best_ms(t, k):
-        times = []
-        for _ in range(6):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            ibp.get_compress_size(t, m[:k], m[:k])
-            b.record()
-            b.synchronize()
-            times.append(a.elapsed_time(b))
-        return min(times)
+    def size_us(t, k):
+        """GPU time of the size kernel."""
+        ibp.get_compress_size(t, m[:k], m[:k])
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            for _ in range(6):
+                ibp.get_compress_size(t, m[:k], m[:k])
+            torch.cuda.synchronize()
+        return min(e.device_time for e in prof.events()
+                   if "size_kernel" in e.name and e.device_type.name == "CUDA")
 
-    many = best_ms(x.view(-1, v // 100), v // 100)
-    few = best_ms(x.view(rows, v), v)
+    many = size_us(x.view(-1, v // 100), v // 100)
+    few = size_us(x.view(rows, v), v)
     assert few < 2 * many, (few, many)
