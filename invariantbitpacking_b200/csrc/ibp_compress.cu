@@ -633,17 +633,16 @@ __device__ __forceinline__ void pack_rows(const PackArgs<U> &a, PackTables<U, NC
             load(batch, 0, x);
             if (!saves_little<U, NC>(a.t, v, x[0])) break;
         }
-        const bool raw = all_raw<U, Q>(a.t, v, [&](int q) {
-            const int64_t r = source(batch, q);
-            return a.src + (r < 0 ? 0 : r) * v;
-        });
-        if (!raw) break;
+        // (a batch with a position that has no row, which must not be read, goes on below)
+        bool whole = true;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const int64_t i = batch * Q + q, r = source(batch, q);
-            if (r >= 0 && !a.in_place) warp_copy<U>(target(i), a.src + r * v, v);
-            if (r < 0 && i < a.nrows && lane == 0) atomicOr(a.status, kStatusBadIndex);
-        }
+        for (int q = 0; q < Q; ++q) whole = whole && source(batch, q) >= 0;
+        if (!whole) break;
+        if (!all_raw<U, Q>(a.t, v, [&](int q) { return a.src + source(batch, q) * v; })) break;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (!a.in_place)
+                warp_copy<U>(target(batch * Q + q), a.src + source(batch, q) * v, v);
     }
     if (ONE && batch < batches) load(batch, 0, x);
     for (; batch < batches; batch += nwarps) {

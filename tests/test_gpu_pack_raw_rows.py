@@ -148,3 +148,28 @@ def test_raw_host_rows_cross_the_link_once():
                    if name in e.name and e.device_type.name == "CUDA")
 
     assert best_us("pack") < 2 * best_us("Memcpy HtoD")
+
+
+@pytest.mark.parametrize("wb,v", [(4, 64), (4, 99), (4, 300), (8, 2), (8, 64), (8, 300)])
+def test_a_set_without_rows_is_never_read(wb, v):
+    """An index into a set of no rows: every position is bad, nothing is read or written."""
+    import ctypes
+
+    from invariantbitpacking_b200 import _capi
+    lib = _capi.lib
+    dtype = torch.from_numpy(np.zeros(1, INT[wb])).dtype
+    mask = torch.ones(v, dtype=dtype, device="cuda")
+    idx = torch.arange(3000, device="cuda")
+    offsets = torch.zeros(3000, dtype=torch.int64, device="cuda")
+    out = torch.full((8,), 7, dtype=dtype, device="cuda")
+    need = lib.ibp_compress_condensed_workspace_size(v, wb)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    status = lib.ibp_compress_condensed(None, 0, v, wb, mask.data_ptr(), mask.data_ptr(),
+                                        idx.data_ptr(), 3000, offsets.data_ptr(), out.data_ptr(),
+                                        ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream)
+    assert status == 0
+    word = torch.zeros(1, dtype=torch.int32)
+    _capi.check(lib.ibp_read_status(ws.data_ptr(), ctypes.c_void_p(word.data_ptr()),
+                                    torch.cuda.current_stream().cuda_stream))
+    assert int(word) & 1
+    assert bool((out == 7).all())
